@@ -1,245 +1,27 @@
-// Kernels of the warm-start MLP: a BF16 GEMM on the 5th-generation tensor
-// cores (tcgen05.mma, accumulator in tensor memory) and the elementwise
-// pieces of the forward pass, the backward pass and the Adam step.
-//
-// GEMM form: D[M x N] (fp32) = A[M x K] . B[N x K]^T (+ D), A and B bf16,
-// row-major with K contiguous ("TN"); every other product of the MLP is
-// brought to this form by explicit transposes.  M, N multiples of 128, K a
-// multiple of 64, leading dimensions multiples of 8 elements.
-//
-// One CTA (4 warps) computes one 128 x 128 tile.  K streams in 64-deep
-// stages through a 3-stage shared-memory ring filled with cp.async; each
-// stage is laid out in the canonical no-swizzle K-major UMMA layout (8-row x
-// 16-byte core matrices; LBO = 128 B between the two K halves of one MMA,
-// SBO = 1024 B between 8-row groups).  Thread 0 issues four
-// tcgen05.mma.kind::f16 (M=128, N=128, K=16) per stage and commits them to
-// the stage's mbarrier; producers wait on that mbarrier before refilling the
-// stage.  The epilogue reads the 128 x 128 fp32 accumulator from TMEM
-// (tcgen05.ld 32x32b: warp w owns lanes 32w..32w+31 = tile rows) and stores
-// it.  Every mbarrier wait is bounded; on timeout the kernel sets *err and
-// finishes without touching further data.
+// Kernels of the warm-start MLP: the launches of its BF16 GEMM on the
+// 5th-generation tensor cores (mlp_gemm.cuh) and the pieces around it: the
+// first layer of outage rows, the loss gradient, bias gradients, the Adam step
+// and the start voltages.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
 
+#include "mlp_gemm.cuh"
+
 namespace gs2g {
 namespace mlp {
 
-constexpr int GT = 128;     // tile M = tile N
-constexpr int GK = 64;      // K per stage
-// operand ring depth: a stage is reloaded once the MMAs of the k-tile before
-// it have completed (STAGES - 2 k-tiles of operands in flight).  6 stages
-// (one CTA per SM) measured no faster than 3 (two CTAs per SM fit): with
-// 128 x 128 tiles the operands are re-read from L2 at about 3.7 TB/s, which
-// bounds the kernel before the ring depth does
-#ifndef GS2G_GEMM_STAGES
-#define GS2G_GEMM_STAGES 3
-#endif
-constexpr int STAGES = GS2G_GEMM_STAGES;
-constexpr int GEMM_THREADS = 128;
-constexpr int TILE_BYTES = GT * GK * 2;  // one operand tile per stage (16 KB)
-constexpr int GEMM_SMEM = STAGES * 2 * TILE_BYTES + 1024;
-constexpr uint64_t WAIT_NS = 2000000000ull;  // bound of one mbarrier wait (2 s)
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src));
-}
-
-// UMMA shared-memory descriptor, K-major, no swizzle.
-__device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr >> 4) & 0x3FFF);
-  d |= (uint64_t)((lbo >> 4) & 0x3FFF) << 16;
-  d |= (uint64_t)((sbo >> 4) & 0x3FFF) << 32;
-  d |= (uint64_t)1 << 46;  // descriptor version for sm_100
-  return d;                // base offset 0, legacy LBO mode, layout SWIZZLE_NONE
-}
-
-// Instruction descriptor: kind::f16, A = B = bf16, D = f32, both K-major.
-__host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
-}
-
-__device__ __forceinline__ uint64_t global_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
-}
-
-// Bounded wait for the phase with the given parity; false after WAIT_NS.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-  const uint64_t t0 = global_ns();
-  for (uint32_t i = 0;; ++i) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (done) return true;
-    if ((i & 255) == 255 && global_ns() - t0 > WAIT_NS) return false;
-  }
-}
-
-__global__ void __launch_bounds__(GEMM_THREADS) gemm_tn_bf16_kernel(const __nv_bfloat16* __restrict__ A, int lda,
-                                                                    const __nv_bfloat16* __restrict__ B, int ldb,
-                                                                    float* __restrict__ D, int ldd, int K,
-                                                                    int accumulate, int* err) {
-  extern __shared__ __align__(1024) unsigned char smem[];
-  __shared__ __align__(8) uint64_t mbar[STAGES];
-  __shared__ uint32_t tmem_base_s;
-  __shared__ int s_fail;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.y * GT, n0 = blockIdx.x * GT;
-  // 1024-byte aligned operand ring
-  const uint32_t ring = (smem_u32(smem) + 1023) & ~1023u;
-  auto a_tile = [&](int s) { return ring + (uint32_t)(s * 2 * TILE_BYTES); };
-  auto b_tile = [&](int s) { return ring + (uint32_t)(s * 2 * TILE_BYTES + TILE_BYTES); };
-
-  if (tid == 0) {
-    for (int s = 0; s < STAGES; ++s)
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&mbar[s])));
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::);
-    s_fail = 0;
-  }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_base_s)),
-                 "r"(GT));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
-  const uint32_t tmem = tmem_base_s;
-
-  const int KT = K / GK;
-  // canonical layout offset of (row r, 16-byte k-chunk c) inside a tile
-  auto load_stage = [&](int kt, int s) {
-    const int k0 = kt * GK;
-#pragma unroll
-    for (int i = 0; i < (GT * GK / 8) / GEMM_THREADS; ++i) {
-      const int idx = tid + i * GEMM_THREADS;  // 0 .. 1023
-      const int r = idx >> 3, c = idx & 7;
-      const uint32_t off = (uint32_t)((r >> 3) * 1024 + c * 128 + (r & 7) * 16);
-      cp_async16(a_tile(s) + off, A + (int64_t)(m0 + r) * lda + k0 + c * 8);
-      cp_async16(b_tile(s) + off, B + (int64_t)(n0 + r) * ldb + k0 + c * 8);
-    }
-  };
-  // Group bookkeeping: the prologue commits k-tiles 0..STAGES-2 as groups
-  // 0..STAGES-2; iteration kt commits one group (k-tile kt+STAGES-1, or
-  // empty), so k-tile kt is always group kt, and at iteration kt the
-  // STAGES-2 most recent groups may still be in flight.
-#pragma unroll
-  for (int s = 0; s < STAGES - 1; ++s) {
-    if (s < KT) load_stage(s, s);
-    asm volatile("cp.async.commit_group;\n" ::);
-  }
-  constexpr uint32_t idesc = umma_idesc_bf16(GT, GT);
-  bool ok = true;
-  int last = -1;  // last k-tile whose MMAs were committed
-  for (int kt = 0; kt < KT; ++kt) {
-    const int s = kt % STAGES;
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2) : "memory");
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-    if (__syncthreads_or(!ok)) {  // a timed-out wait anywhere stops every thread here
-      ok = false;
-      break;
-    }
-    if (tid == 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
-#pragma unroll
-      for (int j = 0; j < GK / 16; ++j) {
-        const uint64_t ad = umma_desc(a_tile(s) + j * 256, 128, 1024);
-        const uint64_t bd = umma_desc(b_tile(s) + j * 256, 128, 1024);
-        const uint32_t en = (kt > 0 || j > 0) ? 1u : 0u;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(tmem),
-            "l"(ad), "l"(bd), "r"(idesc), "r"(en), "r"(0), "r"(0), "r"(0), "r"(0));
-      }
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-          smem_u32(&mbar[s])));
-    }
-    last = kt;
-    // load k-tile kt+STAGES-1 into the stage k-tile kt-1 used (at kt = 0: the
-    // still unused last stage), once k-tile kt-1's MMAs are done
-    const int nk = kt + STAGES - 1;
-    if (nk < KT) {
-      const int ns = nk % STAGES;
-      if (kt >= 1 && !mbar_wait(smem_u32(&mbar[ns]), (uint32_t)(((kt - 1) / STAGES) & 1))) ok = false;
-      if (ok) load_stage(nk, ns);
-    }
-    asm volatile("cp.async.commit_group;\n" ::);
-  }
-  // wait for the last committed MMAs (after a failure too: TMEM is freed
-  // only once they are done, or their wait has run out as well)
-  if (last >= 0 && !mbar_wait(smem_u32(&mbar[last % STAGES]), (uint32_t)((last / STAGES) & 1))) ok = false;
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-  asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
-  if (__syncthreads_or(!ok) && tid == 0) s_fail = 1;
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
-  if (s_fail) {
-    if (tid == 0) atomicExch(err, 1);
-  } else {
-    // epilogue: warp w reads TMEM lanes 32w..32w+31 (tile rows), 16 columns per load
-    const int row = m0 + warp * 32 + lane;
-    float* drow = D + (int64_t)row * ldd + n0;
-#pragma unroll 1
-    for (int c0 = 0; c0 < GT; c0 += 16) {
-      uint32_t v[16];
-      const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0;
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-          : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-            "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-          : "r"(taddr));
-      asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-#pragma unroll
-      for (int q = 0; q < 16; q += 4) {
-        float4 o = make_float4(__uint_as_float(v[q]), __uint_as_float(v[q + 1]), __uint_as_float(v[q + 2]),
-                               __uint_as_float(v[q + 3]));
-        float4* dst = reinterpret_cast<float4*>(drow + c0 + q);
-        if (accumulate) {
-          const float4 old = *dst;
-          o.x += old.x;
-          o.y += old.y;
-          o.z += old.z;
-          o.w += old.w;
-        }
-        *dst = o;
-      }
-    }
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
-  __syncthreads();
-  if (warp == 0) {
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(GT));
-  }
-}
-
 // ------------------------------------------------------------ elementwise
-__device__ __forceinline__ float gelu_f(float x) { return 0.5f * x * (1.f + erff(x * 0.70710678118654752f)); }
-__device__ __forceinline__ float gelu_grad_f(float x) {
-  const float cdf = 0.5f * (1.f + erff(x * 0.70710678118654752f));
-  const float pdf = 0.39894228040143268f * expf(-0.5f * x * x);
-  return cdf + x * pdf;
-}
-
+// Two-dimensional kernels: a thread owns one column and walks over rows.
 // pre[r][c] += bias[c]; act[r][c] = bf16(gelu(pre)) (or bf16(pre) when !gelu)
 __global__ void bias_act_kernel(float* pre, int ldp, const float* bias, __nv_bfloat16* act, int lda, int rows,
                                 int cols, int gelu) {
-  const int64_t n = (int64_t)rows * cols;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int r = (int)(i / cols), c = (int)(i % cols);
-    const float v = pre[(int64_t)r * ldp + c] + bias[c];
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= cols) return;
+  const float b = bias[c];
+  for (int r = blockIdx.y; r < rows; r += gridDim.y) {
+    const float v = pre[(int64_t)r * ldp + c] + b;
     pre[(int64_t)r * ldp + c] = v;
     if (act) act[(int64_t)r * lda + c] = __float2bfloat16(gelu ? gelu_f(v) : v);
   }
@@ -248,32 +30,38 @@ __global__ void bias_act_kernel(float* pre, int ldp, const float* bias, __nv_bfl
 // dpre = dact * gelu'(pre) (fp32 in, bf16 out)
 __global__ void gelu_bwd_kernel(const float* dact, int ldg, const float* pre, int ldp, __nv_bfloat16* dpre, int ldo,
                                 int rows, int cols) {
-  const int64_t n = (int64_t)rows * cols;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int r = (int)(i / cols), c = (int)(i % cols);
-    dpre[(int64_t)r * ldo + c] =
-        __float2bfloat16(dact[(int64_t)r * ldg + c] * gelu_grad_f(pre[(int64_t)r * ldp + c]));
-  }
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= cols) return;
+  for (int r = blockIdx.y; r < rows; r += gridDim.y)
+    dpre[(int64_t)r * ldo + c] = __float2bfloat16(dact[(int64_t)r * ldg + c] * gelu_grad_f(pre[(int64_t)r * ldp + c]));
 }
 
 // dy = scale * (y - t) over the first `cols_valid` columns (0 elsewhere),
-// bf16; loss += sum (y - t)^2 over valid entries.
-__global__ void mse_grad_kernel(const float* y, const float* t, int ld, __nv_bfloat16* dy, int rows, int cols,
-                                int cols_valid, float scale, float* loss) {
-  const int64_t n = (int64_t)rows * cols;
+// bf16; loss += sum (y - t)^2 over valid entries, one atomic per block (one
+// per warp of a grid-stride pass serialised on the loss).
+__global__ void __launch_bounds__(256) mse_grad_kernel(const float* y, const float* t, int ld, __nv_bfloat16* dy,
+                                                       int rows, int cols, int cols_valid, float scale, float* loss) {
+  __shared__ float s_sum[8];
+  const int c = blockIdx.x * 256 + threadIdx.x;
   float acc = 0.f;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(i % cols);
-    float g = 0.f;
-    if (c < cols_valid) {
-      const float d = y[i] - t[i];
-      acc += d * d;
-      g = scale * d;
+  if (c < cols)
+    for (int r = blockIdx.y; r < rows; r += gridDim.y) {
+      const int64_t i = (int64_t)r * ld + c;
+      float g = 0.f;
+      if (c < cols_valid) {
+        const float d = y[i] - t[i];
+        acc += d * d;
+        g = scale * d;
+      }
+      dy[i] = __float2bfloat16(g);
     }
-    dy[i] = __float2bfloat16(g);
-  }
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0 && loss) atomicAdd(loss, acc);
+  if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0 && loss) {
+    for (int w = 1; w < 8; ++w) acc += s_sum[w];
+    atomicAdd(loss, acc);
+  }
 }
 
 // column sums of a bf16 matrix: out[c] += sum_r x[r][c]; block (128 columns)
@@ -532,31 +320,118 @@ int invalid(const char* what) {
   gs2g::set_last_error(what);
   return 1;
 }
+
+// 256 columns per block, rows over at most 148 * 8 blocks in all
+dim3 col_grid(int rows, int cols) {
+  const int gx = (cols + 255) / 256;
+  int gy = (148 * 8 + gx - 1) / gx;
+  if (gy > rows) gy = rows;
+  return dim3(gx, gy < 1 ? 1 : gy);
+}
+
+int sm_count() {
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return 148;
+  return n > 0 ? n : 148;
+}
+
+// The tensor map of one GEMM operand with `rows` M or N indices: K-major
+// X[i][k] in boxes of 64 k x box rows, MN-major X[k][i] in boxes of 64 i x 64 k;
+// what lies past the matrix reads as zero.
+bool operand_map(CUtensorMap* map, const void* p, int ld, bool mn, int rows, int K, int box) {
+  using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                              const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                              CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static const Encode encode = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      f = nullptr;
+    return reinterpret_cast<Encode>(f);
+  }();
+  if (encode == nullptr) return false;
+  const cuuint64_t dims[2] = {(cuuint64_t)(mn ? rows : K), (cuuint64_t)(mn ? K : rows)};
+  const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
+  const cuuint32_t boxes[2] = {64u, (cuuint32_t)(mn ? 64 : box)}, ones[2] = {1u, 1u};
+  return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(p), dims, strides, boxes, ones,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int BN, bool A_MN, bool B_MN>
+cudaError_t launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const GemmShape& g, const Epilogue& e, int* err,
+                        void* stream) {
+  cudaError_t rc = cudaFuncSetAttribute(gemm_bf16_kernel<BN, A_MN, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        gemm_smem<BN>());
+  if (rc != cudaSuccess) return rc;
+  const int tiles = g.tiles_m * g.tiles_n * g.splits, n_sm = sm_count();
+  gemm_bf16_kernel<BN, A_MN, B_MN><<<tiles < n_sm ? tiles : n_sm, GEMM_THREADS, gemm_smem<BN>(),
+                                     (cudaStream_t)stream>>>(ma, mb, g, e, err);
+  return cudaGetLastError();
+}
 }  // namespace
 
 extern "C" {
 
+int64_t gs2g_mlp_gemm_part(int M, int N, int K) {
+  if (M <= 0 || N <= 0 || K <= 0 || M % GT || N % GT || K % GK) return 0;
+  const GemmPlan p = gemm_plan(M, N, K, sm_count(), true);
+  return p.splits > 1 ? (int64_t)p.splits * M * N : 0;
+}
+
+int gs2g_mlp_gemm(const void* A, int lda, int a_mn, const void* B, int ldb, int b_mn, int M, int N, int K, int op,
+                  int accumulate, float* D, int ldd, const float* bias, void* act_bf16, int ld_act, float* part,
+                  int64_t part_elems, int* err, void* stream) {
+  if (M % GT || N % GT || K % GK || M <= 0 || N <= 0 || K <= 0)
+    return invalid("gemm: M, N must be positive multiples of 128 and K of 64");
+  if (lda % 8 || ldb % 8 || lda < (a_mn ? M : K) || ldb < (b_mn ? N : K) || !err)
+    return invalid("gemm: leading dimensions must cover the rows and be 16-byte multiples");
+  if (((uintptr_t)A | (uintptr_t)B) & 15) return invalid("gemm: operands must be 16-byte aligned");
+  if (op < EPI_STORE || op > EPI_GELU_BWD || (!D && op != EPI_GELU) || (D && ldd < N) ||
+      ((op == EPI_BIAS || op == EPI_GELU) && !bias) || ((op == EPI_GELU || op == EPI_GELU_BWD) && (!act_bf16 || ld_act < N)))
+    return invalid("gemm: the epilogue's buffers are missing or too narrow");
+  GemmPlan p = gemm_plan(M, N, K, sm_count(), part != nullptr);
+  if (p.splits > 1 && part_elems < (int64_t)p.splits * M * N) p = gemm_plan(M, N, K, sm_count(), false);
+  GemmShape g{M, N, K / GK, M / GT, (N + p.bn - 1) / p.bn, p.splits, p.kt_split, part};
+  const Epilogue e{op, accumulate, D, ldd, bias, (__nv_bfloat16*)act_bf16, ld_act};
+  CUtensorMap ma, mb;
+  if (!operand_map(&ma, A, lda, a_mn, M, K, GT) || !operand_map(&mb, B, ldb, b_mn, N, K, p.bn)) {
+    gs2g::set_last_error("gemm: the driver rejected a tensor map");
+    return 3;
+  }
+  cudaError_t rc;
+  if (p.bn == 256)
+    rc = a_mn ? (b_mn ? launch_gemm<256, true, true>(ma, mb, g, e, err, stream)
+                      : launch_gemm<256, true, false>(ma, mb, g, e, err, stream))
+              : (b_mn ? launch_gemm<256, false, true>(ma, mb, g, e, err, stream)
+                      : launch_gemm<256, false, false>(ma, mb, g, e, err, stream));
+  else
+    rc = a_mn ? (b_mn ? launch_gemm<128, true, true>(ma, mb, g, e, err, stream)
+                      : launch_gemm<128, true, false>(ma, mb, g, e, err, stream))
+              : (b_mn ? launch_gemm<128, false, true>(ma, mb, g, e, err, stream)
+                      : launch_gemm<128, false, false>(ma, mb, g, e, err, stream));
+  if (rc == cudaSuccess && g.splits > 1) {
+    finish_kernel<<<dim3((N + 255) / 256, M < 512 ? M : 512), 256, 0, (cudaStream_t)stream>>>(g, e);
+    rc = cudaGetLastError();
+  }
+  return status_of(rc);
+}
+
 int gs2g_mlp_gemm_tn_bf16(const void* A, int lda, const void* B, int ldb, float* D, int ldd, int M, int N, int K,
                           int accumulate, int* err, void* stream) {
-  if (M % GT || N % GT || K % GK || M <= 0 || N <= 0 || K <= 0)
-    return invalid("gemm_tn_bf16: M, N must be positive multiples of 128 and K of 64");
-  if (lda % 8 || ldb % 8 || ldd % 4 || lda < K || ldb < K || ldd < N || !err)
-    return invalid("gemm_tn_bf16: leading dimensions must cover the rows and be 16-byte multiples");
-  if (((uintptr_t)A | (uintptr_t)B | (uintptr_t)D) & 15) return invalid("gemm_tn_bf16: operands must be 16-byte aligned");
-  cudaError_t e = cudaFuncSetAttribute(gemm_tn_bf16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM);
-  if (e != cudaSuccess) return status_of(e);
-  dim3 grid(N / GT, M / GT);
-  gemm_tn_bf16_kernel<<<grid, GEMM_THREADS, GEMM_SMEM, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)A, lda, (const __nv_bfloat16*)B, ldb, D, ldd, K, accumulate, err);
-  return status_of(cudaGetLastError());
+  if (ldd % 4 || ((uintptr_t)D & 15)) return invalid("gemm_tn_bf16: D must be 16-byte aligned with 16-byte row steps");
+  return gs2g_mlp_gemm(A, lda, 0, B, ldb, 0, M, N, K, EPI_STORE, accumulate, D, ldd, nullptr, nullptr, 0, nullptr, 0,
+                       err, stream);
 }
 
 int gs2g_mlp_bias_act(float* pre, int ldp, const float* bias, void* act_bf16, int lda, int rows, int cols, int gelu,
                       void* stream) {
   const int64_t n = (int64_t)rows * cols;
   if (n <= 0) return n < 0 ? invalid("bias_act: negative size") : 0;
-  bias_act_kernel<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(pre, ldp, bias, (__nv_bfloat16*)act_bf16, lda,
-                                                                      rows, cols, gelu);
+  bias_act_kernel<<<col_grid(rows, cols), 256, 0, (cudaStream_t)stream>>>(pre, ldp, bias, (__nv_bfloat16*)act_bf16,
+                                                                          lda, rows, cols, gelu);
   return status_of(cudaGetLastError());
 }
 
@@ -564,8 +439,8 @@ int gs2g_mlp_gelu_bwd(const float* dact, int ldg, const float* pre, int ldp, voi
                       int cols, void* stream) {
   const int64_t n = (int64_t)rows * cols;
   if (n <= 0) return n < 0 ? invalid("gelu_bwd: negative size") : 0;
-  gelu_bwd_kernel<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(dact, ldg, pre, ldp, (__nv_bfloat16*)dpre_bf16,
-                                                                      ldo, rows, cols);
+  gelu_bwd_kernel<<<col_grid(rows, cols), 256, 0, (cudaStream_t)stream>>>(dact, ldg, pre, ldp,
+                                                                          (__nv_bfloat16*)dpre_bf16, ldo, rows, cols);
   return status_of(cudaGetLastError());
 }
 
@@ -574,8 +449,8 @@ int gs2g_mlp_mse_grad(const float* y, const float* t, int ld, void* dy_bf16, int
   const int64_t n = (int64_t)rows * cols;
   if (n == 0) return 0;
   if (n < 0 || ld != cols || cols_valid > cols) return invalid("mse_grad: ld must equal cols >= cols_valid");
-  mse_grad_kernel<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(y, t, ld, (__nv_bfloat16*)dy_bf16, rows, cols,
-                                                                      cols_valid, scale, loss);
+  mse_grad_kernel<<<col_grid(rows, cols), 256, 0, (cudaStream_t)stream>>>(y, t, ld, (__nv_bfloat16*)dy_bf16, rows,
+                                                                          cols, cols_valid, scale, loss);
   return status_of(cudaGetLastError());
 }
 

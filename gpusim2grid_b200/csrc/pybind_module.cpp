@@ -526,6 +526,14 @@ void bind_mlp(py::module_& m) {
     check(gs2g_mlp_gemm_tn_bf16(P<void>(A), lda, P<void>(B), ldb, P<float>(D), ldd, M, N, K, accumulate ? 1 : 0,
                                 P<int>(err), S(stream)));
   });
+  mm.def("gemm_part", &gs2g_mlp_gemm_part);
+  mm.def("gemm", [](uintptr_t A, int lda, bool a_mn, uintptr_t B, int ldb, bool b_mn, int M, int N, int K, int op,
+                    bool accumulate, uintptr_t D, int ldd, uintptr_t bias, uintptr_t act, int ld_act, uintptr_t part,
+                    int64_t part_elems, uintptr_t err, uintptr_t stream) {
+    check(gs2g_mlp_gemm(P<void>(A), lda, a_mn ? 1 : 0, P<void>(B), ldb, b_mn ? 1 : 0, M, N, K, op, accumulate ? 1 : 0,
+                        P<float>(D), ldd, P<float>(bias), P<void>(act), ld_act, P<float>(part), part_elems, P<int>(err),
+                        S(stream)));
+  });
   mm.def("bias_act", [](uintptr_t pre, int ldp, uintptr_t bias, uintptr_t act, int lda, int rows, int cols, bool gelu,
                         uintptr_t stream) {
     check(gs2g_mlp_bias_act(P<float>(pre), ldp, P<float>(bias), P<void>(act), lda, rows, cols, gelu ? 1 : 0,

@@ -42,6 +42,8 @@ from ._native import lib
 __all__ = ["WarmStartMLP", "LearnedStart", "make_training_rows", "generate_solutions"]
 
 _M = lib.mlp
+# operations of gs2g_mlp_gemm on a finished sum
+_STORE, _BIAS, _GELU, _GELU_BWD = range(4)
 
 
 def _ceil(x, m):
@@ -149,50 +151,61 @@ class WarmStartMLP:
             return self._ws[key]
         dev, f32, bf = self.device, torch.float32, torch.bfloat16
         L = self.layers
-        w = dict(pre=[torch.empty(B, self.h, dtype=f32, device=dev) for _ in range(L)],
+        # pre[l]: the hidden layers' sums before the activation, which the
+        # backward pass reads (inference only keeps the first layer's, for
+        # predict_trips)
+        w = dict(pre=[torch.empty(B, self.h, dtype=f32, device=dev) if train or l == 0 else None for l in range(L)],
                  act=[torch.empty(B, self.h, dtype=bf, device=dev) for _ in range(L)],
                  y=torch.empty(B, self.o, dtype=f32, device=dev))
+        mnk = [(B, o, i) for o, i in self.shapes]
         if train:
             w.update(dy=torch.empty(B, self.o, dtype=bf, device=dev),
-                     g=torch.empty(B, self.h, dtype=bf, device=dev),
-                     gT=torch.empty(max(self.h, self.o), B, dtype=bf, device=dev),
-                     aT=torch.empty(max(self.h, self.k0), B, dtype=bf, device=dev),
-                     WT=torch.empty(self.h, max(self.h, self.o), dtype=bf, device=dev),
-                     da=torch.empty(B, self.h, dtype=f32, device=dev),
+                     g=[torch.empty(B, self.h, dtype=bf, device=dev) for _ in range(min(L, 2))],
                      loss=torch.zeros(1, dtype=f32, device=dev))
+            mnk += [(o, i, B) for o, i in self.shapes] + [(B, i, o) for o, i in self.shapes[1:]]
+        w["part"] = torch.empty(max(_M.gemm_part(*s) for s in mnk), dtype=f32, device=dev)
         self._ws[key] = w
         return w
 
     # ------------------------------------------------------------- kernels
-    def _gemm(self, A, B, D, acc=False):
-        M, K = A.shape
-        N, K2 = B.shape
-        if K != K2 or tuple(D.shape) != (M, N):
-            raise ValueError(f"gemm shapes {tuple(A.shape)} x {tuple(B.shape)}^T -> {tuple(D.shape)}")
-        _M.gemm_tn_bf16(A.data_ptr(), A.stride(0), B.data_ptr(), B.stride(0), D.data_ptr(), D.stride(0), M, N, K,
-                        acc, self.err.data_ptr(), _stream())
+    def _gemm(self, w, op, A, B, D, a_mn=False, b_mn=False, bias=None, act=None):
+        """One product on gs2g_mlp_gemm: A (M, K), or (K, M) with ``a_mn``; B
+        (N, K), or (K, N) with ``b_mn``; ``op`` and its buffers as there."""
+        M, K = A.shape[::-1] if a_mn else A.shape
+        N, K2 = B.shape[::-1] if b_mn else B.shape
+        if K != K2 or any(t is not None and tuple(t.shape) != (M, N) for t in (D, act)):
+            raise ValueError(f"gemm shapes {tuple(A.shape)} ({a_mn}) x {tuple(B.shape)} ({b_mn})")
+        ptr = lambda t: 0 if t is None else t.data_ptr()
+        ld = lambda t: 0 if t is None else t.stride(0)
+        _M.gemm(A.data_ptr(), A.stride(0), a_mn, B.data_ptr(), B.stride(0), b_mn, M, N, K, op, False, ptr(D), ld(D),
+                ptr(bias), ptr(act), ld(act), w["part"].data_ptr(), w["part"].numel(), self.err.data_ptr(), _stream())
 
     def _wb(self, l):
         return self._view(self.wb, l, False)
 
     def _forward(self, X, w):
-        self._gemm(X, self._wb(0), w["pre"][0])
-        return self._forward_rest(w, X.shape[0])
+        """The network's outputs w['y'] for inputs X; every bias and activation
+        is applied by the product that feeds it."""
+        self._layer(0, X, w)
+        return self._layers_after(0, w)
+
+    def _layer(self, l, a, w):
+        if l < self.layers:
+            self._gemm(w, _GELU, a, self._wb(l), w["pre"][l] if "dy" in w or l == 0 else None, bias=self.b(l), act=w["act"][l])
+        else:
+            self._gemm(w, _BIAS, a, self._wb(l), w["y"], bias=self.b(l))
+
+    def _layers_after(self, l, w):
+        for k in range(l + 1, self.layers + 1):
+            self._layer(k, w["act"][k - 1], w)
+        return w["y"]
 
     def _forward_rest(self, w, B):
-        """The network from the first layer's pre-activations w['pre'][0]
-        (B rows) to its outputs w['y']."""
-        L = self.layers
-        for l in range(L + 1):
-            if l > 0:
-                self._gemm(w["act"][l - 1], self._wb(l), w["pre"][l] if l < L else w["y"])
-            if l < L:
-                _M.bias_act(w["pre"][l].data_ptr(), self.h, self.b(l).data_ptr(), w["act"][l].data_ptr(), self.h,
-                            B, self.h, True, _stream())
-            else:
-                _M.bias_act(w["y"].data_ptr(), self.o, self.b(l).data_ptr(), 0, self.o, B, self.o, False,
-                            _stream())
-        return w["y"]
+        """The network from the first layer's sums w['pre'][0] without bias (B
+        rows) to its outputs w['y']."""
+        _M.bias_act(w["pre"][0].data_ptr(), self.h, self.b(0).data_ptr(), w["act"][0].data_ptr(), self.h, B, self.h,
+                    True, _stream())
+        return self._layers_after(0, w)
 
     def _sparse_first(self):
         """(W0T, base) of the current first-layer weights and input
@@ -245,23 +258,19 @@ class WarmStartMLP:
         st = _stream()
         _M.mse_grad(w["y"].data_ptr(), T.data_ptr(), self.o, w["dy"].data_ptr(), B, self.o, self.n_out, scale,
                     w["loss"].data_ptr(), st)
-        g, gcols = w["dy"], self.o
+        g = w["dy"]
         for l in range(L, -1, -1):
             o, i = self.shapes[l]
             a = X if l == 0 else w["act"][l - 1]
-            gT = w["gT"][:o]
-            aT = w["aT"][:i]
-            _M.transpose_bf16(g.data_ptr(), g.stride(0), gT.data_ptr(), B, B, o, st)
-            _M.transpose_bf16(a.data_ptr(), a.stride(0), aT.data_ptr(), B, B, i, st)
-            self._gemm(gT, aT, self._view(self.grad, l, False))
+            # dW = g^T a over the batch rows, both operands as they lie
+            self._gemm(w, _STORE, g, a, self._view(self.grad, l, False), a_mn=True, b_mn=True)
             _M.colsum_bf16(g.data_ptr(), g.stride(0), B, o, self._view(self.grad, l, True).data_ptr(), st)
             if l > 0:
-                WT = w["WT"][:i, :o]
-                _M.transpose_bf16(self._wb(l).data_ptr(), i, WT.data_ptr(), WT.stride(0), o, i, st)
-                self._gemm(g, WT, w["da"])
-                _M.gelu_bwd(w["da"].data_ptr(), self.h, w["pre"][l - 1].data_ptr(), self.h, w["g"].data_ptr(),
-                            self.h, B, self.h, st)
-                g = w["g"]
+                # dx = g W times the activation's derivative (g and its
+                # successor are different buffers)
+                nxt = w["g"][(l - 1) % len(w["g"])]
+                self._gemm(w, _GELU_BWD, g, self._wb(l), w["pre"][l - 1], b_mn=True, act=nxt)
+                g = nxt
 
     def gradients(self, X, T, scale=None):
         """One forward + backward on a batch (X bf16, T fp32, rows a multiple
@@ -626,11 +635,15 @@ class LearnedStart:
 
     def launches_per_call(self, n_rows, sbus_rows=True):
         """Kernels of this library one ``start_voltages`` call launches: the
-        fused inputs, a GEMM and a bias/activation per layer and chunk, the
-        start voltages; without injection rows (``sbus_rows`` False) the
-        first layer's sparse product (per chunk) replaces the inputs and the
-        first GEMM."""
-        chunks = max(1, -(-_ceil(max(n_rows, 1), 128) // 16384))
-        if not sbus_rows and self.sparse_first_layer:
-            return (2 * self.net.layers + 2) * chunks + 1
-        return 2 * (self.net.layers + 1) * chunks + 2
+        inputs, a GEMM per layer and chunk (and the sum of its partial planes
+        where K is split), the start voltages; without injection rows
+        (``sbus_rows`` False) the first layer's sparse product and its
+        bias/activation (per chunk) replace the inputs and the first GEMM."""
+        sparse = not sbus_rows and self.sparse_first_layer
+        rows = _ceil(max(n_rows, 1), 128)
+        n = 1 if sparse else 2
+        for r0 in range(0, rows, 16384):
+            B = min(16384, rows - r0)
+            gemms = self.net.shapes[1:] if sparse else self.net.shapes
+            n += (2 if sparse else 0) + sum(2 if _M.gemm_part(B, o, i) else 1 for o, i in gemms)
+        return n

@@ -396,9 +396,21 @@ int gs2g_run_rows_noalloc(const gs2g_session* s, int n_rows, const double* v0, i
  * D[M x N] (fp32) = A[M x K] . B[N x K]^T (+ D when accumulate), A, B bf16,
  * on tcgen05 tensor cores.  M, N multiples of 128, K of 64; lda, ldb
  * multiples of 8, ldd of 4; 16-byte aligned bases.  *err is set to 1 if a
- * bounded wait inside the kernel ran out (the tile is then not written). */
+ * bounded wait inside the kernel ran out (D is then not valid). */
 int gs2g_mlp_gemm_tn_bf16(const void* A, int lda, const void* B, int ldb, float* D, int ldd, int M, int N, int K,
                           int accumulate, int* err, void* stream);
+/* The same product with either operand stored the other way round (a_mn: A is
+ * X[k][i], M contiguous; b_mn: B is X[k][j], N contiguous) and an operation on
+ * each finished sum v: op 0: D = v (+ D with accumulate); 1: D = v + bias[c];
+ * 2: z = v + bias[c], D = z unless D is NULL, act = bf16(gelu(z)); 3: act =
+ * bf16(v * gelu'(D)).  part (part_elems floats, NULL: none): room for the
+ * partial sums of a K split, which shapes with few tiles take when it holds
+ * gs2g_mlp_gemm_part(M, N, K) floats (0: the shape is not split).  Sizes,
+ * leading dimensions and alignment of A and B as above; D and act any ld >= N. */
+int64_t gs2g_mlp_gemm_part(int M, int N, int K);
+int gs2g_mlp_gemm(const void* A, int lda, int a_mn, const void* B, int ldb, int b_mn, int M, int N, int K, int op,
+                  int accumulate, float* D, int ldd, const float* bias, void* act_bf16, int ld_act, float* part,
+                  int64_t part_elems, int* err, void* stream);
 /* pre += bias (per column); act = bf16(gelu(pre)) (exact erf GELU) or
  * bf16(pre) when gelu = 0; act may be NULL. */
 int gs2g_mlp_bias_act(float* pre, int ldp, const float* bias, void* act_bf16, int lda, int rows, int cols, int gelu,

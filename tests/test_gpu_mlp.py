@@ -39,6 +39,46 @@ def test_gemm_tn_bf16_matches_fp64(M, N, K):
     assert np.abs(D.cpu().numpy() - 2 * ref).max() < 2 * tol
 
 
+@pytest.mark.parametrize("M,N,K,op", [(128, 128, 64, 0), (128, 384, 192, 2), (384, 640, 4096, 1), (256, 1024, 7232, 3),
+                                      (2944, 896, 128, 2), (1024, 3712, 1024, 0)])
+@pytest.mark.parametrize("a_mn", [False, True])
+@pytest.mark.parametrize("b_mn", [False, True])
+def test_gemm_layouts_and_epilogues_match_fp64(M, N, K, op, a_mn, b_mn):
+    """Both storage orders of each operand, every epilogue, one tile to many, a
+    half-empty last tile, with and without a K split."""
+    import torch
+    from gpusim2grid_b200._native import lib
+    g = torch.Generator().manual_seed(M + N + K + op)
+    r = lambda *s: torch.randn(*s, generator=g)
+    A, B = _bf16(r(M, K)).cuda(), _bf16(r(N, K)).cuda()
+    As, Bs = (A.t().contiguous() if a_mn else A), (B.t().contiguous() if b_mn else B)
+    bias, z0 = r(N).cuda(), r(M, N).cuda()
+    need = lib.mlp.gemm_part(M, N, K)
+    v = A.double() @ B.double().t()
+    tol = 1e-5 * np.sqrt(K) * float(v.abs().max()) + 1e-5  # exact products, fp32 sums of K terms of size ~1
+    gelu = torch.nn.functional.gelu
+    for part in ([None, torch.empty(need, device="cuda")] if need else [None]):
+        D = z0.clone() if op == 3 else torch.full((M, N), float("nan"), device="cuda")
+        act = torch.zeros(M, N, dtype=torch.bfloat16, device="cuda")
+        err = torch.zeros(1, dtype=torch.int32, device="cuda")
+        lib.mlp.gemm(As.data_ptr(), As.stride(0), a_mn, Bs.data_ptr(), Bs.stride(0), b_mn, M, N, K, op, False,
+                     D.data_ptr(), N, bias.data_ptr(), act.data_ptr(), N, part.data_ptr() if part is not None else 0,
+                     need if part is not None else 0, err.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        assert int(err.item()) == 0
+        z = v + bias.double() if op in (1, 2) else v
+        if op < 3:
+            assert float((D.double() - z).abs().max()) < tol
+        if op >= 2:
+            if op == 2:
+                want = gelu(z)
+            else:
+                zz = z0.double().requires_grad_(True)
+                want = torch.autograd.grad(gelu(zz), zz, v)[0]
+            # bf16 rounding of the result (2^-9 relative) on top of the sums'
+            assert bool(((act.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1.2 * tol).all())
+
+
 def test_gemm_rejects_bad_shapes():
     import torch
     from gpusim2grid_b200._native import lib
