@@ -20,7 +20,6 @@ __device__ __noinline__ void factor_at(const DevPlan& P, const SweepArgs& a, con
                                        double2* I, T* HV, T* S, T* s_dense, const unsigned* mbits, bool has_mask) {
   const int tid = threadIdx.x;
   const double2* Y = reinterpret_cast<const double2*>(a.ybus);
-  auto masked = [&](int b) { return has_mask && ((mbits[b >> 5] >> (b & 31)) & 1u); };
   for (int i = tid; i < P.n_bus; i += BS) {
     double2 acc = make_double2(0.0, 0.0);
     for (int k = P.y_indptr[i]; k < P.y_indptr[i + 1]; ++k) {
@@ -31,47 +30,14 @@ __device__ __noinline__ void factor_at(const DevPlan& P, const SweepArgs& a, con
     }
     I[i] = acc;
   }
-  {
-    const int64_t ns = (int64_t)P.nt * P.ld;
-    for (int64_t q = tid; q < ns; q += BS) S[q] = T(0);
-  }
   __syncthreads();
-  for (int k = tid; k < P.nnz_y; k += BS) {
-    const int i = P.y_row[k], j = P.y_indices[k];
-    double out[4];
-    jac_entry(i == j, ed.apply(k, Y[k]), V[i], V[j], I[i], out);
-    if (masked(i) || masked(j)) {
-      const double one = (i == j) ? 1.0 : 0.0;
-      out[0] = one;
-      out[1] = 0.0;
-      out[2] = 0.0;
-      out[3] = one;
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int dst = P.jmap[4 * k + q];
-      if (dst >= 0) HV[dst] = (T)out[q];
-      else if (dst <= -2) S[-(dst + 2)] = (T)out[q];
-    }
-  }
+  const unsigned* row_mask = has_mask ? mbits : nullptr;
+  fill_head<T>(P, ed, Y, V, I, row_mask, HV);
   __syncthreads();
-  for (int lv = 0; lv < P.n_levels; ++lv) {
-    const int t0 = P.lev_ptr[lv], t1 = P.lev_ptr[lv + 1];
-    for (int t = t0 + tid; t < t1; t += BS) {
-      const int out = P.task_out[t];
-      T acc = P.task_has_a[t] ? HV[out] : T(0);
-      for (int q = P.task_pbeg[t]; q < P.task_pend[t]; ++q) acc -= HV[P.pair_l[q]] * HV[P.pair_u[q]];
-      if (out < P.p) acc = clamp_pivot(acc, a.pivot_floor);
-      HV[out] = acc;
-    }
-    __syncthreads();
-    for (int t = t0 + tid; t < t1; t += BS) {
-      const int dg = P.task_diag[t];
-      if (dg >= 0) HV[P.task_out[t]] /= HV[dg];
-    }
-    __syncthreads();
-  }
-  schur_update<T>(P, HV, S);
+  head_lu<T>(P, HV, a.pivot_floor, 0, 1);
+  schur_update<T>(P, HV, S, s_dense);
+  __syncthreads();
+  fill_tail<T>(P, ed, Y, V, I, row_mask, S);
   __syncthreads();
   if (P.nt > 0) dense_lu<T>(S, P.nt, P.ld, s_dense, a.pivot_floor);
   __syncthreads();

@@ -23,7 +23,6 @@
 
 #include <type_traits>
 
-#include "dense_lu.cuh"
 #include "dense_lu_f32.cuh"
 #include "dense_lu_f64.cuh"
 
@@ -38,7 +37,7 @@ namespace {
 constexpr int BS = 256;        // threads per CTA
 constexpr int NWARP = BS / 32;
 constexpr int MAX_EDITS = 64;  // Ybus edits per row held in shared memory
-static_assert(BS == dense::BS, "the dense LU assumes the sweep's CTA size");
+static_assert(BS == dense32::BS && BS == dense64::BS, "the dense LUs assume the sweep's CTA size");
 
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -95,37 +94,39 @@ __device__ __forceinline__ T clamp_pivot(T piv, double floor_) {
   return piv;
 }
 
-// Contribution of one Schur entry (see Plan::se_rec): sum_{c<w} L[c] U[c t].
-// w <= 15 (1 or 2 here: supernodes are buses); the first two products are
-// loaded together.
-template <typename T>
-__device__ __forceinline__ T schur_entry(const T* __restrict__ HV, int4 rec) {
-  const T* Lr = HV + rec.x;
-  const T* Ub = HV + rec.y;
-  const int w = rec.z & 15, t = rec.z >> 4;
-  const T l0 = Lr[0], u0 = Ub[0];
-  const T l1 = w > 1 ? Lr[1] : T(0), u1 = w > 1 ? Ub[t] : T(0);
-  T acc = l0 * u0 + l1 * u1;
-  for (int c = 2; c < w; ++c) acc += Lr[c] * Ub[c * t];
-  return acc;
+// Barrier over every thread of every CTA of the cluster, ordering the
+// memory accesses before it (global and distributed shared) before those
+// after it.  Block-uniform calls only.
+__device__ __forceinline__ void cluster_barrier() {
+  __threadfence();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
 
-// Schur update of the dense tail: warp per tail row, lane per column group
-// (each lane sums every contribution to one entry S[ti][col] and writes it
-// once), four groups per lane in flight: their entry records are loaded
-// together, then their factor values.
+template <typename T>
+__host__ __device__ constexpr int dense_smem_elems() {
+  return sizeof(T) == 4 ? gs2g::dense32::Smem::elems : gs2g::dense64::Smem::elems;
+}
+
 // Sparse head LU, level by level, in place on the head factor values HV.
 // With parts > 1 the `parts` CTAs of a cluster (this one: rank `part`) split
 // each level's tasks and pass cluster barriers instead of block barriers;
 // a task's arithmetic does not depend on who runs it.
+// Bound by load latency: a task is three dependent loads (its record, a pair
+// of positions, the two factor values) and a handful of products.  So a
+// thread runs TU tasks side by side, QU products of each in flight with the
+// next QU pairs -- tasks of a level are sorted by length, so the loops of a
+// thread and of a warp's lanes end together -- and a task's record is one
+// 16-byte load, its pairs one 8-byte load each, consecutive over the lanes.
 template <typename T>
 __device__ __noinline__ void head_lu(const DevPlan P, T* HV, const double pfloor, const int part, const int parts) {
+  constexpr int TU = 2, QU = 4;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gwarp = part * NWARP + warp, nwarps = parts * NWARP;
   const int gtid = part * BS + tid, nthreads = parts * BS;
   auto barrier = [&]() {
     if (parts > 1)
-      dense::cluster_barrier();
+      cluster_barrier();
     else
       __syncthreads();
   };
@@ -133,66 +134,207 @@ __device__ __noinline__ void head_lu(const DevPlan P, T* HV, const double pfloor
     const int t0 = P.lev_ptr[lv], tb = P.lev_big[lv], t1 = P.lev_ptr[lv + 1];
     // long tasks: one warp each, products split over the lanes
     for (int t = t0 + gwarp; t < tb; t += nwarps) {
-      const int out = P.task_out[t];
-      const int q1 = P.task_pend[t];
+      const int4 r = P.task_rec[t];
       T acc_p = T(0);
-      for (int q = P.task_pbeg[t] + lane; q < q1; q += 32) acc_p += HV[P.pair_l[q]] * HV[P.pair_u[q]];
+      for (int q = lane; q < r.w; q += 32) {
+        const int2 pr = P.pairs[r.z + q];
+        acc_p += HV[pr.x] * HV[pr.y];
+      }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) acc_p += __shfl_xor_sync(0xffffffffu, acc_p, o);
       if (lane == 0) {
-        T acc = (P.task_has_a[t] ? HV[out] : T(0)) - acc_p;
-        if (out < P.p) acc = clamp_pivot(acc, pfloor);
-        HV[out] = acc;
+        T acc = (r.y ? HV[r.x] : T(0)) - acc_p;
+        if (r.x < P.p) acc = clamp_pivot(acc, pfloor);
+        HV[r.x] = acc;
       }
     }
-    for (int t = tb + gtid; t < t1; t += nthreads) {
-      const int out = P.task_out[t];
-      T acc = P.task_has_a[t] ? HV[out] : T(0);
-      const int q1 = P.task_pend[t];
-      for (int q = P.task_pbeg[t]; q < q1; ++q) acc -= HV[P.pair_l[q]] * HV[P.pair_u[q]];
-      if (out < P.p) acc = clamp_pivot(acc, pfloor);
-      HV[out] = acc;
+    for (int t = tb + gtid; t < t1; t += TU * nthreads) {
+      int4 r[TU];
+      T acc[TU];
+#pragma unroll
+      for (int u = 0; u < TU; ++u) {
+        const int tu = t + u * nthreads;
+        r[u] = tu < t1 ? P.task_rec[tu] : make_int4(-1, 0, 0, 0);
+      }
+      int2 pr[TU][QU];
+      auto load_pairs = [&](int q) {
+#pragma unroll
+        for (int u = 0; u < TU; ++u)
+#pragma unroll
+          for (int h = 0; h < QU; ++h)
+            pr[u][h] = q + h < r[u].w ? P.pairs[r[u].z + 32 * (q + h)] : make_int2(-1, 0);
+      };
+      load_pairs(0);
+#pragma unroll
+      for (int u = 0; u < TU; ++u) acc[u] = r[u].y ? HV[r[u].x] : T(0);
+      // the first task is the longest
+      for (int q = 0; q < r[0].w; q += QU) {
+        T l[TU][QU], x[TU][QU];
+#pragma unroll
+        for (int u = 0; u < TU; ++u)
+#pragma unroll
+          for (int h = 0; h < QU; ++h) {
+            l[u][h] = pr[u][h].x >= 0 ? HV[pr[u][h].x] : T(0);
+            x[u][h] = pr[u][h].x >= 0 ? HV[pr[u][h].y] : T(0);
+          }
+        load_pairs(q + QU);  // the next pairs travel with this step's values
+#pragma unroll
+        for (int u = 0; u < TU; ++u)
+#pragma unroll
+          for (int h = 0; h < QU; ++h) acc[u] -= l[u][h] * x[u][h];
+      }
+#pragma unroll
+      for (int u = 0; u < TU; ++u) {
+        if (r[u].x < 0) continue;
+        if (r[u].x < P.p) acc[u] = clamp_pivot(acc[u], pfloor);
+        HV[r[u].x] = acc[u];
+      }
     }
     barrier();
-    for (int t = t0 + gtid; t < t1; t += nthreads) {
-      const int dg = P.task_diag[t];
-      if (dg >= 0) HV[P.task_out[t]] /= HV[dg];
+    const int d1 = P.div_ptr[lv + 1];
+    for (int t = P.div_ptr[lv] + gtid; t < d1; t += TU * nthreads) {
+      int2 r[TU];
+      T x[TU], d[TU];
+#pragma unroll
+      for (int u = 0; u < TU; ++u) r[u] = t + u * nthreads < d1 ? P.div_rec[t + u * nthreads] : make_int2(-1, 0);
+#pragma unroll
+      for (int u = 0; u < TU; ++u) {
+        x[u] = r[u].x >= 0 ? HV[r[u].x] : T(0);
+        d[u] = r[u].x >= 0 ? HV[r[u].y] : T(1);
+      }
+#pragma unroll
+      for (int u = 0; u < TU; ++u)
+        if (r[u].x >= 0) HV[r[u].x] = x[u] / d[u];
     }
     barrier();
   }
 }
 
+// Schur update of the dense tail: S <- -(sum of the head's contributions),
+// whole rows (the tail's J coefficients are added afterwards, fill_tail).
+// Warp per tail row, the row's sum in shared memory (scratch: the dense LU's,
+// dense_smem_elems values, divided among the warps; a tail wider than a
+// warp's share takes several passes over the columns).  A chunk is up to 32
+// columns of one supernode: they differ, so the lanes add to the row without
+// conflicts, and its U values and columns are consecutive.  Bound by load
+// latency: 32 records and their L values come in two loads, and CU chunks'
+// columns and U values are in flight together (no branch between the loads).
+// The chunks are added in supernode order.  (One lane per target column,
+// summing the column's contributions one dependent load after another, left
+// the warp waiting for the row's diagonal entries, up to 43 of them.)
 template <typename T>
-__device__ __noinline__ void schur_update(const DevPlan P, const T* __restrict__ HV, T* __restrict__ S, int part = 0,
-                                          int parts = 1) {
+__device__ __noinline__ void schur_update(const DevPlan P, const T* __restrict__ HV, T* __restrict__ S,
+                                          T* __restrict__ scratch, int part = 0, int parts = 1) {
+  constexpr int CAP = dense_smem_elems<T>() / NWARP;
+  constexpr int CU = 8;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  T* acc = scratch + warp * CAP;
   // with parts > 1 the CTAs of a cluster take every parts-th warp's rows
   for (int ti = part * NWARP + warp; ti < P.nt; ti += parts * NWARP) {
     T* Srow = S + (int64_t)ti * P.ld;
-    const int g0 = P.sg_ptr[ti], g1 = P.sg_ptr[ti + 1];
-    for (int gb = g0; gb < g1; gb += 128) {
-      int ge[4], e0[4], e1[4];
+    const int c0 = P.sc_ptr[ti], c1 = P.sc_ptr[ti + 1];
+    for (int b0 = 0; b0 < P.ld; b0 += CAP) {
+      const int nb = min(CAP, P.ld - b0);
+      for (int i = lane; i < nb; i += 32) acc[i] = T(0);
+      __syncwarp();
+      for (int c = c0; c < c1; c += 32) {
+        const int4 mine = c + lane < c1 ? P.sc_rec[c + lane] : make_int4(0, 0, 0, 0);
+        const T ml0 = HV[mine.x], ml1 = (mine.w & 1) ? HV[mine.x + 1] : T(0);
+        const int cnt = min(32, c1 - c);
+        for (int j = 0; j < cnt; j += CU) {
+          int col[CU];
+          T u0[CU], u1[CU];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        ge[u] = gb + lane + 32 * u;
-        const bool in = ge[u] < g1;
-        e0[u] = in ? P.se_ptr[ge[u]] : 0;
-        e1[u] = in ? P.se_ptr[ge[u] + 1] : 0;
+          for (int u = 0; u < CU; ++u) {
+            const int y = __shfl_sync(0xffffffffu, mine.y, j + u) + lane;
+            const int z = __shfl_sync(0xffffffffu, mine.z, j + u) + lane;
+            const int f = __shfl_sync(0xffffffffu, mine.w, j + u);
+            const bool in = lane < ((f >> 1) & 63);
+            col[u] = in ? P.tidx[z] : -1;
+            u0[u] = in ? HV[y] : T(0);
+            u1[u] = in && (f & 1) ? HV[y + (f >> 7)] : T(0);
+          }
+#pragma unroll
+          for (int u = 0; u < CU; ++u) {
+            const T l0 = __shfl_sync(0xffffffffu, ml0, j + u), l1 = __shfl_sync(0xffffffffu, ml1, j + u);
+            if (col[u] >= b0 && col[u] < b0 + nb) acc[col[u] - b0] += l0 * u0[u] + l1 * u1[u];
+            __syncwarp();
+          }
+        }
       }
-      T acc[4] = {T(0), T(0), T(0), T(0)};
-      // first entry of each group (nearly every group has one or two)
-      int4 rec[4];
+      for (int i = lane; i < nb; i += 32) Srow[b0 + i] = T(0) - acc[i];
+      __syncwarp();
+    }
+  }
+}
+
+// One Jacobian entry pair of Ybus entry (i, j) with value yk at voltages
+// Vi, Vj and current Ii (the J-fill formulas): out = {dP/dtheta_j,
+// dP/dVm_j, dQ/dtheta_j, dQ/dVm_j}.
+__device__ __forceinline__ void jac_entry(bool diag, double2 yk, double2 Vi, double2 Vj, double2 Ii, double out[4]) {
+  double2 dVa, dVm;
+  if (diag) {
+    const double2 t = cmul(Vi, conj2(csub(Ii, cmul(yk, Vi))));
+    dVa = make_double2(-t.y, t.x);
+    const double inv = 1.0 / hypot(Vi.x, Vi.y);
+    const double2 vn = make_double2(Vi.x * inv, Vi.y * inv);
+    dVm = cadd(cmul(Vi, conj2(cmul(yk, vn))), cmul(conj2(Ii), vn));
+  } else {
+    const double2 t = cmul(Vi, conj2(cmul(yk, Vj)));
+    dVa = make_double2(t.y, -t.x);
+    const double inv = 1.0 / hypot(Vj.x, Vj.y);
+    const double2 vn = make_double2(Vj.x * inv, Vj.y * inv);
+    dVm = cmul(Vi, conj2(cmul(yk, vn)));
+  }
+  out[0] = dVa.x;
+  out[1] = dVm.x;
+  out[2] = dVa.y;
+  out[3] = dVm.y;
+}
+
+// The J coefficients of Ybus entry k of a row (its voltages V, currents I and
+// edits; mbits: the row's masked buses or nullptr): a masked bus's rows are
+// identity rows, and live rows see no coupling to it.
+__device__ __forceinline__ void row_jac(const DevPlan& P, const RowEdits& ed, const double2* Y, const double2* V,
+                                        const double2* I, const unsigned* mbits, int k, double out[4]) {
+  const int i = P.y_row[k], j = P.y_indices[k];
+  jac_entry(i == j, ed.apply(k, Y[k]), V[i], V[j], I[i], out);
+  if (mbits != nullptr && (((mbits[i >> 5] >> (i & 31)) | (mbits[j >> 5] >> (j & 31))) & 1u)) {
+    const double one = (i == j) ? 1.0 : 0.0;
+    out[0] = one;
+    out[1] = 0.0;
+    out[2] = 0.0;
+    out[3] = one;
+  }
+}
+
+// Scatter J's head coefficients into HV.
+template <typename T>
+__device__ __forceinline__ void fill_head(const DevPlan& P, const RowEdits& ed, const double2* Y, const double2* V,
+                                          const double2* I, const unsigned* mbits, T* HV) {
+  for (int k = threadIdx.x; k < P.nnz_y; k += BS) {
+    double out[4];
+    row_jac(P, ed, Y, V, I, mbits, k, out);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) rec[u] = e0[u] < e1[u] ? P.se_rec[e0[u]] : make_int4(0, 0, 0, 0);
+    for (int q = 0; q < 4; ++q) {
+      const int dst = P.jmap[4 * k + q];
+      if (dst >= 0) HV[dst] = (T)out[q];
+    }
+  }
+}
+
+// Add J's tail coefficients to the Schur update's rows (each S entry has one).
+template <typename T>
+__device__ __forceinline__ void fill_tail(const DevPlan& P, const RowEdits& ed, const double2* Y, const double2* V,
+                                          const double2* I, const unsigned* mbits, T* S) {
+  for (int e = threadIdx.x; e < P.n_y_tail; e += BS) {
+    const int k = P.y_tail[e];
+    double out[4];
+    row_jac(P, ed, Y, V, I, mbits, k, out);
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (e0[u] < e1[u]) acc[u] = schur_entry<T>(HV, rec[u]);
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        for (int e = e0[u] + 1; e < e1[u]; ++e) acc[u] += schur_entry<T>(HV, P.se_rec[e]);
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (ge[u] < g1) Srow[P.sg_col[ge[u]]] -= acc[u];
+    for (int q = 0; q < 4; ++q) {
+      const int dst = P.jmap[4 * k + q];
+      if (dst <= -2) S[-(dst + 2)] += (T)out[q];
     }
   }
 }
@@ -207,21 +349,15 @@ __device__ __forceinline__ double step_alpha(double mdt, double mdv, double max_
   return alpha;
 }
 
-// Dense tail LU: FP32 on the SIMT kernel of dense_lu_f32.cuh, FP64 on its
-// FP64 counterpart (dense_lu_f64.cuh; GS2G_FP64_LU=0 selects the older
-// DMMA-tile LU of dense_lu.cuh); all use the dynamic shared memory as
-// scratch.
-#ifndef GS2G_FP64_LU
-#define GS2G_FP64_LU 1
-#endif
+// Dense tail LU: FP32 on the SIMT kernel of dense_lu_f32.cuh, FP64 on the
+// tensor-pipe kernel of dense_lu_f64.cuh; both use the dynamic shared memory
+// as scratch.
 template <typename T>
 __device__ __forceinline__ void dense_lu(T* S, int n, int ld, T* smem, double pfloor) {
   if constexpr (sizeof(T) == 4)
     gs2g::dense32::lu(S, n, ld, smem, pfloor);
-  else if constexpr (GS2G_FP64_LU == 1)
-    gs2g::dense64::lu(S, n, ld, smem, pfloor);
   else
-    dense::lu<T>(S, n, ld, smem, pfloor);
+    gs2g::dense64::lu(S, n, ld, smem, pfloor);
 }
 // The same factorization by the `parts` CTAs of a cluster (this CTA: rank
 // `part`), bit-identical to dense_lu.
@@ -229,15 +365,8 @@ template <typename T>
 __device__ __forceinline__ void dense_lu_cluster(T* S, int n, int ld, T* smem, double pfloor, int part, int parts) {
   if constexpr (sizeof(T) == 4)
     gs2g::dense32::lu_cluster(S, n, ld, smem, pfloor, part, parts);
-  else if constexpr (GS2G_FP64_LU == 1)
-    gs2g::dense64::lu_cluster(S, n, ld, smem, pfloor, part, parts);
   else
-    dense::lu_cluster(S, n, ld, smem, pfloor, part, parts);
-}
-static_assert(gs2g::dense64::Smem::elems <= dense::Smem<double>::elems, "FP64 LU scratch within the FP64 smem");
-template <typename T>
-__host__ __device__ constexpr int dense_smem_elems() {
-  return sizeof(T) == 4 ? gs2g::dense32::Smem::elems : dense::Smem<T>::elems;
+    gs2g::dense64::lu_cluster(S, n, ld, smem, pfloor, part, parts);
 }
 
 // Staging for the dense solves: warp 0 copies a 32 x 64 tile of the factor
@@ -632,30 +761,6 @@ struct RowShared {
   int* s_cpiv;    // [MAX_COMP]
   double* s_cw;   // [MAX_COMP]
 };
-
-// One Jacobian entry pair of Ybus entry (i, j) with value yk at voltages
-// Vi, Vj and current Ii (the J-fill formulas): out = {dP/dtheta_j,
-// dP/dVm_j, dQ/dtheta_j, dQ/dVm_j}.
-__device__ __forceinline__ void jac_entry(bool diag, double2 yk, double2 Vi, double2 Vj, double2 Ii, double out[4]) {
-  double2 dVa, dVm;
-  if (diag) {
-    const double2 t = cmul(Vi, conj2(csub(Ii, cmul(yk, Vi))));
-    dVa = make_double2(-t.y, t.x);
-    const double inv = 1.0 / hypot(Vi.x, Vi.y);
-    const double2 vn = make_double2(Vi.x * inv, Vi.y * inv);
-    dVm = cadd(cmul(Vi, conj2(cmul(yk, vn))), cmul(conj2(Ii), vn));
-  } else {
-    const double2 t = cmul(Vi, conj2(cmul(yk, Vj)));
-    dVa = make_double2(t.y, -t.x);
-    const double inv = 1.0 / hypot(Vj.x, Vj.y);
-    const double2 vn = make_double2(Vj.x * inv, Vj.y * inv);
-    dVm = cmul(Vi, conj2(cmul(yk, vn)));
-  }
-  out[0] = dVa.x;
-  out[1] = dVm.x;
-  out[2] = dVa.y;
-  out[3] = dVm.y;
-}
 
 // ||F||inf of the row (row-patched Ybus, its Sbus) at voltage Vx, NaN-sticky,
 // without touching the row's workspace
@@ -1219,47 +1324,9 @@ __device__ __forceinline__ void solve_row(const DevPlan& P, const SweepArgs& a, 
         have_factor = true;
         since_factor = 0;
         ++n_factor;
-      // ---- zero the dense tail, then scatter J ------------------------------
-      {
-        const int64_t ns = (int64_t)P.nt * P.ld;
-        for (int64_t q = tid; q < ns; q += BS) S[q] = T(0);
-      }
-      __syncthreads();
-      for (int k = tid; k < P.nnz_y; k += BS) {
-        const int i = P.y_row[k], j = P.y_indices[k];
-        const double2 Vi = V[i], Ii = I[i];
-        const double2 yk = ed.apply(k, Y[k]);
-        double2 dVa, dVm;
-        if (i == j) {
-          const double2 t = cmul(Vi, conj2(csub(Ii, cmul(yk, Vi))));
-          dVa = make_double2(-t.y, t.x);
-          const double inv = 1.0 / hypot(Vi.x, Vi.y);
-          const double2 vn = make_double2(Vi.x * inv, Vi.y * inv);
-          dVm = cadd(cmul(Vi, conj2(cmul(yk, vn))), cmul(conj2(Ii), vn));
-        } else {
-          const double2 Vj = V[j];
-          const double2 t = cmul(Vi, conj2(cmul(yk, Vj)));
-          dVa = make_double2(t.y, -t.x);
-          const double inv = 1.0 / hypot(Vj.x, Vj.y);
-          const double2 vn = make_double2(Vj.x * inv, Vj.y * inv);
-          dVm = cmul(Vi, conj2(cmul(yk, vn)));
-        }
-        double vals[4] = {dVa.x, dVm.x, dVa.y, dVm.y};
-        if (masked(i) || masked(j)) {
-          // a masked bus's rows are identity rows; live rows see no coupling to it
-          const double one = (i == j) ? 1.0 : 0.0;
-          vals[0] = one;
-          vals[1] = 0.0;
-          vals[2] = 0.0;
-          vals[3] = one;
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int dst = P.jmap[4 * k + q];
-          if (dst >= 0) HV[dst] = (T)vals[q];
-          else if (dst <= -2) S[-(dst + 2)] = (T)vals[q];
-        }
-      }
+      // ---- scatter J's head coefficients ------------------------------------
+      const unsigned* row_mask = has_mask ? mbits : nullptr;
+      fill_head<T>(P, ed, Y, V, I, row_mask, HV);
       __syncthreads();
 
       prof.mark(PH_FILL);
@@ -1270,8 +1337,8 @@ __device__ __forceinline__ void solve_row(const DevPlan& P, const SweepArgs& a, 
         // (posted; read by all); the head factor's values and the scattered
         // tail are complete before the first of them
         if (tid == 0) *cl->cmd = CLUSTER_CMD_LU;
-        dense::cluster_barrier();
-        dense::cluster_barrier();
+        cluster_barrier();
+        cluster_barrier();
       }
       head_lu<T>(P, HV, a.pivot_floor, 0, shared_factor ? cl->parts : 1);
 
@@ -1279,13 +1346,17 @@ __device__ __forceinline__ void solve_row(const DevPlan& P, const SweepArgs& a, 
       if (shared_factor) {
         // the Schur update split by tail rows (a barrier), then the shared
         // dense factorization
-        schur_update<T>(P, HV, S, 0, cl->parts);
-        dense::cluster_barrier();
+        schur_update<T>(P, HV, S, s_dense, 0, cl->parts);
+        cluster_barrier();
+        fill_tail<T>(P, ed, Y, V, I, row_mask, S);
+        cluster_barrier();
         prof.mark(PH_SCHUR);
         dense_lu_cluster<T>(S, P.nt, P.ld, s_dense, a.pivot_floor, 0, cl->parts);
       } else {
       // ---- Schur update of the dense tail ----------------------------------
-      schur_update<T>(P, HV, S);
+      schur_update<T>(P, HV, S, s_dense);
+      __syncthreads();
+      fill_tail<T>(P, ed, Y, V, I, row_mask, S);
       __syncthreads();
 
       prof.mark(PH_SCHUR);
@@ -1437,7 +1508,8 @@ __device__ __forceinline__ int ld_shared_rank0(const int* p) {
 // CTA reads it (barrier); then for each factorization the leader posts
 // CLUSTER_CMD_LU (barrier, read, barrier) once the Jacobian is scattered,
 // and all run the head LU (two barriers per level), their Schur rows
-// (barrier) and the dense LU together; after the row it posts
+// (barrier; the leader adds J's tail coefficients; barrier) and the dense LU
+// together; after the row it posts
 // CLUSTER_CMD_DONE (barrier, read, barrier).
 // Largest cluster a row gets (16 needs the non-portable cluster-size opt-in;
 // the launch picks 16 or 8 by the number of rows, see launch_sweep_cluster).
@@ -1496,27 +1568,28 @@ __global__ void __launch_bounds__(BS, GS2G_MIN_CTAS_PER_SM)
   const ClusterLu cl{&s_cmd, parts};
   for (;;) {
     if (rank == 0 && threadIdx.x == 0) s_row = atomicAdd(a.queue, 1);
-    dense::cluster_barrier();
+    cluster_barrier();
     const int q = ld_shared_rank0(&s_row);
-    dense::cluster_barrier();
+    cluster_barrier();
     if (q >= n_rows) break;
     if (rank == 0) {
       solve_row<T>(P, a, a.row_map != nullptr ? a.row_map[q] : q, ws, sh, prof, &cl);
       if (threadIdx.x == 0) s_cmd = CLUSTER_CMD_DONE;
-      dense::cluster_barrier();
-      dense::cluster_barrier();
+      cluster_barrier();
+      cluster_barrier();
     } else {
       for (;;) {
-        dense::cluster_barrier();
+        cluster_barrier();
         const int cmd = ld_shared_rank0(&s_cmd);
-        dense::cluster_barrier();
+        cluster_barrier();
         if (cmd != CLUSTER_CMD_LU) break;
         // the leader's Jacobian values are in place (posted after them): the
-        // head LU's share of each level, the Schur rows, a barrier, then the
-        // shared dense LU
+        // head LU's share of each level, the Schur rows, two barriers (rows
+        // complete, J's tail coefficients added), then the shared dense LU
         head_lu<T>(P, HV, a.pivot_floor, rank, parts);
-        schur_update<T>(P, HV, S, rank, parts);
-        dense::cluster_barrier();
+        schur_update<T>(P, HV, S, reinterpret_cast<T*>(smem_raw), rank, parts);
+        cluster_barrier();
+        cluster_barrier();  // the leader has added J's tail coefficients
         dense_lu_cluster<T>(S, P.nt, P.ld, reinterpret_cast<T*>(smem_raw), a.pivot_floor, rank, parts);
       }
     }
@@ -1589,7 +1662,7 @@ __global__ void __launch_bounds__(BS, GS2G_MIN_CTAS_PER_SM)
 
 template <typename T>
 int smem_bytes() {
-  return sizeof(T) == 4 ? gs2g::dense32::Smem::bytes : dense::Smem<T>::bytes;
+  return sizeof(T) == 4 ? gs2g::dense32::Smem::bytes : gs2g::dense64::Smem::bytes;
 }
 
 }  // namespace

@@ -13,34 +13,25 @@ enum RowStatusCode : int { ROW_CONVERGED = 0, ROW_MAX_ITER = 1, ROW_DIVERGED = 2
 
 // Device copy of a Plan (see plan.hpp); every pointer is device memory.
 struct DevPlan {
-  int n_bus, nnz_y, dim, p, nt, ld, n_hv, n_levels;
+  int n_bus, nnz_y, dim, p, nt, ld, n_hv, n_levels, n_y_tail;
   const int* y_indptr;
   const int* y_indices;
   const int* y_row;
   const int* jmap;     // [4 * nnz_y]
+  const int* y_tail;   // [n_y_tail] Ybus entries with a coefficient in the dense tail
   const int* fP;       // [n_bus]
   const int* fQ;       // [n_bus]
   const int* lev_ptr;  // [n_levels + 1] into tasks
   const int* lev_big;  // [n_levels]: tasks [lev_ptr[l], lev_big[l]) are long (warp per task)
-  const int* task_out;
-  const int* task_diag;
-  const int* task_pbeg;
-  const int* task_pend;
-  const uint8_t* task_has_a;
-  const int* pair_l;
-  const int* pair_u;
+  const int4* task_rec;  // per task: out, has_a, first product, products (see plan.hpp)
+  const int2* pairs;     // (l, u) HV positions of the products
+  const int* div_ptr;    // [n_levels + 1] into div_rec
+  const int2* div_rec;   // L entries by level: HV position, HV position of its pivot
   const int* lev_piv_ptr;  // [n_levels + 1] into lev_piv
   const int* lev_piv;      // head pivots by level
-  const int* sn_w;
-  const int* sn_t;
-  const int* sn_L;
-  const int* sn_U;
-  const int* sn_tidx;
-  const int* tidx;
-  const int* sg_ptr;  // [nt + 1] Schur column groups per tail row
-  const int* sg_col;  // tail column of each group
-  const int* se_ptr;  // [groups + 1] entries per group
-  const int4* se_rec;  // per entry: HV offset of its L values, of its first U value, w | t << 4 (U stride t)
+  const int* tidx;     // tail columns of the Schur chunks
+  const int* sc_ptr;   // [nt + 1] Schur chunks per tail row
+  const int4* sc_rec;  // per chunk: L position, U position, offset into tidx, h | n << 1 | t << 7
   const int* fw_ptr;  // [dim + 1]
   const int* fw_col;
   const int* fw_pos;

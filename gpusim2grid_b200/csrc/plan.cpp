@@ -429,24 +429,31 @@ Plan build_plan(int n_bus, const int* ybus_indptr, const int* ybus_indices,
     for (int k : by_level[lv]) P.lev_piv.push_back(k);
     P.lev_piv_ptr.push_back((int)P.lev_piv.size());
   }
-  auto add_task = [&](int out, bool has_a, int diag) {
-    P.task_out.push_back(out);
-    P.task_has_a.push_back(has_a ? 1 : 0);
-    P.task_diag.push_back(diag);
-    P.task_pbeg.push_back((int)P.pair_l.size());
+  struct Task {
+    int out, has_a, diag, beg, end;
   };
-  auto end_task = [&]() { P.task_pend.push_back((int)P.pair_l.size()); };
+  std::vector<Task> tasks;              // of one level
+  std::vector<std::pair<int, int>> prod;  // their products
+  P.div_ptr.assign(1, 0);
+  auto add_task = [&](int out, bool has_a, int diag) {
+    tasks.push_back({out, has_a ? 1 : 0, diag, (int)prod.size(), 0});
+  };
+  auto end_task = [&]() { tasks.back().end = (int)prod.size(); };
+  std::vector<int> mi, mk;
   for (int lv = 0; lv < P.n_levels; ++lv) {
+    tasks.clear();
+    prod.clear();
     for (int k : by_level[lv]) {
       // u_kk
       add_task(k, jnz(k, k), -1);
-      for (int h = rptr[k]; h < rptr[k + 1]; ++h) { P.pair_l.push_back(rL[h]); P.pair_u.push_back(rU[h]); }
+      for (int h = rptr[k]; h < rptr[k + 1]; ++h) prod.emplace_back(rL[h], rU[h]);
       end_task();
       for (size_t q = 0; q < vst[k].size(); ++q) {
         int i = vst[k][q];
         // merge S(i) and S(k) (both sorted, all < k for S(k); S(i) may hold k itself, skip m >= k)
         int a = rptr[i], ae = rptr[i + 1], b = rptr[k], be = rptr[k + 1];
-        std::vector<int> mi, mk;
+        mi.clear();
+        mk.clear();
         while (a < ae && b < be) {
           int ma = rcol[a], mb = rcol[b];
           if (ma >= k) break;
@@ -456,42 +463,47 @@ Plan build_plan(int n_bus, const int* ybus_indptr, const int* ybus_indices,
         }
         // L entry l_ik
         add_task(posL(i, k, (int)q), jnz(i, k), k);
-        for (size_t z = 0; z < mi.size(); ++z) { P.pair_l.push_back(rL[mi[z]]); P.pair_u.push_back(rU[mk[z]]); }
+        for (size_t z = 0; z < mi.size(); ++z) prod.emplace_back(rL[mi[z]], rU[mk[z]]);
         end_task();
         // U entry u_ki
         add_task(posU(k, i, (int)q), jnz(k, i), -1);
-        for (size_t z = 0; z < mi.size(); ++z) { P.pair_l.push_back(rL[mk[z]]); P.pair_u.push_back(rU[mi[z]]); }
+        for (size_t z = 0; z < mi.size(); ++z) prod.emplace_back(rL[mk[z]], rU[mi[z]]);
         end_task();
       }
     }
-    // long tasks first (a warp each on the device), longest first
-    {
-      const int t0 = P.lev_ptr.back(), t1 = (int)P.task_out.size();
-      std::vector<int> idx(t1 - t0);
-      std::iota(idx.begin(), idx.end(), t0);
-      auto len = [&](int t) { return P.task_pend[t] - P.task_pbeg[t]; };
-      std::stable_sort(idx.begin(), idx.end(), [&](int a, int b) {
-        const bool ba = len(a) >= Plan::kBigTask, bb = len(b) >= Plan::kBigTask;
-        if (ba != bb) return ba;
-        return ba ? len(a) > len(b) : false;
-      });
-      auto permute = [&](auto& v) {
-        auto tmp = v;
-        for (int q = 0; q < t1 - t0; ++q) v[t0 + q] = tmp[idx[q]];
-      };
-      permute(P.task_out);
-      permute(P.task_diag);
-      permute(P.task_pbeg);
-      permute(P.task_pend);
-      permute(P.task_has_a);
-      int nbig = 0;
-      for (int t = t0; t < t1; ++t)
-        if (len(t) >= Plan::kBigTask) ++nbig;
-      P.lev_big.push_back(t0 + nbig);
+    // longest first: the long ones (a warp each on the device), then the rest
+    // in slices of 32 of nearly equal length
+    std::stable_sort(tasks.begin(), tasks.end(),
+                     [](const Task& x, const Task& y) { return x.end - x.beg > y.end - y.beg; });
+    const int nt_lv = (int)tasks.size();
+    int nbig = 0;
+    while (nbig < nt_lv && tasks[nbig].end - tasks[nbig].beg >= Plan::kBigTask) ++nbig;
+    auto put = [&](const Task& t, int first) {
+      P.task_rec.insert(P.task_rec.end(), {t.out, t.has_a, first, t.end - t.beg});
+      if (t.diag >= 0) P.div_rec.insert(P.div_rec.end(), {t.out, t.diag});
+    };
+    for (int t = 0; t < nbig; ++t) {
+      put(tasks[t], (int)P.pairs.size() / 2);
+      for (int z = tasks[t].beg; z < tasks[t].end; ++z)
+        P.pairs.insert(P.pairs.end(), {prod[z].first, prod[z].second});
     }
-    P.lev_ptr.push_back((int)P.task_out.size());
+    for (int t0s = nbig; t0s < nt_lv; t0s += 32) {
+      const int first = (int)P.pairs.size() / 2, len = tasks[t0s].end - tasks[t0s].beg;
+      P.pairs.resize(P.pairs.size() + size_t(64) * len, 0);
+      for (int t = t0s; t < std::min(nt_lv, t0s + 32); ++t) {
+        put(tasks[t], first + (t - t0s));
+        for (int z = tasks[t].beg; z < tasks[t].end; ++z) {
+          int* pr = &P.pairs[2 * (size_t(first) + (t - t0s) + size_t(32) * (z - tasks[t].beg))];
+          pr[0] = prod[z].first;
+          pr[1] = prod[z].second;
+        }
+      }
+    }
+    P.head_madds += (int64_t)prod.size();
+    P.lev_big.push_back(P.lev_ptr.back() + nbig);
+    P.lev_ptr.push_back((int)P.task_rec.size() / 4);
+    P.div_ptr.push_back((int)P.div_rec.size() / 2);
   }
-  P.head_madds = (int64_t)P.pair_l.size();
 
   // ---- Schur items per tail row ----------------------------------------
   P.schur_ptr.assign(P.nt + 1, 0);
@@ -515,43 +527,18 @@ Plan build_plan(int n_bus, const int* ybus_indptr, const int* ybus_indices,
     }
     P.schur_ptr[ti + 1] = (int)P.schur_sn.size();
   }
-  // column groups of the Schur update (see plan.hpp)
-  {
-    struct Ent {
-      int col, L, U, wt, ord;
-    };
-    std::vector<Ent> ents;
-    P.sg_ptr.assign(P.nt + 1, 0);
-    P.se_ptr.assign(1, 0);
-    for (int ti = 0; ti < P.nt; ++ti) {
-      ents.clear();
-      for (int q = P.schur_ptr[ti]; q < P.schur_ptr[ti + 1]; ++q) {
-        const int s = P.schur_sn[q], a = P.schur_a[q], w = P.sn_w[s], t = P.sn_t[s];
-        if (w >= 16 || t >= (1 << 27)) throw std::logic_error("build_plan: supernode too large for the Schur map");
-        for (int b = 0; b < t; ++b)
-          ents.push_back({P.tidx[P.sn_tidx[s] + b], P.sn_L[s] + a * w, P.sn_U[s] + b, w | (t << 4), (int)ents.size()});
-      }
-      std::sort(ents.begin(), ents.end(),
-                [](const Ent& x, const Ent& y) { return x.col != y.col ? x.col < y.col : x.ord < y.ord; });
-      for (size_t e = 0; e < ents.size(); ++e) {
-        if (e == 0 || ents[e].col != ents[e - 1].col) {
-          if (e > 0) P.se_ptr.push_back((int)P.se_L.size());
-          P.sg_col.push_back(ents[e].col);
-        }
-        P.se_L.push_back(ents[e].L);
-        P.se_U.push_back(ents[e].U);
-        P.se_wt.push_back(ents[e].wt);
-      }
-      if (!ents.empty()) P.se_ptr.push_back((int)P.se_L.size());
-      P.sg_ptr[ti + 1] = (int)P.sg_col.size();
+  // column chunks of the Schur update (see plan.hpp)
+  P.sc_ptr.assign(P.nt + 1, 0);
+  for (int ti = 0; ti < P.nt; ++ti) {
+    for (int q = P.schur_ptr[ti]; q < P.schur_ptr[ti + 1]; ++q) {
+      const int s = P.schur_sn[q], a = P.schur_a[q], w = P.sn_w[s], t = P.sn_t[s];
+      if (t >= (1 << 22)) throw std::logic_error("build_plan: supernode too large for the Schur map");
+      for (int k = 0; k < w; k += 2)
+        for (int b = 0; b < t; b += 32)
+          P.sc_rec.insert(P.sc_rec.end(), {P.sn_L[s] + a * w + k, P.sn_U[s] + k * t + b, P.sn_tidx[s] + b,
+                                           (k + 1 < w ? 1 : 0) | (std::min(32, t - b) << 1) | (t << 7)});
     }
-    P.se_rec.resize(4 * P.se_L.size());
-    for (size_t e = 0; e < P.se_L.size(); ++e) {
-      P.se_rec[4 * e] = P.se_L[e];
-      P.se_rec[4 * e + 1] = P.se_U[e];
-      P.se_rec[4 * e + 2] = P.se_wt[e];
-      P.se_rec[4 * e + 3] = 0;
-    }
+    P.sc_ptr[ti + 1] = (int)P.sc_rec.size() / 4;
   }
   for (int64_t k = 0; k < P.nt; ++k) P.dense_madds += (P.nt - 1 - k) * (P.nt - 1 - k);
 
@@ -625,6 +612,8 @@ Plan build_plan(int n_bus, const int* ybus_indptr, const int* ybus_indices,
         P.nnz_j++;
       }
   }
+  for (int k = 0; k < P.nnz_y; ++k)
+    if (*std::min_element(&P.jmap[size_t(4) * k], &P.jmap[size_t(4) * k] + 4) <= -2) P.y_tail.push_back(k);
   int64_t nl = 0;
   for (int c = 0; c < p; ++c) nl += (int64_t)vst[c].size();
   nl += (int64_t)P.nt * (P.nt - 1) / 2;

@@ -63,16 +63,23 @@ struct Plan {
   int n_levels = 0;
   std::vector<int> lev_ptr;
   // within level l, tasks [lev_ptr[l], lev_big[l]) have at least kBigTask
-  // products (one warp each on the device), the rest one thread each
+  // products (one warp each on the device), the rest one thread each, longest
+  // first
   std::vector<int> lev_big;
   static constexpr int kBigTask = 24;
   // head pivots by level (for the level-scheduled triangular solves)
   std::vector<int> lev_piv_ptr, lev_piv;
-  // head tasks: out position in HV; has_a flag; diag position for L entries
-  // (divide after accumulation) or -1; pair range.
-  std::vector<int> task_out, task_diag, task_pbeg, task_pend;
-  std::vector<uint8_t> task_has_a;
-  std::vector<int> pair_l, pair_u;  // HV positions of l and u in each product
+  // head tasks: [4 * tasks] (out position in HV, 1 when the entry starts from
+  // a J coefficient and 0 when it is fill, first product, products).  Products
+  // are (l, u) pairs of HV positions in pairs[2 * q]: a long task's are q = first,
+  // first + 1, ...; the short tasks of a level are taken in slices of 32 and
+  // their products lie transposed, q = first + 32 * j (padded to the slice's
+  // longest task), so that the lanes of a warp read consecutive pairs.
+  std::vector<int> task_rec;
+  std::vector<int> pairs;
+  // L entries of level l, [div_ptr[l], div_ptr[l+1]): (HV position, HV position
+  // of the pivot that divides it), two ints each
+  std::vector<int> div_ptr, div_rec;
   int64_t head_madds = 0;
 
   // head supernodes (for the tail blocks and the Schur update)
@@ -81,13 +88,13 @@ struct Plan {
   std::vector<int> tidx;  // tail-local row index of every tail row of every supernode
   // Schur items per tail row: [schur_ptr[ti], schur_ptr[ti+1]) of (sn, a)
   std::vector<int> schur_ptr, schur_sn, schur_a;
-  // The same update as column groups, the form the device runs: tail row ti
-  // owns groups [sg_ptr[ti], sg_ptr[ti+1]); group g updates S[ti][sg_col[g]]
-  // with the sum over entries [se_ptr[g], se_ptr[g+1]) of
-  //   sum_{c < w} HV[se_L[e] + c] * HV[se_U[e] + c * t],  w | t << 4 = se_wt[e]
-  // (entries of a group in supernode order).
-  std::vector<int> sg_ptr, sg_col, se_ptr, se_L, se_U, se_wt;
-  std::vector<int> se_rec;  // [4 * entries]: (se_L, se_U, se_wt, 0) packed for one 16-byte load
+  // The same update as chunks of up to 32 columns of one or two columns of a
+  // supernode, the form the device runs: row ti owns chunks [sc_ptr[ti],
+  // sc_ptr[ti+1]), in supernode order; chunk c (four ints at sc_rec[4 c]: L
+  // position x, U position y, offset z into tidx, h | n << 1 | t << 7)
+  // subtracts from S[ti][tidx[z + b]], b < n,
+  //   HV[x] * HV[y + b] + (h ? HV[x + 1] * HV[y + t + b] : 0).
+  std::vector<int> sc_ptr, sc_rec;
   int64_t schur_madds = 0, schur_volume = 0;
   int64_t dense_madds = 0;
 
@@ -108,6 +115,7 @@ struct Plan {
   // per Ybus entry k: destinations of its J11 (P-θ), J12 (P-Vm), J21 (Q-θ),
   // J22 (Q-Vm) coefficients, encoded as described above.
   std::vector<int> jmap;  // [4 * nnz_y]
+  std::vector<int> y_tail;  // Ybus entries with a coefficient in the dense tail
 
   // ---- statistics --------------------------------------------------------
   int64_t nnz_j = 0, nnz_lu = 0;

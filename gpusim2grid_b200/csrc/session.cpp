@@ -188,29 +188,21 @@ void upload_plan(gs2g_session* s) {
   D.y_indices = upload_vec(s, P.y_indices);
   D.y_row = upload_vec(s, P.y_row);
   D.jmap = upload_vec(s, P.jmap);
+  D.n_y_tail = (int)P.y_tail.size();
+  D.y_tail = upload_vec(s, P.y_tail);
   D.fP = upload_vec(s, P.fP);
   D.fQ = upload_vec(s, P.fQ);
   D.lev_ptr = upload_vec(s, P.lev_ptr);
   D.lev_big = upload_vec(s, P.lev_big);
-  D.task_out = upload_vec(s, P.task_out);
-  D.task_diag = upload_vec(s, P.task_diag);
-  D.task_pbeg = upload_vec(s, P.task_pbeg);
-  D.task_pend = upload_vec(s, P.task_pend);
-  D.task_has_a = upload_vec(s, P.task_has_a);
-  D.pair_l = upload_vec(s, P.pair_l);
-  D.pair_u = upload_vec(s, P.pair_u);
+  D.task_rec = reinterpret_cast<const int4*>(upload_vec(s, P.task_rec));
+  D.pairs = reinterpret_cast<const int2*>(upload_vec(s, P.pairs));
+  D.div_ptr = upload_vec(s, P.div_ptr);
+  D.div_rec = reinterpret_cast<const int2*>(upload_vec(s, P.div_rec));
   D.lev_piv_ptr = upload_vec(s, P.lev_piv_ptr);
   D.lev_piv = upload_vec(s, P.lev_piv);
-  D.sn_w = upload_vec(s, P.sn_w);
-  D.sn_t = upload_vec(s, P.sn_t);
-  D.sn_L = upload_vec(s, P.sn_L);
-  D.sn_U = upload_vec(s, P.sn_U);
-  D.sn_tidx = upload_vec(s, P.sn_tidx);
   D.tidx = upload_vec(s, P.tidx);
-  D.sg_ptr = upload_vec(s, P.sg_ptr);
-  D.sg_col = upload_vec(s, P.sg_col);
-  D.se_ptr = upload_vec(s, P.se_ptr);
-  D.se_rec = reinterpret_cast<const int4*>(upload_vec(s, P.se_rec));
+  D.sc_ptr = upload_vec(s, P.sc_ptr);
+  D.sc_rec = reinterpret_cast<const int4*>(upload_vec(s, P.sc_rec));
   D.fw_ptr = upload_vec(s, P.fw_ptr);
   D.fw_col = upload_vec(s, P.fw_col);
   D.fw_pos = upload_vec(s, P.fw_pos);
