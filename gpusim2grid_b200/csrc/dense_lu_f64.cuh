@@ -1,20 +1,27 @@
 // Dense FP64 LU (no pivoting) of one matrix by one CTA of 256 threads (or by
 // the CTAs of a cluster), for the tail of the FP64 batched Newton–Raphson
 // factorization: the FP64 arm, the FP64 re-solve of unconverged rows and
-// the adjoint.  Device code only.  The design of dense_lu_f32.cuh with
-// 32-wide panels, so that a row or column of a panel fits in 64 registers:
-//   1. the kb x kb diagonal block is copied to shared memory (identity
+// the adjoint.  Device code only.  Crout order on 32-wide panels: step k0
+// brings in everything the panel's columns and rows still owe,
+//   1. C -= A B on the FP64 tensor pipe (mma.sync m8n8k4) for the panel's
+//      column block (rows k0.., K = k0) and its row block (columns right of
+//      it, K = k0), in 128 x 32 and 32 x 128 tiles: every element of the
+//      matrix is read and written once for all updates before it (the
+//      accumulators start from C and run over K in order), and the K loop is
+//      long, fed by a 3-stage cp.async ring of 16-deep slabs;
+//   2. the kb x kb diagonal block is copied to shared memory (identity
 //      padded to 32 x 32) and factored by one warp holding one row per lane
 //      in registers (no block barrier inside);
-//   2. L21 = A21 U11^-1: one thread per row of A21, the row in registers,
-//      forward substitution against U11 rows read as broadcast double2;
-//   3. U12 = L11^-1 A12: one thread per column of A12, the column in
-//      registers, substitution against the rows of L11^T (unit diagonal);
-//   4. A22 -= L21 U12 on 64 x 64 output tiles: the tile's A (64 x 32) and B
-//      (32 x 64) operands are staged by cp.async in one piece, each thread
-//      accumulates a 4 x 4 block (rows tr + 16 i, columns 2 tc + 32 h + e),
-//      and the next tile's operands are in flight while a tile's results are
-//      written back.
+//   3. L21 = A21 U11^-1, one thread per row, and U12 = L11^-1 A12, one thread
+//      per column, the row or column in registers, substitution against rows
+//      read as broadcast double2.
+// Why this shape: with two rows' matrices per SM in flight (2.1 MB each at
+// n = 518) nothing stays in L2, so a right-looking update, which rewrites the
+// trailing matrix for every panel, moves 24 MB per factorization through
+// HBM; here 16 MB, almost all of it operand reads ahead of use.  mma.sync
+// runs FP64 at the FMA pipe's rate (36.6 of 37 TFLOP/s measured, one
+// accumulator chain per warp already at 31) with a fifth of the shared-memory
+// reads of a 4 x 4 DFMA block, which bounded the update before.
 // A is row-major in global memory with leading dimension ld, a multiple of
 // 2 (rows 16-byte aligned); panels start at multiples of 32.
 #pragma once
@@ -29,19 +36,30 @@ namespace dense64 {
 constexpr int BS = 256;
 constexpr int KP = 32;          // panel width
 constexpr int SD = KP + 2;      // diagonal block stride (16-byte rows)
-constexpr int TM = 64, TN = 64;
-constexpr int SA = KP + 2;      // A tile [TM][SA]
-constexpr int SB = TN + 2;      // B tile [KP][SB]
+constexpr int KS = 16;          // slab depth of the update's operand ring
+constexpr int NSTAGE = 3;
+// operand strides = 4 mod 16 doubles: the fragment loads of a half-warp (4
+// rows x 4 k) fall into 16 different banks
+constexpr int SAK = KS + 4;
+template <int TN>
+__host__ __device__ constexpr int sbn() {
+  return TN + 4;
+}
+template <int TM, int TN>
+__host__ __device__ constexpr int stage_elems() {
+  return TM * SAK + KS * sbn<TN>();
+}
 
 struct Smem {
   static constexpr int d_elems = KP * SD;
   static constexpr int r_elems = KP;  // reciprocal pivots
-  static constexpr int a_elems = TM * SA;
-  static constexpr int b_elems = KP * SB;
-  static constexpr int elems = d_elems + r_elems + a_elems + b_elems;
+  static constexpr int stage = stage_elems<128, 32>() > stage_elems<32, 128>() ? stage_elems<128, 32>()
+                                                                              : stage_elems<32, 128>();
+  // outside the update the ring holds L11^T and a 32-row block per warp
+  static constexpr int ring = NSTAGE * stage > 9 * d_elems ? NSTAGE * stage : 9 * d_elems;
+  static constexpr int elems = d_elems + r_elems + ring;
   static constexpr int bytes = elems * 8;
 };
-
 __device__ __forceinline__ double clamp_piv(double piv, double floor_) {
   if (fabs(piv) < floor_) return piv < 0.0 ? -floor_ : floor_;
   return piv;
@@ -64,112 +82,143 @@ __device__ __forceinline__ double lds1(const double* p) {
   return v;
 }
 
-__device__ __forceinline__ void cp_async16(double* smem, const double* gmem, int src_bytes) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(src_bytes));
+// This thread's share of a tile's operand slabs: PA 16-byte chunks of A (rows
+// i0 + ra + i * RA) and PB of B (k rows kb + i * RB, columns j0 + n..), the
+// same places in every slab, so the addresses only advance.  Rows past M and
+// columns past N are zero-filled.
+template <int TM, int TN>
+struct Stager {
+  static constexpr int PA = TM * KS / 2 / BS, RA = TM / PA, PB = TN * KS / 2 / BS, RB = KS / PB;
+  static_assert(PA * RA == TM && PB * RB == KS && RA * (KS / 2) == BS && RB * (TN / 2) == BS, "whole chunks");
+  const double* a;
+  const double* b;
+  int64_t lda, ldb, step_b;
+  unsigned sa, sb;  // shared-memory byte offsets within a stage
+  int arows, bbytes;
+  __device__ __forceinline__ Stager(const double* A, const double* B, int ld, int M, int N, int i0, int j0) {
+    const int tid = threadIdx.x;
+    const int ra = tid / (KS / 2), ka = (tid % (KS / 2)) * 2;
+    const int kb = tid / (TN / 2), n = (tid % (TN / 2)) * 2;
+    arows = M - i0 - ra;  // chunk i is in range for i * RA < arows
+    bbytes = (N - j0 - n) * 8;
+    bbytes = bbytes < 0 ? 0 : (bbytes > 16 ? 16 : bbytes);
+    a = A + (int64_t)(i0 + ra) * ld + ka;
+    b = B + (int64_t)kb * ld + j0 + n;
+    lda = (int64_t)RA * ld;
+    ldb = (int64_t)RB * ld;
+    step_b = (int64_t)KS * ld;
+    sa = (unsigned)(ra * SAK + ka) * 8;
+    sb = (unsigned)(TM * SAK + kb * sbn<TN>() + n) * 8;
+  }
+  // the next slab into the stage at shared-memory byte address st
+  __device__ __forceinline__ void next(unsigned st) {
+#pragma unroll
+    for (int i = 0; i < PA; ++i) {
+      const int bytes = i * RA < arows ? 16 : 0;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(st + sa + i * RA * SAK * 8),
+                   "l"(bytes ? a + i * lda : a), "r"(bytes));
+    }
+#pragma unroll
+    for (int i = 0; i < PB; ++i)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(st + sb + i * RB * sbn<TN>() * 8),
+                   "l"(b + i * ldb), "r"(bbytes));
+    a += KS;
+    b += step_b;
+  }
+};
+
+__device__ __forceinline__ void mma884(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
 }
 
-// Stage the A (rows i0.., 32 columns) and B (32 rows, columns j0..) tiles of
-// the trailing update, zero-filled outside [M) rows / [N) columns.
-__device__ __forceinline__ void stage_tile(double* sA, double* sB, const double* A21, const double* A12, int ld, int M,
-                                           int N, int i0, int j0) {
-  const int tid = threadIdx.x;
+// C[i0.., j0..] -= A[i0.., 0..K) B[0..K, j0..) for one TM x TN tile of an
+// M x N block (A, B, C parts of one matrix, leading dimension ld; K a
+// positive multiple of KS).  8 warps as WM x WN, each a grid of 8 x 8 mma
+// tiles.  An element's sum runs over K in order from C, whatever the tile
+// shape, so every tiling gives the same bits.  Ends without a barrier; the
+// ring may be refilled only after one.
+template <int TM, int TN, int WM, int WN>
+__device__ __noinline__ void update_tile(double* C, const double* A, const double* B, int ld, int M, int N, int K,
+                                         int i0, int j0, double* ring) {
+  constexpr int MT = TM / (8 * WM), NT = TN / (8 * WN);
+  constexpr int SE = stage_elems<TM, TN>();
+  static_assert(WM * WN * 32 == BS && MT > 0 && NT > 0, "8 warps tile TM x TN");
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, q = lane & 3;
+  const int wr = (warp / WN) * 8 * MT, wc = (warp % WN) * 8 * NT;
+  const int nslab = K / KS;
+  const unsigned sring = (unsigned)__cvta_generic_to_shared(ring);
+  Stager<TM, TN> stager(A, B, ld, M, N, i0, j0);
 #pragma unroll
-  for (int q = 0; q < (TM * KP / 2) / BS; ++q) {  // 4 chunks per thread
-    const int c = tid + q * BS;
-    const int r = c >> 4, k = (c & 15) * 2;
-    const bool in = i0 + r < M;
-    cp_async16(sA + r * SA + k, in ? A21 + (int64_t)(i0 + r) * ld + k : A21, in ? 16 : 0);
+  for (int s = 0; s < NSTAGE - 1; ++s) {
+    if (s < nslab) stager.next(sring + s * SE * 8);
+    asm volatile("cp.async.commit_group;\n" ::);
   }
+  int cur = 0, fill = NSTAGE - 1;  // ring positions of slab t and of slab t + NSTAGE - 1
+  double acc[MT][NT][2];
 #pragma unroll
-  for (int q = 0; q < (KP * TN / 2) / BS; ++q) {  // 4 chunks per thread
-    const int c = tid + q * BS;
-    const int k = c >> 5, n = (c & 31) * 2;
-    int bytes = (N - j0 - n) * 8;
-    bytes = bytes < 0 ? 0 : (bytes > 16 ? 16 : bytes);
-    cp_async16(sB + k * SB + n, bytes ? A12 + (int64_t)k * ld + j0 + n : A12, bytes);
-  }
-  asm volatile("cp.async.commit_group;\n" ::);
-}
-
-// A22[M x N] -= A21[M x 32] A12[32 x N].  With parts > 1 the CTA takes the
-// output tiles part, part + parts, ... (the CTAs of a cluster split them).
-__device__ __noinline__ void trailing_update(double* A22, const double* A21, const double* A12, int ld, int M, int N,
-                                             double* sA, double* sB, int part = 0, int parts = 1) {
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int tr = (warp >> 1) * 4 + (lane >> 3);  // 0..15
-  const int tc = (warp & 1) * 8 + (lane & 7);    // 0..15
-  const int n_ti = (M + TM - 1) / TM, n_tj = (N + TN - 1) / TN;
-  const int n_tiles = n_ti * n_tj;
-  if (part >= n_tiles) {
-    __syncthreads();
-    return;
-  }
-  stage_tile(sA, sB, A21, A12, ld, M, N, (part / n_tj) * TM, (part % n_tj) * TN);
-  for (int t = part; t < n_tiles; t += parts) {
-    const int i0 = (t / n_tj) * TM, j0 = (t % n_tj) * TN;
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    __syncthreads();
-    double acc[4][4];
+  for (int i = 0; i < MT; ++i) {
+    const int r = i0 + wr + 8 * i + g;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
-#pragma unroll 4
-    for (int k = 0; k < KP; ++k) {
-      double a[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = sA[(tr + 16 * i) * SA + k];
-      const double2 b0 = *reinterpret_cast<const double2*>(sB + k * SB + 2 * tc);
-      const double2 b1 = *reinterpret_cast<const double2*>(sB + k * SB + 32 + 2 * tc);
-      const double b[4] = {b0.x, b0.y, b1.x, b1.y};
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();  // every thread is done reading this tile's operands
-    if (t + parts < n_tiles) {
-      const int t1 = t + parts;
-      stage_tile(sA, sB, A21, A12, ld, M, N, (t1 / n_tj) * TM, (t1 % n_tj) * TN);
-    }
-    // epilogue: all loads of the thread's block before its stores
-    double2 cv[4][2];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = i0 + tr + 16 * i;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int c = j0 + 32 * h + 2 * tc;
-        cv[i][h] = (r < M && c + 1 < N) ? *reinterpret_cast<const double2*>(A22 + (int64_t)r * ld + c)
-                                        : make_double2(0.0, 0.0);
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = i0 + tr + 16 * i;
-      if (r >= M) continue;
-      double* crow = A22 + (int64_t)r * ld;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int c = j0 + 32 * h + 2 * tc;
-        const double* a = acc[i] + 2 * h;
-        if (c + 1 < N)
-          *reinterpret_cast<double2*>(crow + c) = make_double2(cv[i][h].x - a[0], cv[i][h].y - a[1]);
-        else if (c < N)
-          crow[c] -= a[0];
-      }
+    for (int j = 0; j < NT; ++j) {
+      const int c = j0 + wc + 8 * j + 2 * q;
+      double2 v = make_double2(0.0, 0.0);
+      const double* src = C + (int64_t)r * ld + c;
+      if (r < M && c + 1 < N) v = *reinterpret_cast<const double2*>(src);
+      else if (r < M && c < N) v.x = *src;
+      acc[i][j][0] = v.x;
+      acc[i][j][1] = v.y;
     }
   }
-  __syncthreads();
+  for (int t = 0; t < nslab; ++t) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(NSTAGE - 2) : "memory");
+    __syncthreads();  // slab t has landed; every warp is done with slab t - 1
+    if (t + NSTAGE - 1 < nslab) stager.next(sring + fill * SE * 8);
+    asm volatile("cp.async.commit_group;\n" ::);
+    const double* sA = ring + cur * SE + (wr + g) * SAK + q;
+    const double* sB = ring + cur * SE + TM * SAK + q * sbn<TN>() + wc + g;
+    cur = cur + 1 < NSTAGE ? cur + 1 : 0;
+    fill = fill + 1 < NSTAGE ? fill + 1 : 0;
+#pragma unroll
+    for (int k = 0; k < KS; k += 4) {
+      double a[MT], b[NT];
+#pragma unroll
+      for (int i = 0; i < MT; ++i) a[i] = -sA[8 * i * SAK + k];
+#pragma unroll
+      for (int j = 0; j < NT; ++j) b[j] = sB[k * sbn<TN>() + 8 * j];
+#pragma unroll
+      for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int j = 0; j < NT; ++j) mma884(acc[i][j], a[i], b[j]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < MT; ++i) {
+    const int r = i0 + wr + 8 * i + g;
+    if (r >= M) continue;
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+      const int c = j0 + wc + 8 * j + 2 * q;
+      double* dst = C + (int64_t)r * ld + c;
+      if (c + 1 < N) *reinterpret_cast<double2*>(dst) = make_double2(acc[i][j][0], acc[i][j][1]);
+      else if (c < N) *dst = acc[i][j][0];
+    }
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 }
 
 // Factor the identity-padded 32 x 32 block D (stride SD) in place; rp gets
 // the reciprocal pivots.  Warp 0 holds one row per lane in registers.  Step
-// j: lane j clamps its pivot and publishes its row (final: L part, pivot, U
-// part) to D; the lanes below take l = x_j / u_jj and x_c -= l u_jc (c > j),
-// reading row j as broadcast double2.  Warps 1..7 skip.
-__device__ __noinline__ void factor_diag(double* D, double* rp, double pfloor) {
+// j: lane j clamps its pivot and publishes its reciprocal and the rest of its
+// row (U part) to D; the lanes below take l = x_j rp_j and x_c -= l u_jc (c >
+// j), reading row j as broadcast double2.  The chain of a step is one
+// division (85 cycles), a store and a load through shared memory; the
+// division was on it twice when every lane formed 1 / u_jj itself.  The L
+// part is written at the end.  Only the first kb steps are taken; warps 1..7
+// skip.
+__device__ __noinline__ void factor_diag(double* D, double* rp, double pfloor, int kb) {
   const int r = threadIdx.x;
   if (r < KP) {
     double x[KP];
@@ -182,16 +231,18 @@ __device__ __noinline__ void factor_diag(double* D, double* rp, double pfloor) {
     __syncwarp();  // all rows read before any is rewritten
 #pragma unroll
     for (int j = 0; j < KP; ++j) {
+      if (j >= kb) continue;  // the padding needs no step
       if (r == j) {
         x[j] = clamp_piv(x[j], pfloor);
-        rp[j] = 1.0 / x[j];
 #pragma unroll
-        for (int q = 0; q < KP / 2; ++q) *reinterpret_cast<double2*>(D + j * SD + 2 * q) = make_double2(x[2 * q], x[2 * q + 1]);
+        for (int q = j / 2; q < KP / 2; ++q)
+          *reinterpret_cast<double2*>(D + j * SD + 2 * q) = make_double2(x[2 * q], x[2 * q + 1]);
+        rp[j] = 1.0 / x[j];
       }
       __syncwarp();
       if (r > j) {
         const double* uj = D + j * SD;
-        const double l = x[j] * (1.0 / lds1(uj + j));
+        const double l = x[j] * lds1(rp + j);
         x[j] = l;
         if (((j + 1) & 1) && j + 1 < KP) x[j + 1] = fma(-l, lds1(uj + j + 1), x[j + 1]);
 #pragma unroll
@@ -202,6 +253,10 @@ __device__ __noinline__ void factor_diag(double* D, double* rp, double pfloor) {
         }
       }
     }
+    // row r: L part left of the diagonal (the rest is in place)
+#pragma unroll
+    for (int c = 0; c < KP; ++c)
+      if (c < r) D[r * SD + c] = x[c];
   }
   __syncthreads();
 }
@@ -228,44 +283,78 @@ __device__ __forceinline__ void subst32(double (&x)[KP], const double* M, const 
   }
 }
 
-// L21 = A21 U11^-1 (x U11 = a per row), one thread per row (with parts > 1:
-// rows part * BS + tid, then every parts * BS).
-__device__ __noinline__ void trsm_rows(double* A21, int ld, int M, const double* D, const double* rp, int part = 0,
-                                       int parts = 1) {
-  for (int r = part * BS + threadIdx.x; r < M; r += BS * parts) {
-    double2* row = reinterpret_cast<double2*>(A21 + (int64_t)r * ld);
+// L21 = A21 U11^-1 (x U11 = a per row) for 32 rows (n of them valid) by one
+// warp, a row per lane in registers.  The rows pass through the warp's block
+// of shared memory (stride SD: conflict-free) so that global memory is read
+// and written two whole rows at a time; with every lane on its own row a load
+// touched 32 lines, and the substitution took 21 k cycles a panel instead of
+// 9 k at n = 518.
+__device__ __forceinline__ void trsm_rows32(double* A21, int ld, int n, const double* D, const double* rp,
+                                            double* buf) {
+  const int lane = threadIdx.x & 31, r2 = lane >> 4, c2 = (lane & 15) * 2;
+#pragma unroll
+  for (int h = 0; h < KP; h += 2)
+    if (h + r2 < n)
+      *reinterpret_cast<double2*>(buf + (h + r2) * SD + c2) =
+          *reinterpret_cast<const double2*>(A21 + (int64_t)(h + r2) * ld + c2);
+  __syncwarp();
+  if (lane < n) {
     double x[KP];
 #pragma unroll
     for (int q = 0; q < KP / 2; ++q) {
-      const double2 v = row[q];
+      const double2 v = lds2(buf + lane * SD + 2 * q);
       x[2 * q] = v.x;
       x[2 * q + 1] = v.y;
     }
     subst32<true>(x, D, rp);
 #pragma unroll
-    for (int q = 0; q < KP / 2; ++q) row[q] = make_double2(x[2 * q], x[2 * q + 1]);
+    for (int q = 0; q < KP / 2; ++q)
+      *reinterpret_cast<double2*>(buf + lane * SD + 2 * q) = make_double2(x[2 * q], x[2 * q + 1]);
   }
+  __syncwarp();
+#pragma unroll
+  for (int h = 0; h < KP; h += 2)
+    if (h + r2 < n)
+      *reinterpret_cast<double2*>(A21 + (int64_t)(h + r2) * ld + c2) =
+          *reinterpret_cast<const double2*>(buf + (h + r2) * SD + c2);
+  __syncwarp();
 }
 
 // U12 = L11^-1 A12 (per column: y^T L11^T = a^T, L11^T upper with unit
-// diagonal, given by its rows LT = rows of L11^T), one thread per column.
-__device__ __noinline__ void trsm_cols(double* A12, int ld, int N, const double* LT, int part = 0, int parts = 1) {
-  for (int c = part * BS + threadIdx.x; c < N; c += BS * parts) {
-    double y[KP];
-    const double* src = A12 + c;
+// diagonal, given by its rows LT), one column of A12 in registers.
+__device__ __forceinline__ void trsm_col(double* colp, int ld, const double* LT) {
+  double y[KP];
+  const double* src = colp;
 #pragma unroll
-    for (int r = 0; r < KP; ++r, src += ld) {
-      y[r] = *src;
-      if ((r & 15) == 15) asm volatile("" ::: "memory");  // at most 16 loads in flight
+  for (int r = 0; r < KP; ++r, src += ld) {
+    y[r] = *src;
+    if ((r & 15) == 15) asm volatile("" ::: "memory");  // at most 16 loads in flight
+  }
+  subst32<false>(y, LT, nullptr);
+  // the stores walk the column again from an opaque copy of ld, so the 32
+  // load addresses are not kept alive across the substitution
+  int ld2;
+  asm volatile("mov.b32 %0, %1;\n" : "=r"(ld2) : "r"(ld));
+  double* dst = colp;
+#pragma unroll
+  for (int r = 0; r < KP; ++r, dst += ld2) *dst = y[r];
+}
+
+// Both substitutions of a panel with m rows below and m columns to the right
+// of its diagonal block, in groups of 32 rows or 32 columns taken by the
+// warps of the `parts` CTAs (this one: part).  LT: L11^T, followed by a block
+// per warp.
+__device__ __noinline__ void trsm_panel(double* A21, double* A12, int ld, int m, const double* D, const double* rp,
+                                        double* LT, int part, int parts) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int ng = (m + 31) / 32;
+  for (int t = part * (BS / 32) + warp; t < 2 * ng; t += parts * (BS / 32)) {
+    if (t < ng) {
+      trsm_rows32(A21 + (int64_t)t * 32 * ld, ld, min(32, m - 32 * t), D, rp, LT + Smem::d_elems * (1 + warp));
+    } else {
+      const int c = (t - ng) * 32 + lane;
+      if (c < m) trsm_col(A12 + c, ld, LT);
     }
-    subst32<false>(y, LT, nullptr);
-    // the stores walk the column again from an opaque copy of ld, so the 32
-    // load addresses are not kept alive across the substitution
-    int ld2;
-    asm volatile("mov.b32 %0, %1;\n" : "=r"(ld2) : "r"(ld));
-    double* dst = A12 + c;
-#pragma unroll
-    for (int r = 0; r < KP; ++r, dst += ld2) *dst = y[r];
   }
 }
 
@@ -289,33 +378,37 @@ __device__ __forceinline__ void transpose_l11(double* LT, const double* D) {
 __device__ void lu(double* A, int n, int ld, double* smem, double pfloor) {
   double* D = smem;
   double* rp = D + Smem::d_elems;
-  double* sA = rp + Smem::r_elems;
-  double* sB = sA + Smem::a_elems;
+  double* ring = rp + Smem::r_elems;
   const int tid = threadIdx.x;
   for (int k0 = 0; k0 < n; k0 += KP) {
     const int kb = min(KP, n - k0);
+    const int m = n - k0 - kb;  // > 0 only with kb == 32
     double* Akk = A + (int64_t)k0 * ld + k0;
+    const double* Arow = A + (int64_t)k0 * ld;  // rows k0.. of the columns before the panel
+    if (k0 > 0) {
+      for (int i0 = 0; i0 < n - k0; i0 += 128) {
+        update_tile<128, 32, 8, 1>(Akk, Arow, A + k0, ld, n - k0, kb, k0, i0, 0, ring);
+        __syncthreads();
+      }
+      for (int j0 = 0; j0 < m; j0 += 128) {
+        update_tile<32, 128, 1, 8>(Akk + kb, Arow, A + k0 + kb, ld, kb, m, k0, 0, j0, ring);
+        __syncthreads();
+      }
+    }
     load_diag(D, Akk, ld, kb);
     __syncthreads();
-    factor_diag(D, rp, pfloor);
+    factor_diag(D, rp, pfloor, kb);
     for (int idx = tid; idx < kb * kb; idx += BS) {
       const int r = idx / kb, c = idx % kb;
       Akk[(int64_t)r * ld + c] = D[r * SD + c];
     }
-    const int m = n - k0 - kb;  // > 0 only with kb == 32
     if (m > 0) {
-      double* A21 = A + (int64_t)(k0 + kb) * ld + k0;
-      double* A12 = A + (int64_t)k0 * ld + k0 + kb;
-      double* A22 = A + (int64_t)(k0 + kb) * ld + k0 + kb;
-      double* LT = sA;
+      double* LT = ring;
       transpose_l11(LT, D);
       __syncthreads();
-      trsm_rows(A21, ld, m, D, rp);
-      trsm_cols(A12, ld, m, LT);
-      __syncthreads();  // L21 and U12 complete (global writes of other threads)
-      trailing_update(A22, A21, A12, ld, m, m, sA, sB);
+      trsm_panel(A + (int64_t)(k0 + kb) * ld + k0, Akk + kb, ld, m, D, rp, LT, 0, 1);
     }
-    __syncthreads();
+    __syncthreads();  // L21, U12 and the diagonal block complete
   }
 }
 
@@ -329,36 +422,43 @@ __device__ __forceinline__ void cluster_sync_all() {
 }
 
 // The same LU as lu(), by the `parts` CTAs of a cluster together (this CTA
-// has rank `part`); A in global memory, every CTA with its own scratch.
-// Each CTA factors the diagonal block itself (every CTA needs it in its own
-// shared memory), the row and column substitutions and the trailing-update
-// tiles are split by rank, and three cluster barriers per panel order the
-// stages.  Every element goes through the same operations in the same order
-// as in lu(), so the factor is bit-identical.  Every CTA of the cluster must
-// call it with the same n.
+// has rank `part`); A in global memory, every CTA with its own scratch.  The
+// update's blocks are split into 32 x 32 tiles by rank (its critical path is
+// the K loop of one tile), each CTA factors the diagonal block itself (every
+// CTA needs it in its own shared memory), the substitutions are split by rank,
+// and three cluster barriers per panel order the stages.  Every element goes
+// through the same operations in the same order as in lu(), so the factor is
+// bit-identical.  Every CTA of the cluster must call it with the same n.
 __device__ void lu_cluster(double* A, int n, int ld, double* smem, double pfloor, int part, int parts) {
   double* D = smem;
   double* rp = D + Smem::d_elems;
-  double* sA = rp + Smem::r_elems;
-  double* sB = sA + Smem::a_elems;
+  double* ring = rp + Smem::r_elems;
   const int tid = threadIdx.x;
   for (int k0 = 0; k0 < n; k0 += KP) {
     const int kb = min(KP, n - k0);
+    const int m = n - k0 - kb;
     double* Akk = A + (int64_t)k0 * ld + k0;
+    const double* Arow = A + (int64_t)k0 * ld;
+    if (k0 > 0) {
+      const int nc = (n - k0 + 31) / 32, nr = (m + 31) / 32;
+      for (int t = part; t < nc + nr; t += parts) {
+        if (t < nc)
+          update_tile<32, 32, 4, 2>(Akk, Arow, A + k0, ld, n - k0, kb, k0, 32 * t, 0, ring);
+        else
+          update_tile<32, 32, 4, 2>(Akk + kb, Arow, A + k0 + kb, ld, kb, m, k0, 0, 32 * (t - nc), ring);
+        __syncthreads();
+      }
+      cluster_sync_all();  // the panel's blocks complete
+    }
     load_diag(D, Akk, ld, kb);
     __syncthreads();
-    factor_diag(D, rp, pfloor);
+    factor_diag(D, rp, pfloor, kb);
     cluster_sync_all();  // every CTA holds the block: rank 0 may write it back below
-    const int m = n - k0 - kb;
-    double* A21 = A + (int64_t)(k0 + kb) * ld + k0;
-    double* A12 = A + (int64_t)k0 * ld + k0 + kb;
-    double* A22 = A + (int64_t)(k0 + kb) * ld + k0 + kb;
     if (m > 0) {
-      double* LT = sA;
+      double* LT = ring;
       transpose_l11(LT, D);
       __syncthreads();
-      trsm_rows(A21, ld, m, D, rp, part, parts);
-      trsm_cols(A12, ld, m, LT, part, parts);
+      trsm_panel(A + (int64_t)(k0 + kb) * ld + k0, Akk + kb, ld, m, D, rp, LT, part, parts);
     }
     if (part == 0)
       for (int idx = tid; idx < kb * kb; idx += BS) {
@@ -366,8 +466,6 @@ __device__ void lu_cluster(double* A, int n, int ld, double* smem, double pfloor
         Akk[(int64_t)r * ld + c] = D[r * SD + c];
       }
     cluster_sync_all();  // L21, U12 and the diagonal block complete
-    if (m > 0) trailing_update(A22, A21, A12, ld, m, m, sA, sB, part, parts);
-    cluster_sync_all();  // A22 complete
   }
 }
 
