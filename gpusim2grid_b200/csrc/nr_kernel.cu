@@ -1560,8 +1560,8 @@ __global__ void __launch_bounds__(BS, GS2G_MIN_CTAS_PER_SM)
     prof.flush(a.phase_cycles);
     return;
   }
-  // the row lives in the leader's workspace
-  char* ws = a.workspace + (int64_t)(blockIdx.x - rank) * a.ws_stride;
+  // one workspace per cluster
+  char* ws = a.workspace + (int64_t)(blockIdx.x / parts) * a.ws_stride;
   T* S = reinterpret_cast<T*>(ws + ws_layout<T>(P).S);
   T* HV = reinterpret_cast<T*>(ws + ws_layout<T>(P).HV);
   prof.init(a.phase_cycles != nullptr && threadIdx.x == 0 && rank == 0);

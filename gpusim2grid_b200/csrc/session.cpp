@@ -659,6 +659,9 @@ gs2g::SweepArgs make_args(gs2g_session* s, const gs2g_run_opts& o, int n_rows, c
   return a;
 }
 
+// Dense tail from which a row's factorizations are shared by a cluster.
+constexpr int kClusterTail = 64;
+
 // Cluster size for `rows` rows that each get a cluster within `n_ctas`
 // CTAs: 16, else 8, else 0 (one CTA per row).
 int cluster_for(int rows, int n_ctas) {
@@ -742,11 +745,12 @@ float launch(gs2g_session* s, const gs2g_run_opts& o, int n_rows, const double* 
     a.alt_s = nullptr;
     a.alt_i = nullptr;
   }
-  // hand-offs with a dense tail worth sharing: a cluster of 16 (or 8) CTAs
-  // per row when every row gets one (the rows are few and each of their
-  // factorizations would otherwise run on one SM after every other row has
-  // finished)
-  const int csize = chord && s->handoff_cluster && s->dplan.nt >= 64 ? cluster_for(n_next, n_ctas) : 0;
+  // rows with a dense tail worth sharing, few enough that each gets a cluster
+  // of 16 (or 8) CTAs: the hand-offs, whose factorizations would otherwise run
+  // on one SM each after every other row has finished, and small batches
+  // (a single solve among them), which would leave the other SMs idle
+  const bool few = s->handoff_cluster && s->dplan.nt >= kClusterTail && (chord || n_rows <= n_ctas);
+  const int csize = few ? cluster_for(n_next, chord ? n_ctas : gs2g::sweep_ctas(o.precision, s->device)) : 0;
   if (n_next > 0 && csize > 0) {
     ck((cudaError_t)gs2g::launch_sweep_cluster(s->dplan, a, o.precision, csize, n_next * csize, s->stream),
        "hand-off cluster launch");
@@ -1611,7 +1615,7 @@ int gs2g_run_subset(gs2g_session* s, const gs2g_run_opts* o_, int n_sub, const i
   int n_ctas = o.n_ctas > 0 ? o.n_ctas : gs2g::sweep_ctas(o.precision, s->device);
   // few rows with a dense tail worth sharing (an FP64 re-solve of the rows
   // a mixed sweep did not converge): a cluster of CTAs per row
-  const int csize = s->handoff_cluster && s->dplan.nt >= 64 ? cluster_for(n_sub, n_ctas) : 0;
+  const int csize = s->handoff_cluster && s->dplan.nt >= kClusterTail ? cluster_for(n_sub, n_ctas) : 0;
   const bool cluster = n_sub > 0 && csize > 0;
   n_ctas = cluster ? n_sub * csize : std::max(1, std::min(n_ctas, std::max(n_sub, 1)));
   const int64_t wsb = gs2g::workspace_bytes(s->dplan, o.precision);
