@@ -11,8 +11,8 @@
 // of two tensor-memory accumulators; warps 2..9 empty the other one through a
 // padded shared-memory block each, so that global memory sees 128-byte rows,
 // and apply the epilogue there while the next tile's products run.
-// BN = 256 halves the shared-memory operand bytes per product against 128 x
-// 128 tiles (which cap the tensor pipe near half rate); BN = 128 and a split
+// BN = 256 takes 3/4 of the operand bytes per product of 128 x 128 tiles, and
+// those bytes bound the kernel (64 bytes a cycle into an SM); BN = 128 and a split
 // of K into partial planes (summed in order by finish_kernel with the same
 // epilogue) serve shapes with fewer tiles than SMs.  gemm_plan picks both by
 // the waves they take.
@@ -73,25 +73,42 @@ struct Epilogue {
   int lda;
 };
 
-__device__ __forceinline__ void epilogue(const Epilogue& e, int r, int c, float v) {
-  float* d = e.D + (int64_t)r * e.ldd + c;
-  switch (e.op) {
-    case EPI_STORE:
-      *d = e.accumulate ? v + *d : v;
-      break;
-    case EPI_BIAS:
-      *d = v + e.bias[c];
-      break;
-    case EPI_GELU: {
-      const float z = v + e.bias[c];
-      if (e.D != nullptr) *d = z;
-      e.act[(int64_t)r * e.lda + c] = __float2bfloat16(gelu_f(z));
-      break;
+// The epilogue of column c, rows r0, r0 + 1, ..: OP the operation at compile
+// time, or EPI_ANY to look at it per element.  (With the operation looked up and
+// the addresses formed per element, the GELU epilogue took longer than the
+// products of a K = 1024 layer.)
+constexpr int EPI_ANY = -1;
+template <int OP>
+struct ColumnEpilogue {
+  const int op;
+  const int accumulate;
+  const float bias;
+  float* d;
+  __nv_bfloat16* act;
+  const int64_t ldd, lda;
+  __device__ __forceinline__ ColumnEpilogue(const Epilogue& e, int r0, int c)
+      : op(OP == EPI_ANY ? e.op : OP),
+        accumulate(e.accumulate),
+        bias(op == EPI_BIAS || op == EPI_GELU ? e.bias[c] : 0.f),
+        d(e.D != nullptr ? e.D + (int64_t)r0 * e.ldd + c : nullptr),
+        act(op >= EPI_GELU ? e.act + (int64_t)r0 * e.lda + c : nullptr),
+        ldd(e.ldd),
+        lda(e.lda) {}
+  __device__ __forceinline__ void row(int q, float v) const {
+    float* dq = d + q * ldd;
+    if (op == EPI_STORE) {
+      *dq = accumulate ? v + *dq : v;
+    } else if (op == EPI_BIAS) {
+      *dq = v + bias;
+    } else if (op == EPI_GELU) {
+      const float z = v + bias;
+      if (d != nullptr) *dq = z;
+      act[q * lda] = __float2bfloat16(gelu_f(z));
+    } else {
+      act[q * lda] = __float2bfloat16(v * gelu_grad_f(*dq));
     }
-    default:
-      e.act[(int64_t)r * e.lda + c] = __float2bfloat16(v * gelu_grad_f(*d));
   }
-}
+};
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -117,8 +134,10 @@ __device__ __forceinline__ uint64_t global_ns() {
 
 // Bounded wait for the phase with the given parity; false after WAIT_NS, or as
 // soon as another wait of the CTA has failed (*fail, nullptr: not looked at).
+// The timer is first read after 64 tries: reading it on every wait took longer
+// than a 64-deep step's products.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* fail) {
-  const uint64_t t0 = global_ns();
+  uint64_t t0 = 0;
   for (uint32_t i = 0;; ++i) {
     uint32_t done;
     asm volatile(
@@ -131,7 +150,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     if (done) return true;
     if ((i & 63) == 63) {
       if (fail != nullptr && *fail) return false;
-      if (global_ns() - t0 > WAIT_NS) {
+      const uint64_t now = global_ns();
+      if (t0 == 0) {
+        t0 = now;
+      } else if (now - t0 > WAIT_NS) {
         if (fail != nullptr) *fail = 1;
         return false;
       }
@@ -161,7 +183,7 @@ struct GemmShape {
   float* part;
 };
 
-template <int BN, bool A_MN, bool B_MN>
+template <int BN, bool A_MN, bool B_MN, int OP>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
     gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                      const GemmShape g, const Epilogue e, int* err) {
@@ -315,8 +337,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 #pragma unroll 8
             for (int q = 0; q < 32; ++q) p[(int64_t)q * g.N] = buf[q * EPI_LD + lane];
           } else {
+            const ColumnEpilogue<OP> ep(e, r0, c);
 #pragma unroll 8
-            for (int q = 0; q < 32; ++q) epilogue(e, r0 + q, c, buf[q * EPI_LD + lane]);
+            for (int q = 0; q < 32; ++q) ep.row(q, buf[q * EPI_LD + lane]);
           }
         }
         __syncwarp();
@@ -341,6 +364,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 }
 
 // Sums the partial planes of a split product in order and applies the epilogue.
+template <int OP>
 __global__ void __launch_bounds__(256) finish_kernel(const GemmShape g, const Epilogue e) {
   const int64_t plane = (int64_t)g.M * g.N;
   const int c = blockIdx.x * 256 + threadIdx.x;
@@ -354,15 +378,18 @@ __global__ void __launch_bounds__(256) finish_kernel(const GemmShape g, const Ep
 #pragma unroll
     for (int s = 1; s < MAX_SPLIT; ++s)
       if (s < g.splits) v += x[s];
-    epilogue(e, r, c, v);
+    ColumnEpilogue<OP>(e, r, c).row(0, v);
   }
 }
 
 // Tile width and K split of an M x N x K product on n_sm SMs: the pair that
-// takes the fewest cycles in whole waves.  A 64-deep step of a 128 x 256 tile
-// takes about 300 cycles, of a 128 x 128 tile about 200 (bound by its operand
-// reads); a tile costs about 2500 more (filling the ring, the last epilogue),
-// and a split a pass over its planes.
+// takes the fewest cycles in whole waves.  A 64-deep step brings 48 KB (128 x 256
+// tile) or 32 KB (128 x 128) into the SM, and that, not the tensor pipe (540 or
+// 270 cycles), sets its time: about 850 and 700 cycles measured.  A tile costs
+// about 3000 more (filling the ring, the last epilogue).  A split adds a launch
+// and a pass over its planes: K = 7232 on 2944 x 1024 took 51 us whole and 63 in
+// three, on 1024 x 1024 44 us in two and 35 in four; K = 3712 on 1024 x 1024 43
+// us whole, 30 in two.
 struct GemmPlan {
   int bn, splits, kt_split;
 };
@@ -377,8 +404,8 @@ inline GemmPlan gemm_plan(int M, int N, int K, int n_sm, bool may_split) {
       const int kts = (KT + s - 1) / s;
       if ((s - 1) * kts >= KT) continue;  // an empty split
       const double waves = (double)((tiles * s + n_sm - 1) / n_sm);
-      double cost = waves * (kts * (bn == 256 ? 300.0 : 200.0) + 2500.0);
-      if (s > 1) cost += 4000.0 + (double)M * N * 4.0 * (s + 1) / 3000.0;  // the finishing launch
+      double cost = waves * (kts * (bn == 256 ? 850.0 : 700.0) + 3000.0);
+      if (s > 1) cost += 6000.0 + (double)M * N * 4.0 * (s + 1) / 2000.0;  // the finishing launch
       if (cost < best_cost) {
         best_cost = cost;
         best = {bn, s, kts};

@@ -7,6 +7,7 @@
 
 #include <cstdint>
 
+#include "../../include/gs2g.h"
 #include "mlp_gemm.cuh"
 
 namespace gs2g {
@@ -45,6 +46,7 @@ __global__ void __launch_bounds__(256) mse_grad_kernel(const float* y, const flo
   const int c = blockIdx.x * 256 + threadIdx.x;
   float acc = 0.f;
   if (c < cols)
+#pragma unroll 4
     for (int r = blockIdx.y; r < rows; r += gridDim.y) {
       const int64_t i = (int64_t)r * ld + c;
       float g = 0.f;
@@ -66,14 +68,14 @@ __global__ void __launch_bounds__(256) mse_grad_kernel(const float* y, const flo
 
 // column sums of a bf16 matrix: out[c] += sum_r x[r][c]; block (128 columns)
 // x (a chunk of COLSUM_ROWS rows), one atomicAdd per column and chunk
-constexpr int COLSUM_ROWS = 256;
+constexpr int COLSUM_ROWS = 64;
 __global__ void colsum_bf16_kernel(const __nv_bfloat16* x, int ld, int rows, int cols, float* out) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= cols) return;
   const int r0 = blockIdx.y * COLSUM_ROWS;
   const int r1 = min(rows, r0 + COLSUM_ROWS);
   float s = 0.f;
-#pragma unroll 8
+#pragma unroll 16
   for (int r = r0; r < r1; ++r) s += __bfloat162float(x[(int64_t)r * ld + c]);
   atomicAdd(out + c, s);
 }
@@ -360,16 +362,34 @@ bool operand_map(CUtensorMap* map, const void* p, int ld, bool mn, int rows, int
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BN, bool A_MN, bool B_MN>
+template <int BN, bool A_MN, bool B_MN, int OP>
 cudaError_t launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const GemmShape& g, const Epilogue& e, int* err,
                         void* stream) {
-  cudaError_t rc = cudaFuncSetAttribute(gemm_bf16_kernel<BN, A_MN, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        gemm_smem<BN>());
+  cudaError_t rc = cudaFuncSetAttribute(gemm_bf16_kernel<BN, A_MN, B_MN, OP>,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_smem<BN>());
   if (rc != cudaSuccess) return rc;
   const int tiles = g.tiles_m * g.tiles_n * g.splits, n_sm = sm_count();
-  gemm_bf16_kernel<BN, A_MN, B_MN><<<tiles < n_sm ? tiles : n_sm, GEMM_THREADS, gemm_smem<BN>(),
-                                     (cudaStream_t)stream>>>(ma, mb, g, e, err);
+  gemm_bf16_kernel<BN, A_MN, B_MN, OP><<<tiles < n_sm ? tiles : n_sm, GEMM_THREADS, gemm_smem<BN>(),
+                                         (cudaStream_t)stream>>>(ma, mb, g, e, err);
   return cudaGetLastError();
+}
+
+// The network's own combinations of layout and epilogue have kernels of their
+// own; any other pair runs with the operation looked up per element.
+template <int BN>
+cudaError_t launch_gemm_any(bool a_mn, bool b_mn, const CUtensorMap& ma, const CUtensorMap& mb, const GemmShape& g,
+                            const Epilogue& e, int* err, void* stream) {
+  if (!a_mn && !b_mn && e.op == EPI_GELU) return launch_gemm<BN, false, false, EPI_GELU>(ma, mb, g, e, err, stream);
+  if (!a_mn && !b_mn && e.op == EPI_BIAS) return launch_gemm<BN, false, false, EPI_BIAS>(ma, mb, g, e, err, stream);
+  if (!a_mn && !b_mn && e.op == EPI_STORE) return launch_gemm<BN, false, false, EPI_STORE>(ma, mb, g, e, err, stream);
+  if (a_mn && b_mn && e.op == EPI_STORE) return launch_gemm<BN, true, true, EPI_STORE>(ma, mb, g, e, err, stream);
+  if (!a_mn && b_mn && e.op == EPI_GELU_BWD)
+    return launch_gemm<BN, false, true, EPI_GELU_BWD>(ma, mb, g, e, err, stream);
+  if (a_mn)
+    return b_mn ? launch_gemm<BN, true, true, EPI_ANY>(ma, mb, g, e, err, stream)
+                : launch_gemm<BN, true, false, EPI_ANY>(ma, mb, g, e, err, stream);
+  return b_mn ? launch_gemm<BN, false, true, EPI_ANY>(ma, mb, g, e, err, stream)
+              : launch_gemm<BN, false, false, EPI_ANY>(ma, mb, g, e, err, stream);
 }
 }  // namespace
 
@@ -401,19 +421,14 @@ int gs2g_mlp_gemm(const void* A, int lda, int a_mn, const void* B, int ldb, int 
     gs2g::set_last_error("gemm: the driver rejected a tensor map");
     return 3;
   }
-  cudaError_t rc;
-  if (p.bn == 256)
-    rc = a_mn ? (b_mn ? launch_gemm<256, true, true>(ma, mb, g, e, err, stream)
-                      : launch_gemm<256, true, false>(ma, mb, g, e, err, stream))
-              : (b_mn ? launch_gemm<256, false, true>(ma, mb, g, e, err, stream)
-                      : launch_gemm<256, false, false>(ma, mb, g, e, err, stream));
-  else
-    rc = a_mn ? (b_mn ? launch_gemm<128, true, true>(ma, mb, g, e, err, stream)
-                      : launch_gemm<128, true, false>(ma, mb, g, e, err, stream))
-              : (b_mn ? launch_gemm<128, false, true>(ma, mb, g, e, err, stream)
-                      : launch_gemm<128, false, false>(ma, mb, g, e, err, stream));
+  cudaError_t rc = p.bn == 256 ? launch_gemm_any<256>(a_mn != 0, b_mn != 0, ma, mb, g, e, err, stream)
+                               : launch_gemm_any<128>(a_mn != 0, b_mn != 0, ma, mb, g, e, err, stream);
   if (rc == cudaSuccess && g.splits > 1) {
-    finish_kernel<<<dim3((N + 255) / 256, M < 512 ? M : 512), 256, 0, (cudaStream_t)stream>>>(g, e);
+    const dim3 grid((N + 255) / 256, M < 512 ? M : 512);
+    cudaStream_t st = (cudaStream_t)stream;
+    if (op == EPI_GELU) finish_kernel<EPI_GELU><<<grid, 256, 0, st>>>(g, e);
+    else if (op == EPI_GELU_BWD) finish_kernel<EPI_GELU_BWD><<<grid, 256, 0, st>>>(g, e);
+    else finish_kernel<EPI_ANY><<<grid, 256, 0, st>>>(g, e);
     rc = cudaGetLastError();
   }
   return status_of(rc);
@@ -543,6 +558,57 @@ int gs2g_mlp_start_voltages(const float* y, int ldy, const float* y_mean, const 
   start_voltages_kernel<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(
       y, ldy, y_mean, y_std, va_index, vm_index, (const double2*)vinit, n_bus, (double2*)v0, rows);
   return status_of(cudaGetLastError());
+}
+
+// ---- whole passes of the network, one call each
+
+static int net_ok(const gs2g_mlp_net* n, const char* what) {
+  if (!n || n->layers < 1 || n->rows <= 0 || n->rows % GT || n->k0 % GT || n->h % GT || n->o % GT || !n->w_off ||
+      !n->b_off || !n->wb || !n->master || !n->act || !n->y || !n->err)
+    return invalid(what);
+  return 0;
+}
+
+int gs2g_mlp_net_forward(const gs2g_mlp_net* n, int first, void* stream) {
+  if (int rc = net_ok(n, "net_forward: bad network")) return rc;
+  const size_t bh = (size_t)n->rows * n->h;
+  for (int l = first; l <= n->layers; ++l) {
+    const int in = l == 0 ? n->k0 : n->h, out = l == n->layers ? n->o : n->h;
+    const void* a = l == 0 ? n->x : (const void*)((const __nv_bfloat16*)n->act + (l - 1) * bh);
+    const void* w = (const __nv_bfloat16*)n->wb + n->w_off[l];
+    const float* b = n->master + n->b_off[l];
+    const bool last = l == n->layers;
+    const int rc = gs2g_mlp_gemm(a, l == 0 ? n->ldx : in, 0, w, in, 0, n->rows, out, in, last ? EPI_BIAS : EPI_GELU, 0,
+                                 last ? n->y : (n->pre && (l == 0 || n->dy) ? n->pre + l * bh : nullptr), out, b,
+                                 last ? nullptr : (void*)((__nv_bfloat16*)n->act + l * bh), out, n->part,
+                                 n->part_elems, n->err, stream);
+    if (rc) return rc;
+  }
+  return 0;
+}
+
+int gs2g_mlp_net_backward(const gs2g_mlp_net* n, const float* t, int n_out, float scale, void* stream) {
+  if (int rc = net_ok(n, "net_backward: bad network")) return rc;
+  if (!n->pre || !n->grad || !n->dy || !n->g || !t || !n->loss) return invalid("net_backward: training buffers missing");
+  const size_t bh = (size_t)n->rows * n->h;
+  int rc = gs2g_mlp_mse_grad(n->y, t, n->o, n->dy, n->rows, n->o, n_out, scale, n->loss, stream);
+  const __nv_bfloat16* g = (const __nv_bfloat16*)n->dy;
+  for (int l = n->layers; l >= 0 && !rc; --l) {
+    const int in = l == 0 ? n->k0 : n->h, out = l == n->layers ? n->o : n->h;
+    const void* a = l == 0 ? n->x : (const void*)((const __nv_bfloat16*)n->act + (l - 1) * bh);
+    // dW = g^T a over the batch rows, both operands as they lie
+    rc = gs2g_mlp_gemm(g, out, 1, a, l == 0 ? n->ldx : in, 1, out, in, n->rows, EPI_STORE, 0, n->grad + n->w_off[l], in,
+                       nullptr, nullptr, 0, n->part, n->part_elems, n->err, stream);
+    if (!rc) rc = gs2g_mlp_colsum_bf16(g, out, n->rows, out, n->grad + n->b_off[l], stream);
+    if (l > 0 && !rc) {
+      // the layer below's g = (g W) gelu', into the buffer g is not in
+      __nv_bfloat16* nxt = (__nv_bfloat16*)n->g + ((l - 1) & 1) * bh;
+      rc = gs2g_mlp_gemm(g, out, 0, (const __nv_bfloat16*)n->wb + n->w_off[l], in, 1, n->rows, in, out, EPI_GELU_BWD, 0,
+                         n->pre + (l - 1) * bh, in, nullptr, nxt, in, n->part, n->part_elems, n->err, stream);
+      g = nxt;
+    }
+  }
+  return rc;
 }
 
 }  // extern "C"

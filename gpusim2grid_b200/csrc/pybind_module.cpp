@@ -534,6 +534,54 @@ void bind_mlp(py::module_& m) {
                         P<float>(D), ldd, P<float>(bias), P<void>(act), ld_act, P<float>(part), part_elems, P<int>(err),
                         S(stream)));
   });
+  // a network's layout and buffers (raw device pointers; the caller's tensors
+  // outlive the calls), the input rows given per call
+  struct Net {
+    gs2g_mlp_net n{};
+    std::vector<int64_t> w_off, b_off;
+  };
+  py::class_<Net>(mm, "Net")
+      .def(py::init([](int rows, int k0, int h, int o, std::vector<int64_t> w_off, std::vector<int64_t> b_off,
+                       uintptr_t wb, uintptr_t master, uintptr_t grad, uintptr_t pre, uintptr_t act, uintptr_t y,
+                       uintptr_t dy, uintptr_t g, uintptr_t loss, uintptr_t part, int64_t part_elems, uintptr_t err) {
+        auto net = std::make_unique<Net>();
+        net->w_off = std::move(w_off);
+        net->b_off = std::move(b_off);
+        gs2g_mlp_net& n = net->n;
+        n.layers = (int)net->w_off.size() - 1;
+        n.rows = rows;
+        n.k0 = k0;
+        n.h = h;
+        n.o = o;
+        n.w_off = net->w_off.data();
+        n.b_off = net->b_off.data();
+        n.wb = P<void>(wb);
+        n.master = P<float>(master);
+        n.grad = P<float>(grad);
+        n.pre = P<float>(pre);
+        n.act = P<void>(act);
+        n.y = P<float>(y);
+        n.dy = P<void>(dy);
+        n.g = P<void>(g);
+        n.loss = P<float>(loss);
+        n.part = P<float>(part);
+        n.part_elems = part_elems;
+        n.err = P<int>(err);
+        return net;
+      }))
+      .def("forward",
+           [](Net& net, uintptr_t x, int ldx, int first, uintptr_t stream) {
+             gs2g_mlp_net n = net.n;
+             n.x = P<void>(x);
+             n.ldx = ldx;
+             check(gs2g_mlp_net_forward(&n, first, S(stream)));
+           })
+      .def("backward", [](Net& net, uintptr_t x, int ldx, uintptr_t t, int n_out, float scale, uintptr_t stream) {
+        gs2g_mlp_net n = net.n;
+        n.x = P<void>(x);
+        n.ldx = ldx;
+        check(gs2g_mlp_net_backward(&n, P<float>(t), n_out, scale, S(stream)));
+      });
   mm.def("bias_act", [](uintptr_t pre, int ldp, uintptr_t bias, uintptr_t act, int lda, int rows, int cols, bool gelu,
                         uintptr_t stream) {
     check(gs2g_mlp_bias_act(P<float>(pre), ldp, P<float>(bias), P<void>(act), lda, rows, cols, gelu ? 1 : 0,

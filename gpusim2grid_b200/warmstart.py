@@ -42,8 +42,6 @@ from ._native import lib
 __all__ = ["WarmStartMLP", "LearnedStart", "make_training_rows", "generate_solutions"]
 
 _M = lib.mlp
-# operations of gs2g_mlp_gemm on a finished sum
-_STORE, _BIAS, _GELU, _GELU_BWD = range(4)
 
 
 def _ceil(x, m):
@@ -152,15 +150,15 @@ class WarmStartMLP:
         dev, f32, bf = self.device, torch.float32, torch.bfloat16
         L = self.layers
         # pre[l]: the hidden layers' sums before the activation, which the
-        # backward pass reads (inference only keeps the first layer's, for
+        # backward pass reads (inference keeps the first layer's, for
         # predict_trips)
-        w = dict(pre=[torch.empty(B, self.h, dtype=f32, device=dev) if train or l == 0 else None for l in range(L)],
-                 act=[torch.empty(B, self.h, dtype=bf, device=dev) for _ in range(L)],
+        w = dict(pre=torch.empty(L if train else 1, B, self.h, dtype=f32, device=dev),
+                 act=torch.empty(L, B, self.h, dtype=bf, device=dev),
                  y=torch.empty(B, self.o, dtype=f32, device=dev))
         mnk = [(B, o, i) for o, i in self.shapes]
         if train:
             w.update(dy=torch.empty(B, self.o, dtype=bf, device=dev),
-                     g=[torch.empty(B, self.h, dtype=bf, device=dev) for _ in range(min(L, 2))],
+                     g=torch.empty(2, B, self.h, dtype=bf, device=dev),
                      loss=torch.zeros(1, dtype=f32, device=dev))
             mnk += [(o, i, B) for o, i in self.shapes] + [(B, i, o) for o, i in self.shapes[1:]]
         w["part"] = torch.empty(max(_M.gemm_part(*s) for s in mnk), dtype=f32, device=dev)
@@ -168,36 +166,27 @@ class WarmStartMLP:
         return w
 
     # ------------------------------------------------------------- kernels
-    def _gemm(self, w, op, A, B, D, a_mn=False, b_mn=False, bias=None, act=None):
-        """One product on gs2g_mlp_gemm: A (M, K), or (K, M) with ``a_mn``; B
-        (N, K), or (K, N) with ``b_mn``; ``op`` and its buffers as there."""
-        M, K = A.shape[::-1] if a_mn else A.shape
-        N, K2 = B.shape[::-1] if b_mn else B.shape
-        if K != K2 or any(t is not None and tuple(t.shape) != (M, N) for t in (D, act)):
-            raise ValueError(f"gemm shapes {tuple(A.shape)} ({a_mn}) x {tuple(B.shape)} ({b_mn})")
-        ptr = lambda t: 0 if t is None else t.data_ptr()
-        ld = lambda t: 0 if t is None else t.stride(0)
-        _M.gemm(A.data_ptr(), A.stride(0), a_mn, B.data_ptr(), B.stride(0), b_mn, M, N, K, op, False, ptr(D), ld(D),
-                ptr(bias), ptr(act), ld(act), w["part"].data_ptr(), w["part"].numel(), self.err.data_ptr(), _stream())
+    def _net(self, w):
+        """The native network over the current weights and the buffers w."""
+        ptr = lambda k: w[k].data_ptr() if k in w else 0
+        return _M.Net(w["y"].shape[0], self.k0, self.h, self.o, [a for a, _ in self._offs],
+                      [b for _, b in self._offs], self.wb.data_ptr(), self.master.data_ptr(), self.grad.data_ptr(),
+                      ptr("pre"), ptr("act"), ptr("y"), ptr("dy"), ptr("g"), ptr("loss"),
+                      ptr("part"), w["part"].numel(), self.err.data_ptr())
 
     def _wb(self, l):
         return self._view(self.wb, l, False)
 
+    def _input(self, X, w):
+        B = w["y"].shape[0]
+        if X.shape[0] != B or X.shape[1] != self.k0:
+            raise ValueError(f"inputs must be ({B}, {self.k0}), got {tuple(X.shape)}")
+        return X.data_ptr(), X.stride(0)
+
     def _forward(self, X, w):
         """The network's outputs w['y'] for inputs X; every bias and activation
         is applied by the product that feeds it."""
-        self._layer(0, X, w)
-        return self._layers_after(0, w)
-
-    def _layer(self, l, a, w):
-        if l < self.layers:
-            self._gemm(w, _GELU, a, self._wb(l), w["pre"][l] if "dy" in w or l == 0 else None, bias=self.b(l), act=w["act"][l])
-        else:
-            self._gemm(w, _BIAS, a, self._wb(l), w["y"], bias=self.b(l))
-
-    def _layers_after(self, l, w):
-        for k in range(l + 1, self.layers + 1):
-            self._layer(k, w["act"][k - 1], w)
+        self._net(w).forward(*self._input(X, w), 0, _stream())
         return w["y"]
 
     def _forward_rest(self, w, B):
@@ -205,7 +194,8 @@ class WarmStartMLP:
         rows) to its outputs w['y']."""
         _M.bias_act(w["pre"][0].data_ptr(), self.h, self.b(0).data_ptr(), w["act"][0].data_ptr(), self.h, B, self.h,
                     True, _stream())
-        return self._layers_after(0, w)
+        self._net(w).forward(0, self.k0, 1, _stream())
+        return w["y"]
 
     def _sparse_first(self):
         """(W0T, base) of the current first-layer weights and input
@@ -253,24 +243,8 @@ class WarmStartMLP:
     def _backward(self, X, T, w, scale):
         """Gradients of 0.5 * scale * ||y - T||^2 over the valid columns into
         self.grad; accumulates the squared error into w['loss']."""
-        B = X.shape[0]
-        L = self.layers
-        st = _stream()
-        _M.mse_grad(w["y"].data_ptr(), T.data_ptr(), self.o, w["dy"].data_ptr(), B, self.o, self.n_out, scale,
-                    w["loss"].data_ptr(), st)
-        g = w["dy"]
-        for l in range(L, -1, -1):
-            o, i = self.shapes[l]
-            a = X if l == 0 else w["act"][l - 1]
-            # dW = g^T a over the batch rows, both operands as they lie
-            self._gemm(w, _STORE, g, a, self._view(self.grad, l, False), a_mn=True, b_mn=True)
-            _M.colsum_bf16(g.data_ptr(), g.stride(0), B, o, self._view(self.grad, l, True).data_ptr(), st)
-            if l > 0:
-                # dx = g W times the activation's derivative (g and its
-                # successor are different buffers)
-                nxt = w["g"][(l - 1) % len(w["g"])]
-                self._gemm(w, _GELU_BWD, g, self._wb(l), w["pre"][l - 1], b_mn=True, act=nxt)
-                g = nxt
+        T = T.contiguous()
+        self._net(w).backward(*self._input(X, w), T.data_ptr(), self.n_out, float(scale), _stream())
 
     def gradients(self, X, T, scale=None):
         """One forward + backward on a batch (X bf16, T fp32, rows a multiple
@@ -283,8 +257,8 @@ class WarmStartMLP:
         self._forward(X, w)
         self._backward(X, T, w, scale)
         self.check()
-        grads = [(self._view(self.grad, l, False).clone(), self._view(self.grad, l, True).clone())
-                 for l in range(self.layers + 1)]
+        flat = self.grad.clone()
+        grads = [(self._view(flat, l, False), self._view(flat, l, True)) for l in range(self.layers + 1)]
         return grads, float(w["loss"].item())
 
     def check(self):

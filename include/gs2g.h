@@ -411,6 +411,36 @@ int64_t gs2g_mlp_gemm_part(int M, int N, int K);
 int gs2g_mlp_gemm(const void* A, int lda, int a_mn, const void* B, int ldb, int b_mn, int M, int N, int K, int op,
                   int accumulate, float* D, int ldd, const float* bias, void* act_bf16, int ld_act, float* part,
                   int64_t part_elems, int* err, void* stream);
+/* A whole network x -> [Linear -> GELU] x layers -> Linear -> y on `rows` rows
+ * (a multiple of 128) in one call: widths k0, h (hidden), o, all multiples of
+ * 128; layer l's weights W_l (out x in, row-major) at element w_off[l] and its
+ * bias at b_off[l] of wb (bf16) / master (fp32) / grad (fp32).  act [layers]
+ * [rows][h] bf16; pre, the sums before the activation: [layers][rows][h] in
+ * training (dy given), the first layer's alone otherwise (may be NULL); for
+ * training also dy [rows][o], g [2][rows][h] bf16 and loss. */
+typedef struct gs2g_mlp_net {
+  int layers, rows, k0, h, o, ldx;
+  const void* x;
+  const int64_t* w_off;
+  const int64_t* b_off;
+  const void* wb;
+  const float* master;
+  float* grad;
+  float* pre;
+  void* act;
+  float* y;
+  void* dy;
+  void* g;
+  float* loss;
+  float* part; /* partial sums of K splits, part_elems floats (gs2g_mlp_gemm) */
+  int64_t part_elems;
+  int* err;
+} gs2g_mlp_net;
+/* Layers first.. of the forward pass (first > 0: act[first - 1] is in place). */
+int gs2g_mlp_net_forward(const gs2g_mlp_net* net, int first, void* stream);
+/* Gradients of 0.5 * scale * ||y - t||^2 over the first n_out columns into
+ * grad, after a forward pass with pre; *loss += the squared error. */
+int gs2g_mlp_net_backward(const gs2g_mlp_net* net, const float* t, int n_out, float scale, void* stream);
 /* pre += bias (per column); act = bf16(gelu(pre)) (exact erf GELU) or
  * bf16(pre) when gelu = 0; act may be NULL. */
 int gs2g_mlp_bias_act(float* pre, int ldp, const float* bias, void* act_bf16, int lda, int rows, int cols, int gelu,
