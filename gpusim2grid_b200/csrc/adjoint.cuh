@@ -128,7 +128,7 @@ __device__ __noinline__ void solve_transposed(const DevPlan& P, const T* __restr
 // entries of masked buses, get 0.
 template <typename T>
 __global__ void __launch_bounds__(BS, GS2G_MIN_CTAS_PER_SM)
-    adjoint_kernel(const DevPlan P, const SweepArgs a, const double* __restrict__ rhs, double* __restrict__ lam) {
+    adjoint_kernel(const __grid_constant__ DevPlan P, const __grid_constant__ SweepArgs a, const double* __restrict__ rhs, double* __restrict__ lam) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_row;
   __shared__ int s_ne;

@@ -54,17 +54,6 @@
 #endif
 constexpr int CK = GS2G_CHORD_ROWS;  // rows per CTA
 
-// Unrolling of the chord loops whose loads form dependent chains (index ->
-// right-hand side): the head and tail solves' entry loops and the dense
-// product's column loop.  Build-time; the defaults were measured fastest.
-#ifndef GS2G_CHORD_SOLVE_UNROLL
-#define GS2G_CHORD_SOLVE_UNROLL 4
-#endif
-#ifndef GS2G_CHORD_DENSE_UNROLL
-#define GS2G_CHORD_DENSE_UNROLL 8
-#endif
-#define GS2G_PRAGMA(x) _Pragma(#x)
-#define GS2G_UNROLL(n) GS2G_PRAGMA(unroll n)
 constexpr int CB_MAX = 10;  // Broyden steps kept per row (the memory restarts beyond)
 
 // the CK right-hand sides of one unknown, loaded as one vector (or two)
@@ -166,9 +155,20 @@ __device__ __forceinline__ void comp_apply(const int i, const int dim, const uns
 #pragma unroll
   for (int s = 0; s < CK; ++s) {
     if (!(comp >> s & 1)) continue;
+    // the columns in batches of CB loads in flight (a single outage touches up
+    // to 4 positions, a pair up to 8): one load after another, this sum took
+    // 130 k of the 740 k cycles of a 2000-bus N-1 step
+    constexpr int CB = 4;
     const int r = s_cr[s][0];
     T acc = T(0);
-    for (int c = 0; c < r; ++c) acc += Minv[(int64_t)s_cr[s][1 + c] * dim + i] * (T)s_cw[s][c];
+    for (int c = 0; c < r; c += CB) {
+      T m[CB];
+#pragma unroll
+      for (int u = 0; u < CB; ++u) m[u] = c + u < r ? Minv[(int64_t)s_cr[s][1 + c + u] * dim + i] : T(0);
+#pragma unroll
+      for (int u = 0; u < CB; ++u)
+        if (c + u < r) acc += m[u] * (T)s_cw[s][c + u];
+    }
     yi.v[s] -= acc;
   }
 }
@@ -278,41 +278,68 @@ __device__ __noinline__ void chord_broyden(const int dim, const unsigned mask, C
 }
 
 // F and ||F||inf of the slots in `mask` (bit s: slot s): one sweep over the
-// Ybus rows, each entry read once for all slots.  Row edits are applied as
+// Ybus rows, each entry read once for all slots, a row per lane in slices of
+// rows of one length (the lanes read consecutive entries; the next slice's
+// records are on their way while a slice is summed).  Row edits are applied as
 // corrections on the buses of the edited Ybus rows (edit e subtracts ev[e]
 // from Y at the entry of row er[e], column ec[e]).  F goes straight into the
 // slots' lanes of the interleaved right-hand sides y (the chord solve's
 // input, in T); lanes of slots outside `mask` are kept only where `keep`
-// has their bit (others are not read before they are written again).
-template <typename T>
-__device__ __noinline__ void chord_mismatch(const DevPlan P, const SweepArgs a, const unsigned mask,
+// has their bit (others are not read before they are written again).  MU: Ybus
+// entries in flight per lane, of CK voltages each (2 fit in the registers of 2
+// CTAs per SM, 1 in those of 3).
+template <typename T, int MU>
+__device__ __noinline__ void chord_mismatch(const DevPlan& P, const SweepArgs& a, const unsigned mask,
                                             const unsigned keep, const ChordSlot* sl, const int* s_ne,
                                             const int (*s_er)[MAX_EDITS], const int (*s_ec)[MAX_EDITS],
                                             const double2 (*s_ev)[MAX_EDITS], const double2* Vs, SlotVec<T>* y,
                                             double* nrm_out, double* s_red_slots) {
-  const int n = P.n_bus;
-  const double2* Y = reinterpret_cast<const double2*>(a.ybus);
+  const int4* __restrict__ yl_rec = P.yl_rec;
+  const int* __restrict__ yl_col = P.yl_col;
+  const double2* __restrict__ yl_val = P.yl_val;
+  const int* __restrict__ fPs = P.fP;
+  const int* __restrict__ fQs = P.fQ;
+  const int n_ysl = P.n_ysl;
   const double2* sb[CK];
 #pragma unroll
   for (int s = 0; s < CK; ++s)
     sb[s] = reinterpret_cast<const double2*>(a.sbus) + (int64_t)(sl[s].row < 0 ? 0 : sl[s].row) * a.sbus_stride;
   double lmax[CK] = {};
-  for (int i = threadIdx.x; i < n; i += BS) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int4 none = make_int4(-1, 0, 0, 0);
+  int4 next = warp < n_ysl ? yl_rec[warp * 32 + lane] : none;
+  for (int sl_i = warp; sl_i < n_ysl; sl_i += NWARP) {
+    const int4 r = next;
+    next = sl_i + NWARP < n_ysl ? yl_rec[(sl_i + NWARP) * 32 + lane] : none;
+    const int i = r.x;
+    if (i < 0) continue;
     double2 acc[CK];
 #pragma unroll
     for (int s = 0; s < CK; ++s) acc[s] = make_double2(0.0, 0.0);
-    for (int k = P.y_indptr[i]; k < P.y_indptr[i + 1]; ++k) {
-      const double2 yk = Y[k];
-      const int j = P.y_indices[k];
+    // every slot's lane is summed (a lane outside `mask` is not used)
+    for (int q = 0; q < r.y; q += MU) {
+      double2 yk[MU], vj[MU][CK];
+      int j[MU];
 #pragma unroll
-      for (int s = 0; s < CK; ++s) {
-        if (!(mask >> s & 1)) continue;
-        const double2 vj = Vs[(int64_t)j * CK + s];
-        acc[s].x = fma(yk.x, vj.x, fma(-yk.y, vj.y, acc[s].x));
-        acc[s].y = fma(yk.x, vj.y, fma(yk.y, vj.x, acc[s].y));
-      }
+      for (int h = 0; h < MU; ++h)
+        if (q + h < r.y) j[h] = yl_col[r.z + 32 * (q + h)];
+#pragma unroll
+      for (int h = 0; h < MU; ++h)
+        if (q + h < r.y) {
+          yk[h] = yl_val[r.z + 32 * (q + h)];
+#pragma unroll
+          for (int s = 0; s < CK; ++s) vj[h][s] = Vs[(int64_t)j[h] * CK + s];
+        }
+#pragma unroll
+      for (int h = 0; h < MU; ++h)
+        if (q + h < r.y)
+#pragma unroll
+          for (int s = 0; s < CK; ++s) {
+            acc[s].x = fma(yk[h].x, vj[h][s].x, fma(-yk[h].y, vj[h][s].y, acc[s].x));
+            acc[s].y = fma(yk[h].x, vj[h][s].y, fma(yk[h].y, vj[h][s].x, acc[s].y));
+          }
     }
-    const int fp = P.fP[i], fq = P.fQ[i];
+    const int fp = fPs[i], fq = fQs[i];
     SlotVec<T> rp{}, rq{};
     if (keep) {
       if (fp >= 0) rp = y[fp];
@@ -355,7 +382,7 @@ __device__ __noinline__ void chord_mismatch(const DevPlan P, const SweepArgs a, 
 // are bit-identical to chord_mismatch's for this slot.  Writes only the
 // slot's lane of y.
 template <typename T>
-__device__ __noinline__ void chord_mismatch_alt(const DevPlan P, const SweepArgs a, const int s, const ChordSlot* sl,
+__device__ __noinline__ void chord_mismatch_alt(const DevPlan& P, const SweepArgs& a, const int s, const ChordSlot* sl,
                                                 const int* s_ne, const int (*s_er)[MAX_EDITS],
                                                 const int (*s_ec)[MAX_EDITS], const double2 (*s_ev)[MAX_EDITS],
                                                 const double2* Vs, const double2* __restrict__ Ia, SlotVec<T>* y,
@@ -385,45 +412,94 @@ __device__ __noinline__ void chord_mismatch_alt(const DevPlan P, const SweepArgs
   __syncthreads();
 }
 
-// Forward over the head levels, all slots at once.  fwv: the factor's
-// values in solve order (one sequential stream beside fw_col).
-template <typename T>
-__device__ __noinline__ void chord_head_fw(const DevPlan P, const T* __restrict__ fwv, SlotVec<T>* y) {
-  for (int lv = 0; lv < P.n_levels; ++lv) {
-    for (int q0 = P.lev_piv_ptr[lv] + threadIdx.x; q0 < P.lev_piv_ptr[lv + 1]; q0 += BS) {
-      const int i = P.lev_piv[q0];
-      SlotVec<T> acc = y[i];
-      GS2G_UNROLL(GS2G_CHORD_SOLVE_UNROLL)
-      for (int q = P.fw_ptr[i]; q < P.fw_ptr[i + 1]; ++q) fms_slots(acc, fwv[q], y[P.fw_col[q]]);
-      y[i] = acc;
+// Lists [l0, l1) of the plan's slices, all slots at once, a barrier after
+// each (see row_lists, the one-row form).  sv: the entries' values in slice
+// order.
+template <typename T, bool DIV>
+__device__ __noinline__ void chord_lists(const DevPlan& P, const T* __restrict__ sv, const T* __restrict__ fHV,
+                                         SlotVec<T>* y, const int l0, const int l1) {
+  constexpr int PF = 4;  // entries per lane and batch
+  const int* __restrict__ lev = P.sl_lev;
+  const int4* __restrict__ rec = P.sl_rec;
+  const int* __restrict__ cols = P.sl_col;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  struct Batch {
+    int col[PF];
+    T v[PF];
+  };
+  auto record = [&](const SliceCursor& c) {
+    return c.l < l1 ? rec[c.s * 32 + lane] : make_int4(-1, 0, 0, 1);
+  };
+  auto load = [&](const int4& r, int q, Batch& b) {
+#pragma unroll
+    for (int h = 0; h < PF; ++h) {
+      const bool in = q + h < r.y;
+      b.col[h] = in ? cols[r.z + 32 * (q + h)] : -1;
+      b.v[h] = in ? sv[r.z + 32 * (q + h)] : T(0);
+    }
+  };
+  auto run = [&](const int4& r, Batch b, T d) {
+    SlotVec<T> acc{};
+    for (int q = 0;;) {
+#pragma unroll
+      for (int h = 0; h < PF; ++h)
+        if (b.col[h] >= 0) fms_slots(acc, b.v[h], y[b.col[h]]);
+      q += PF;
+      if (q >= r.y) break;
+      load(r, q, b);
+    }
+    for (int o = 1; o < r.w; o <<= 1)  // r.w: the same in a slice
+#pragma unroll
+      for (int s = 0; s < CK; ++s) acc.v[s] += __shfl_xor_sync(0xffffffffu, acc.v[s], o);
+    if (r.x >= 0 && (lane & (r.w - 1)) == 0) {
+      SlotVec<T> v = y[r.x];
+#pragma unroll
+      for (int s = 0; s < CK; ++s) {
+        v.v[s] += acc.v[s];
+        if (DIV) v.v[s] = v.v[s] / d;
+      }
+      y[r.x] = v;
+    }
+  };
+  SliceCursor a(lev, l0, l1, warp), c = a;
+  int4 ra = record(a);
+  Batch ba;
+  load(ra, 0, ba);
+  T da = DIV && ra.x >= 0 ? fHV[ra.x] : T(1);
+  c.next(warp);
+  int4 rc = record(c);
+  for (int l = l0; l < l1; ++l) {
+    while (a.l == l) {
+      Batch bn;
+      load(rc, 0, bn);
+      const T dn = DIV && rc.x >= 0 ? fHV[rc.x] : T(1);
+      SliceCursor n = c;
+      n.next(warp);
+      const int4 rn = record(n);
+      run(ra, ba, da);
+      a = c;
+      ra = rc;
+      ba = bn;
+      da = dn;
+      c = n;
+      rc = rn;
     }
     __syncthreads();
   }
 }
 
-// The tail rows against the head.
-template <typename T>
-__device__ __noinline__ void chord_tail_fw(const DevPlan P, const T* __restrict__ fwv, SlotVec<T>* y) {
-  for (int ti = threadIdx.x; ti < P.nt; ti += BS) {
-    const int i = P.p + ti;
-    SlotVec<T> acc = y[i];
-    GS2G_UNROLL(GS2G_CHORD_SOLVE_UNROLL)
-    for (int q = P.fw_ptr[i]; q < P.fw_ptr[i + 1]; ++q) fms_slots(acc, fwv[q], y[P.fw_col[q]]);
-    y[i] = acc;
-  }
-  __syncthreads();
-}
-
 // y_t <- Sinv y_t for all slots: the tail block of the base inverse (column j
 // at Minv + (p + j) * dim + p) times the CK columns held in shared memory.
 // Each thread owns up to four tail rows per pass; for each column a warp
-// reads 32 consecutive entries.
+// reads 32 consecutive entries.  Eight columns in flight: 16 were no faster, and
+// loading the next 4 while 4 are multiplied was 1.8 times as slow.
 template <typename T>
-__device__ __noinline__ void chord_dense(const DevPlan P, const T* __restrict__ Minv, SlotVec<T>* y, SlotVec<T>* ys) {
-  const int tid = threadIdx.x, nt = P.nt;
-  for (int i = tid; i < nt; i += BS) ys[i] = y[P.p + i];
+__device__ __noinline__ void chord_dense(const int p, const int nt, const int dim, const T* __restrict__ Minv,
+                                          SlotVec<T>* y, SlotVec<T>* ys) {
+  const int tid = threadIdx.x;
+  for (int i = tid; i < nt; i += BS) ys[i] = y[p + i];
   __syncthreads();
-  const T* Sinv = Minv + (int64_t)P.p * P.dim + P.p;
+  const T* Sinv = Minv + (int64_t)p * dim + p;
   for (int r0 = 0; r0 < nt; r0 += 4 * BS) {
     SlotVec<T> acc[4];
 #pragma unroll
@@ -432,46 +508,26 @@ __device__ __noinline__ void chord_dense(const DevPlan P, const T* __restrict__ 
       for (int s = 0; s < CK; ++s) acc[u].v[s] = T(0);
     const int nr = min(4, (nt - r0 - tid + BS - 1) / BS);  // rows of this thread in the pass (may be <= 0)
     const T* base = Sinv + r0 + tid;
-    GS2G_UNROLL(GS2G_CHORD_DENSE_UNROLL)
+#pragma unroll 8
     for (int j = 0; j < nt; ++j) {
       const SlotVec<T> yj = ys[j];
-      const T* col = base + (int64_t)j * P.dim;
+      const T* col = base + (int64_t)j * dim;
 #pragma unroll
       for (int u = 0; u < 4; ++u)
         if (u < nr) fms_slots(acc[u], -col[u * BS], yj);
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u)
-      if (u < nr) y[P.p + r0 + tid + u * BS] = acc[u];
+      if (u < nr) y[p + r0 + tid + u * BS] = acc[u];
   }
   __syncthreads();
-}
-
-// Backward over the head levels (bwv: values in solve order, fHV for the
-// pivots).
-template <typename T>
-__device__ __noinline__ void chord_head_bw(const DevPlan P, const T* __restrict__ fHV, const T* __restrict__ bwv,
-                                           SlotVec<T>* y) {
-  for (int lv = P.n_levels - 1; lv >= 0; --lv) {
-    for (int q0 = P.lev_piv_ptr[lv] + threadIdx.x; q0 < P.lev_piv_ptr[lv + 1]; q0 += BS) {
-      const int k = P.lev_piv[q0];
-      SlotVec<T> acc = y[k];
-      GS2G_UNROLL(GS2G_CHORD_SOLVE_UNROLL)
-      for (int q = P.bw_ptr[k]; q < P.bw_ptr[k + 1]; ++q) fms_slots(acc, bwv[q], y[P.bw_row[q]]);
-      const T d = fHV[k];
-#pragma unroll
-      for (int s = 0; s < CK; ++s) acc.v[s] = acc.v[s] / d;
-      y[k] = acc;
-    }
-    __syncthreads();
-  }
 }
 
 // Outputs of a slot's row as it leaves: V (the slot's lane of the
 // interleaved voltages, V[i * CK]), and either the final status (flows
 // included, from the row's output copy) or the hand-off to the single-row
 // kernel.
-__device__ __noinline__ void chord_leave(const SweepArgs a, const ChordSlot sl, const double2* V, const int n,
+__device__ __noinline__ void chord_leave(const SweepArgs& a, const ChordSlot sl, const double2* V, const int n,
                                          double* s_red) {
   const int tid = threadIdx.x;
   const int row = sl.row;
@@ -594,8 +650,7 @@ __device__ __forceinline__ void chord_body(const DevPlan& P, const SweepArgs& a,
   T* St = reinterpret_cast<T*>(ws + L.S);
   const WsLayout BL = ws_layout<T>(P);  // layout of the base factor's workspace
   const T* fHV = reinterpret_cast<const T*>(a.base_ws + BL.HV);
-  const T* fwv = reinterpret_cast<const T*>(a.base_fwv);
-  const T* bwv = reinterpret_cast<const T*>(a.base_bwv);
+  const T* slv = reinterpret_cast<const T*>(a.base_slv);
   const T* Minv = reinterpret_cast<const T*>(a.base_inv);
   const double2* Y = reinterpret_cast<const double2*>(a.ybus);
   const double2* Vbase = reinterpret_cast<const double2*>(a.base_v);
@@ -610,7 +665,7 @@ __device__ __forceinline__ void chord_body(const DevPlan& P, const SweepArgs& a,
   __syncthreads();
   for (;;) {
     // ---- refill empty slots from the row queue ----------------------------
-    for (int s = 0; s < CK; ++s) {
+    for (int s = 0; s < a.chord_slots; ++s) {
       if (sl[s].row >= 0) continue;
       for (;;) {
         // every thread reads the flag before thread 0 may pull (and clear it)
@@ -677,7 +732,7 @@ __device__ __forceinline__ void chord_body(const DevPlan& P, const SweepArgs& a,
     if (active == 0) break;
 
     // ---- mismatch of every slot, start selection for new rows --------------
-    chord_mismatch<T>(P, a, active, 0u, sl, s_ne, s_er, s_ec, s_ev, Vs, y, s_nrm, s_red_slots);
+    chord_mismatch<T, Y_SMEM ? 2 : 1>(P, a, active, 0u, sl, s_ne, s_er, s_ec, s_ev, Vs, y, s_nrm, s_red_slots);
     for (int s = 0; s < CK; ++s) {
       if (!(active >> s & 1) || !sl[s].fresh) continue;
       const RowEdits ed{s_ne[s], s_ek[s], s_ev[s]};
@@ -700,7 +755,7 @@ __device__ __forceinline__ void chord_body(const DevPlan& P, const SweepArgs& a,
           chord_mismatch_alt<T>(P, a, s, sl, s_ne, s_er, s_ec, s_ev, Vs, reinterpret_cast<const double2*>(a.alt_i),
                                 y, s_nrm, s_red);
         else
-          chord_mismatch<T>(P, a, 1u << s, active & ~(1u << s), sl, s_ne, s_er, s_ec, s_ev, Vs, y, s_nrm,
+          chord_mismatch<T, Y_SMEM ? 2 : 1>(P, a, 1u << s, active & ~(1u << s), sl, s_ne, s_er, s_ec, s_ev, Vs, y, s_nrm,
                             s_red_slots);
       }
     }
@@ -743,13 +798,16 @@ __device__ __forceinline__ void chord_body(const DevPlan& P, const SweepArgs& a,
 
     // ---- one solve on the base factor for every remaining slot (F is in y;
     // the lanes of slots that left are not read) ------------------------------
-    chord_head_fw<T>(P, fwv, y);
+    // forward: head levels, then the tail rows (list n_levels); the tail; the
+    // head rows' tail columns (all at once), then the head levels backward
+    chord_lists<T, false>(P, slv, fHV, y, 0, P.n_levels);
     prof.mark(PH_SOLVE);
-    chord_tail_fw<T>(P, fwv, y);
+    chord_lists<T, false>(P, slv, fHV, y, P.n_levels, P.n_levels + 1);
     prof.mark(PH_SOLVE_TAIL);
-    if (P.nt > 0) chord_dense<T>(P, Minv, y, ys);
+    if (P.nt > 0) chord_dense<T>(P.p, P.nt, P.dim, Minv, y, ys);
     prof.mark(PH_SOLVE_DENSE);
-    chord_head_bw<T>(P, fHV, bwv, y);
+    chord_lists<T, false>(P, slv, fHV, y, P.n_levels + 1, P.n_levels + 2);
+    chord_lists<T, true>(P, slv, fHV, y, P.n_levels + 2, 2 * P.n_levels + 2);
     {
       unsigned comp = 0;
       for (int s = 0; s < CK; ++s) comp |= ((solve >> s & 1) && sl[s].comp ? 1u : 0u) << s;
@@ -821,7 +879,7 @@ __device__ __forceinline__ void chord_body(const DevPlan& P, const SweepArgs& a,
 }
 
 template <typename T>
-__global__ void __launch_bounds__(BS, GS2G_CHORD_CTAS_PER_SM) chord_kernel(const DevPlan P, const SweepArgs a) {
+__global__ void __launch_bounds__(BS, GS2G_CHORD_CTAS_PER_SM) chord_kernel(const __grid_constant__ DevPlan P, const __grid_constant__ SweepArgs a) {
   PhaseProf prof;
   prof.init(a.phase_cycles != nullptr && threadIdx.x == 0);
   chord_body<T>(P, a, prof);
@@ -832,7 +890,7 @@ __global__ void __launch_bounds__(BS, GS2G_CHORD_CTAS_PER_SM) chord_kernel(const
 // whose dim x 4 values fit beside the tail copy): every solve's gathers are
 // shared-memory loads, at 2 CTAs per SM instead of 3.
 template <typename T>
-__global__ void __launch_bounds__(BS, 2) chord_kernel_ysmem(const DevPlan P, const SweepArgs a) {
+__global__ void __launch_bounds__(BS, 2) chord_kernel_ysmem(const __grid_constant__ DevPlan P, const __grid_constant__ SweepArgs a) {
   PhaseProf prof;
   prof.init(a.phase_cycles != nullptr && threadIdx.x == 0);
   chord_body<T, true>(P, a, prof);

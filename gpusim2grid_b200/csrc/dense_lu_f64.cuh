@@ -10,8 +10,7 @@
 //      accumulators start from C and run over K in order), and the K loop is
 //      long, fed by a 3-stage cp.async ring of 16-deep slabs;
 //   2. the kb x kb diagonal block is copied to shared memory (identity
-//      padded to 32 x 32) and factored by one warp holding one row per lane
-//      in registers (no block barrier inside);
+//      padded to 32 x 32) and factored there, a row over 8 lanes;
 //   3. L21 = A21 U11^-1, one thread per row, and U12 = L11^-1 A12, one thread
 //      per column, the row or column in registers, substitution against rows
 //      read as broadcast double2.
@@ -209,55 +208,58 @@ __device__ __noinline__ void update_tile(double* C, const double* A, const doubl
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 }
 
-// Factor the identity-padded 32 x 32 block D (stride SD) in place; rp gets
-// the reciprocal pivots.  Warp 0 holds one row per lane in registers.  Step
-// j: lane j clamps its pivot and publishes its reciprocal and the rest of its
-// row (U part) to D; the lanes below take l = x_j rp_j and x_c -= l u_jc (c >
-// j), reading row j as broadcast double2.  The chain of a step is one
-// division (85 cycles), a store and a load through shared memory; the
-// division was on it twice when every lane formed 1 / u_jj itself.  The L
-// part is written at the end.  Only the first kb steps are taken; warps 1..7
-// skip.
+// Factor the identity-padded 32 x 32 block D (stride SD) in place, its first kb
+// steps; rp gets the reciprocal pivots.  All 8 warps: thread (r, q) holds
+// columns 4 q .. 4 q + 3 of row r in registers (a row is 8 lanes of one warp).
+// Step j: row j's lanes clamp the pivot and publish the row and the pivot's
+// reciprocal (two buffers, one barrier per step); the rows below take l = x_j
+// rp (x_j from its lane by shuffle) and x_c -= l u_jc for c > j.  A step's
+// chain is the division (85 cycles), a store, a barrier and a load: 0.19 k
+// cycles against 0.36 k for one warp with a row per lane, whose 32 - j loads and
+// products per lane were on it too.
 __device__ __noinline__ void factor_diag(double* D, double* rp, double pfloor, int kb) {
-  const int r = threadIdx.x;
-  if (r < KP) {
-    double x[KP];
-#pragma unroll
-    for (int q = 0; q < KP / 2; ++q) {
-      const double2 v = lds2(D + r * SD + 2 * q);
-      x[2 * q] = v.x;
-      x[2 * q + 1] = v.y;
-    }
-    __syncwarp();  // all rows read before any is rewritten
-#pragma unroll
-    for (int j = 0; j < KP; ++j) {
-      if (j >= kb) continue;  // the padding needs no step
-      if (r == j) {
-        x[j] = clamp_piv(x[j], pfloor);
-#pragma unroll
-        for (int q = j / 2; q < KP / 2; ++q)
-          *reinterpret_cast<double2*>(D + j * SD + 2 * q) = make_double2(x[2 * q], x[2 * q + 1]);
-        rp[j] = 1.0 / x[j];
-      }
-      __syncwarp();
-      if (r > j) {
-        const double* uj = D + j * SD;
-        const double l = x[j] * lds1(rp + j);
-        x[j] = l;
-        if (((j + 1) & 1) && j + 1 < KP) x[j + 1] = fma(-l, lds1(uj + j + 1), x[j + 1]);
-#pragma unroll
-        for (int c2 = ((j + 1) + 1) & ~1; c2 < KP; c2 += 2) {
-          const double2 u = lds2(uj + c2);
-          x[c2] = fma(-l, u.x, x[c2]);
-          x[c2 + 1] = fma(-l, u.y, x[c2 + 1]);
-        }
-      }
-    }
-    // row r: L part left of the diagonal (the rest is in place)
-#pragma unroll
-    for (int c = 0; c < KP; ++c)
-      if (c < r) D[r * SD + c] = x[c];
+  __shared__ __align__(16) double prow[2][KP];
+  const int r = threadIdx.x >> 3, q = threadIdx.x & 7, lane = threadIdx.x & 31;
+  double x[4];
+  {
+    const double2 v0 = *reinterpret_cast<const double2*>(D + r * SD + 4 * q);
+    const double2 v1 = *reinterpret_cast<const double2*>(D + r * SD + 4 * q + 2);
+    x[0] = v0.x;
+    x[1] = v0.y;
+    x[2] = v1.x;
+    x[3] = v1.y;
   }
+#pragma unroll
+  for (int j = 0; j < KP; ++j) {
+    if (j >= kb) break;  // the padding needs no step
+    if (r == j) {
+      if (q == j >> 2) {
+        x[j & 3] = clamp_piv(x[j & 3], pfloor);
+        rp[j] = 1.0 / x[j & 3];
+      }
+      *reinterpret_cast<double2*>(&prow[j & 1][4 * q]) = make_double2(x[0], x[1]);
+      *reinterpret_cast<double2*>(&prow[j & 1][4 * q + 2]) = make_double2(x[2], x[3]);
+    }
+    __syncthreads();
+    const double xj = __shfl_sync(0xffffffffu, x[j & 3], (lane & 24) | (j >> 2));
+    if (r > j && q >= j >> 2) {
+      const double l = xj * rp[j];
+      const double2 u0 = *reinterpret_cast<const double2*>(&prow[j & 1][4 * q]);
+      const double2 u1 = *reinterpret_cast<const double2*>(&prow[j & 1][4 * q + 2]);
+      const double u[4] = {u0.x, u0.y, u1.x, u1.y};
+      if (q > j >> 2) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) x[c] = fma(-l, u[c], x[c]);
+      } else {
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if (c > (j & 3)) x[c] = fma(-l, u[c], x[c]);
+        x[j & 3] = l;
+      }
+    }
+  }
+  *reinterpret_cast<double2*>(D + r * SD + 4 * q) = make_double2(x[0], x[1]);
+  *reinterpret_cast<double2*>(D + r * SD + 4 * q + 2) = make_double2(x[2], x[3]);
   __syncthreads();
 }
 

@@ -119,7 +119,16 @@ __host__ __device__ constexpr int dense_smem_elems() {
 // thread and of a warp's lanes end together -- and a task's record is one
 // 16-byte load, its pairs one 8-byte load each, consecutive over the lanes.
 template <typename T>
-__device__ __noinline__ void head_lu(const DevPlan P, T* HV, const double pfloor, const int part, const int parts) {
+__device__ __noinline__ void head_lu(const DevPlan& P, T* HV, const double pfloor, const int part, const int parts) {
+  // the plan's fields in registers: a store through T* would force reloads
+  const int4* __restrict__ task_rec = P.task_rec;
+  const int2* __restrict__ pairs = P.pairs;
+  const int2* __restrict__ div_rec = P.div_rec;
+  const int* __restrict__ lev_ptr = P.lev_ptr;
+  const int* __restrict__ lev_big = P.lev_big;
+  const int* __restrict__ div_ptr = P.div_ptr;
+  const int n_levels = P.n_levels;
+  const int p = P.p;
   constexpr int TU = 2, QU = 4;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gwarp = part * NWARP + warp, nwarps = parts * NWARP;
@@ -130,21 +139,21 @@ __device__ __noinline__ void head_lu(const DevPlan P, T* HV, const double pfloor
     else
       __syncthreads();
   };
-  for (int lv = 0; lv < P.n_levels; ++lv) {
-    const int t0 = P.lev_ptr[lv], tb = P.lev_big[lv], t1 = P.lev_ptr[lv + 1];
+  for (int lv = 0; lv < n_levels; ++lv) {
+    const int t0 = lev_ptr[lv], tb = lev_big[lv], t1 = lev_ptr[lv + 1];
     // long tasks: one warp each, products split over the lanes
     for (int t = t0 + gwarp; t < tb; t += nwarps) {
-      const int4 r = P.task_rec[t];
+      const int4 r = task_rec[t];
       T acc_p = T(0);
       for (int q = lane; q < r.w; q += 32) {
-        const int2 pr = P.pairs[r.z + q];
+        const int2 pr = pairs[r.z + q];
         acc_p += HV[pr.x] * HV[pr.y];
       }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) acc_p += __shfl_xor_sync(0xffffffffu, acc_p, o);
       if (lane == 0) {
         T acc = (r.y ? HV[r.x] : T(0)) - acc_p;
-        if (r.x < P.p) acc = clamp_pivot(acc, pfloor);
+        if (r.x < p) acc = clamp_pivot(acc, pfloor);
         HV[r.x] = acc;
       }
     }
@@ -154,7 +163,7 @@ __device__ __noinline__ void head_lu(const DevPlan P, T* HV, const double pfloor
 #pragma unroll
       for (int u = 0; u < TU; ++u) {
         const int tu = t + u * nthreads;
-        r[u] = tu < t1 ? P.task_rec[tu] : make_int4(-1, 0, 0, 0);
+        r[u] = tu < t1 ? task_rec[tu] : make_int4(-1, 0, 0, 0);
       }
       int2 pr[TU][QU];
       auto load_pairs = [&](int q) {
@@ -162,7 +171,7 @@ __device__ __noinline__ void head_lu(const DevPlan P, T* HV, const double pfloor
         for (int u = 0; u < TU; ++u)
 #pragma unroll
           for (int h = 0; h < QU; ++h)
-            pr[u][h] = q + h < r[u].w ? P.pairs[r[u].z + 32 * (q + h)] : make_int2(-1, 0);
+            pr[u][h] = q + h < r[u].w ? pairs[r[u].z + 32 * (q + h)] : make_int2(-1, 0);
       };
       load_pairs(0);
 #pragma unroll
@@ -186,17 +195,17 @@ __device__ __noinline__ void head_lu(const DevPlan P, T* HV, const double pfloor
 #pragma unroll
       for (int u = 0; u < TU; ++u) {
         if (r[u].x < 0) continue;
-        if (r[u].x < P.p) acc[u] = clamp_pivot(acc[u], pfloor);
+        if (r[u].x < p) acc[u] = clamp_pivot(acc[u], pfloor);
         HV[r[u].x] = acc[u];
       }
     }
     barrier();
-    const int d1 = P.div_ptr[lv + 1];
-    for (int t = P.div_ptr[lv] + gtid; t < d1; t += TU * nthreads) {
+    const int d1 = div_ptr[lv + 1];
+    for (int t = div_ptr[lv] + gtid; t < d1; t += TU * nthreads) {
       int2 r[TU];
       T x[TU], d[TU];
 #pragma unroll
-      for (int u = 0; u < TU; ++u) r[u] = t + u * nthreads < d1 ? P.div_rec[t + u * nthreads] : make_int2(-1, 0);
+      for (int u = 0; u < TU; ++u) r[u] = t + u * nthreads < d1 ? div_rec[t + u * nthreads] : make_int2(-1, 0);
 #pragma unroll
       for (int u = 0; u < TU; ++u) {
         x[u] = r[u].x >= 0 ? HV[r[u].x] : T(0);
@@ -212,57 +221,88 @@ __device__ __noinline__ void head_lu(const DevPlan P, T* HV, const double pfloor
 
 // Schur update of the dense tail: S <- -(sum of the head's contributions),
 // whole rows (the tail's J coefficients are added afterwards, fill_tail).
-// Warp per tail row, the row's sum in shared memory (scratch: the dense LU's,
-// dense_smem_elems values, divided among the warps; a tail wider than a
-// warp's share takes several passes over the columns).  A chunk is up to 32
-// columns of one supernode: they differ, so the lanes add to the row without
-// conflicts, and its U values and columns are consecutive.  Bound by load
-// latency: 32 records and their L values come in two loads, and CU chunks'
-// columns and U values are in flight together (no branch between the loads).
-// The chunks are added in supernode order.  (One lane per target column,
-// summing the column's contributions one dependent load after another, left
-// the warp waiting for the row's diagonal entries, up to 43 of them.)
+// A warp takes two tail rows at a time, each summed in shared memory (scratch:
+// the dense LU's, dense_smem_elems values, divided among the warps' rows; a
+// wider tail takes several passes over the columns) and written once.  A
+// chunk is up to 32 columns of one supernode: they differ, so the lanes add to
+// the row without conflicts, and its U values are consecutive.  The chunks of
+// a row are added in supernode order.  Bound by the chain and the instructions
+// of a chunk (17 columns on average): so a lane reads all it needs of a chunk
+// in one 16-byte record (column, U and L positions), loaded ahead, and the two
+// rows' additions overlap.  (Records shared by the warp and handed out by
+// shuffles, one row at a time: 15.8e9 SM cycles of a 2000-bus FP64 sweep; one
+// lane per target column, summing its contributions one dependent load after
+// another: 37e9.)
 template <typename T>
-__device__ __noinline__ void schur_update(const DevPlan P, const T* __restrict__ HV, T* __restrict__ S,
+__device__ __noinline__ void schur_update(const DevPlan& P, const T* __restrict__ HV, T* __restrict__ S,
                                           T* __restrict__ scratch, int part = 0, int parts = 1) {
-  constexpr int CAP = dense_smem_elems<T>() / NWARP;
-  constexpr int CU = 8;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  T* acc = scratch + warp * CAP;
-  // with parts > 1 the CTAs of a cluster take every parts-th warp's rows
-  for (int ti = part * NWARP + warp; ti < P.nt; ti += parts * NWARP) {
-    T* Srow = S + (int64_t)ti * P.ld;
-    const int c0 = P.sc_ptr[ti], c1 = P.sc_ptr[ti + 1];
-    for (int b0 = 0; b0 < P.ld; b0 += CAP) {
-      const int nb = min(CAP, P.ld - b0);
-      for (int i = lane; i < nb; i += 32) acc[i] = T(0);
+  constexpr int RW = 2;  // rows per warp at a time
+  constexpr int CU = 2;  // chunks of each in flight
+  constexpr int CAP = dense_smem_elems<T>() / (NWARP * RW);
+  const int* __restrict__ sc_ptr = P.sc_ptr;
+  const int2* __restrict__ sc_rec = P.sc_rec;
+  const int2* __restrict__ sc_lane = P.sc_lane;
+  const int nt = P.nt, ld = P.ld;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  T* acc = scratch + warp * RW * CAP;
+  // with parts > 1 the warps of all CTAs of a cluster share the rows
+  for (int t0 = (part * NWARP + warp) * RW; t0 < nt; t0 += parts * NWARP * RW) {
+    int c0[RW], c1[RW], n_max = 0;
+#pragma unroll
+    for (int r = 0; r < RW; ++r) {
+      c0[r] = t0 + r < nt ? sc_ptr[t0 + r] : 0;
+      c1[r] = t0 + r < nt ? sc_ptr[t0 + r + 1] : 0;
+      n_max = max(n_max, c1[r] - c0[r]);
+    }
+    for (int b0 = 0; b0 < ld; b0 += CAP) {
+      const int nb = min(CAP, ld - b0);
+      int2 rec[RW][CU], own[RW][CU];
+      auto load = [&](int j) {
+#pragma unroll
+        for (int r = 0; r < RW; ++r)
+#pragma unroll
+          for (int u = 0; u < CU; ++u) {
+            const int c = c0[r] + j + u;
+            rec[r][u] = c < c1[r] ? sc_rec[c] : make_int2(0, 0);
+            own[r][u] = c < c1[r] ? sc_lane[(int64_t)c * 32 + lane] : make_int2(-1, 0);
+          }
+      };
+      load(0);
+#pragma unroll
+      for (int r = 0; r < RW; ++r)
+        for (int i = lane; i < nb; i += 32) acc[r * CAP + i] = T(0);
       __syncwarp();
-      for (int c = c0; c < c1; c += 32) {
-        const int4 mine = c + lane < c1 ? P.sc_rec[c + lane] : make_int4(0, 0, 0, 0);
-        const T ml0 = HV[mine.x], ml1 = (mine.w & 1) ? HV[mine.x + 1] : T(0);
-        const int cnt = min(32, c1 - c);
-        for (int j = 0; j < cnt; j += CU) {
-          int col[CU];
-          T u0[CU], u1[CU];
+      for (int j = 0; j < n_max; j += CU) {
+        T u0[RW][CU], u1[RW][CU], l0[RW][CU], l1[RW][CU];
+        int col[RW][CU];
+#pragma unroll
+        for (int r = 0; r < RW; ++r)
 #pragma unroll
           for (int u = 0; u < CU; ++u) {
-            const int y = __shfl_sync(0xffffffffu, mine.y, j + u) + lane;
-            const int z = __shfl_sync(0xffffffffu, mine.z, j + u) + lane;
-            const int f = __shfl_sync(0xffffffffu, mine.w, j + u);
-            const bool in = lane < ((f >> 1) & 63);
-            col[u] = in ? P.tidx[z] : -1;
-            u0[u] = in ? HV[y] : T(0);
-            u1[u] = in && (f & 1) ? HV[y + (f >> 7)] : T(0);
+            const int2 q = rec[r][u], o = own[r][u];
+            const bool in = o.x >= 0, two = in && q.y > 0;
+            col[r][u] = o.x;
+            l0[r][u] = in ? HV[q.x] : T(0);
+            u0[r][u] = in ? HV[o.y] : T(0);
+            l1[r][u] = two ? HV[q.x + 1] : T(0);
+            u1[r][u] = two ? HV[o.y + q.y] : T(0);
           }
+        load(j + CU);
 #pragma unroll
-          for (int u = 0; u < CU; ++u) {
-            const T l0 = __shfl_sync(0xffffffffu, ml0, j + u), l1 = __shfl_sync(0xffffffffu, ml1, j + u);
-            if (col[u] >= b0 && col[u] < b0 + nb) acc[col[u] - b0] += l0 * u0[u] + l1 * u1[u];
-            __syncwarp();
+        for (int u = 0; u < CU; ++u) {
+#pragma unroll
+          for (int r = 0; r < RW; ++r) {
+            const int c = col[r][u] - b0;
+            if (col[r][u] >= 0 && c >= 0 && c < nb)
+              acc[r * CAP + c] += l0[r][u] * u0[r][u] + l1[r][u] * u1[r][u];
           }
+          __syncwarp();
         }
       }
-      for (int i = lane; i < nb; i += 32) Srow[b0 + i] = T(0) - acc[i];
+#pragma unroll
+      for (int r = 0; r < RW; ++r)
+        if (t0 + r < nt)
+          for (int i = lane; i < nb; i += 32) S[(int64_t)(t0 + r) * ld + b0 + i] = T(0) - acc[r * CAP + i];
       __syncwarp();
     }
   }
@@ -690,9 +730,111 @@ __device__ __forceinline__ void tail_inverse_product(const T* Sinv, int64_t ld, 
   }
 }
 
+// A warp's walk over its slices of lists [.., l1): list l, slice s of it; the
+// next slice is NWARP further in the list or the warp's first one of a later
+// list.
+struct SliceCursor {
+  const int* lev;
+  int l1, l, s;
+  __device__ __forceinline__ SliceCursor(const int* lev_, int l0, int l1_, int warp) : lev(lev_), l1(l1_), l(l0) {
+    s = lev[l0] + warp;
+    settle(warp);
+  }
+  __device__ __forceinline__ void settle(int warp) {
+    while (l < l1 && s >= lev[l + 1]) {
+      ++l;
+      s = lev[l] + warp;
+    }
+  }
+  __device__ __forceinline__ void next(int warp) {
+    if (l >= l1) return;
+    s += NWARP;
+    settle(warp);
+  }
+};
+
+// Lists [l0, l1) of the plan's slices for one right-hand side, a barrier after
+// each: y[row] -= sum of HV[pos] * y[col] over the row's entries, with DIV
+// also divided by the row's pivot HV[row].  A slice per warp, 1 to 32 lanes per
+// row, so that a lane has at most four entries (see plan.hpp): a list waits for
+// the one before it, and one thread's walk along the longest row (20 to 80
+// entries) used to set the time of each.  A warp's next slices are loaded
+// ahead of the barriers: the record two slices ahead, columns and positions
+// with it one ahead, so that behind a barrier only the gathers remain.
+template <typename T, bool DIV>
+__device__ __noinline__ void row_lists(const DevPlan& P, const T* __restrict__ HV, T* y, const int l0, const int l1) {
+  constexpr int PF = 4;  // entries per lane and batch
+  const int* __restrict__ lev = P.sl_lev;
+  const int4* __restrict__ rec = P.sl_rec;
+  const int* __restrict__ cols = P.sl_col;
+  const int* __restrict__ poss = P.sl_pos;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  struct Batch {
+    int col[PF];
+    T v[PF];
+  };
+  auto record = [&](const SliceCursor& c) {
+    return c.l < l1 ? rec[c.s * 32 + lane] : make_int4(-1, 0, 0, 1);
+  };
+  auto load = [&](const int4& r, int q, Batch& b) {
+    int pos[PF];
+#pragma unroll
+    for (int h = 0; h < PF; ++h) {
+      b.col[h] = q + h < r.y ? cols[r.z + 32 * (q + h)] : -1;
+      pos[h] = q + h < r.y ? poss[r.z + 32 * (q + h)] : 0;
+    }
+#pragma unroll
+    for (int h = 0; h < PF; ++h) b.v[h] = b.col[h] >= 0 ? HV[pos[h]] : T(0);
+  };
+  auto run = [&](const int4& r, Batch b, T d) {
+    T acc = T(0);
+    for (int q = 0;;) {
+      T x[PF];
+#pragma unroll
+      for (int h = 0; h < PF; ++h) x[h] = b.col[h] >= 0 ? y[b.col[h]] : T(0);
+#pragma unroll
+      for (int h = 0; h < PF; ++h) acc += b.v[h] * x[h];
+      q += PF;
+      if (q >= r.y) break;
+      load(r, q, b);
+    }
+    for (int o = 1; o < r.w; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);  // r.w: the same in a slice
+    if (r.x >= 0 && (lane & (r.w - 1)) == 0) {
+      const T v = y[r.x] - acc;
+      y[r.x] = DIV ? v / d : v;
+    }
+  };
+  SliceCursor a(lev, l0, l1, warp), c = a;
+  int4 ra = record(a);
+  Batch ba;
+  load(ra, 0, ba);
+  T da = DIV && ra.x >= 0 ? HV[ra.x] : T(1);
+  c.next(warp);
+  int4 rc = record(c);
+  for (int l = l0; l < l1; ++l) {
+    while (a.l == l) {
+      Batch bn;
+      load(rc, 0, bn);
+      const T dn = DIV && rc.x >= 0 ? HV[rc.x] : T(1);
+      SliceCursor n = c;
+      n.next(warp);
+      const int4 rn = record(n);
+      run(ra, ba, da);
+      a = c;
+      ra = rc;
+      ba = bn;
+      da = dn;
+      c = n;
+      rc = rn;
+    }
+    __syncthreads();
+  }
+}
+
 // y <- (LU)^-1 y with a factor (head values fHV, dense tail fS): forward
 // over the head levels, the tail rows against the head, the dense tail
-// forward + backward, backward over the head levels.  With Minv (the
+// forward + backward, the head rows against the tail, backward over the head
+// levels.  With Minv (the
 // factor's explicit inverse, column c at Minv + c * dim, in the plan's
 // ordering) the dense tail is applied as a product with its tail block,
 // which is the inverse of the dense Schur complement.
@@ -700,23 +842,9 @@ template <typename T>
 __device__ __forceinline__ void apply_factor(const DevPlan& P, const T* fHV, const T* fS, T* y, T* s_blk, T* s_dense,
                                              PhaseProf& prof, const T* Minv = nullptr) {
   const int tid = threadIdx.x;
-  for (int lv = 0; lv < P.n_levels; ++lv) {
-    for (int q0 = P.lev_piv_ptr[lv] + tid; q0 < P.lev_piv_ptr[lv + 1]; q0 += BS) {
-      const int i = P.lev_piv[q0];
-      T acc = y[i];
-      for (int q = P.fw_ptr[i]; q < P.fw_ptr[i + 1]; ++q) acc -= fHV[P.fw_pos[q]] * y[P.fw_col[q]];
-      y[i] = acc;
-    }
-    __syncthreads();
-  }
+  row_lists<T, false>(P, fHV, y, 0, P.n_levels);
   prof.mark(PH_SOLVE);
-  for (int ti = tid; ti < P.nt; ti += BS) {
-    const int i = P.p + ti;
-    T acc = y[i];
-    for (int q = P.fw_ptr[i]; q < P.fw_ptr[i + 1]; ++q) acc -= fHV[P.fw_pos[q]] * y[P.fw_col[q]];
-    y[i] = acc;
-  }
-  __syncthreads();
+  row_lists<T, false>(P, fHV, y, P.n_levels, P.n_levels + 1);
   prof.mark(PH_SOLVE_TAIL);
   if (P.nt > 0 && Minv != nullptr && P.nt <= dense_smem_elems<T>()) {
     for (int i = tid; i < P.nt; i += BS) s_dense[i] = y[P.p + i];
@@ -732,16 +860,8 @@ __device__ __forceinline__ void apply_factor(const DevPlan& P, const T* fHV, con
     dense_solves<T>(fS, P.nt, P.ld, y + P.p, s_blk, ys, sbuf);
   }
   prof.mark(PH_SOLVE_DENSE);
-  for (int lv = P.n_levels - 1; lv >= 0; --lv) {
-    for (int q0 = P.lev_piv_ptr[lv] + tid; q0 < P.lev_piv_ptr[lv + 1]; q0 += BS) {
-      const int k = P.lev_piv[q0];
-      T acc = y[k];
-      for (int q = P.bw_ptr[k]; q < P.bw_ptr[k + 1]; ++q) acc -= fHV[P.bw_pos[q]] * y[P.bw_row[q]];
-      y[k] = acc / fHV[k];
-    }
-    __syncthreads();
-  }
-
+  row_lists<T, false>(P, fHV, y, P.n_levels + 1, P.n_levels + 2);
+  row_lists<T, true>(P, fHV, y, P.n_levels + 2, 2 * P.n_levels + 2);
   prof.mark(PH_SOLVE_BACK);
 }
 
@@ -764,7 +884,7 @@ struct RowShared {
 
 // ||F||inf of the row (row-patched Ybus, its Sbus) at voltage Vx, NaN-sticky,
 // without touching the row's workspace
-__device__ __noinline__ double mismatch_norm(const DevPlan P, const RowEdits ed, const double2* Y, const double2* Vx,
+__device__ __noinline__ double mismatch_norm(const DevPlan& P, const RowEdits ed, const double2* Y, const double2* Vx,
                                              const double2* sb, double* s_red) {
   double lmax = 0.0;
   for (int i = threadIdx.x; i < P.n_bus; i += BS) {
@@ -786,7 +906,7 @@ __device__ __noinline__ double mismatch_norm(const DevPlan P, const RowEdits ed,
 // Va conj(Y Va) on the unedited Ybus is shared by all rows, and a row's
 // edits change S only at the buses of the edited Ybus rows, by
 // Va_i conj(dY_k Va_j) per edited entry k = (i, j).
-__device__ __noinline__ double alt_mismatch_norm(const DevPlan P, const RowEdits ed, const double2* Va,
+__device__ __noinline__ double alt_mismatch_norm(const DevPlan& P, const RowEdits ed, const double2* Va,
                                                  const double2* Sa, const double2* sb, double* s_red) {
   double lmax = 0.0;
   for (int i = threadIdx.x; i < P.n_bus; i += BS) {
@@ -813,7 +933,7 @@ __device__ __noinline__ double alt_mismatch_norm(const DevPlan P, const RowEdits
 // Returns false (no compensation) when the row touches too many positions.
 // Run by a CTA of NT threads.
 template <typename T, int NT = BS>
-__device__ __noinline__ bool setup_compensation(const DevPlan P, const RowEdits ed, const double2* Y,
+__device__ __noinline__ bool setup_compensation(const DevPlan& P, const RowEdits ed, const double2* Y,
                                                 const double2* Vb, const T* Minv, const RowShared<T> sh) {
   const int tid = threadIdx.x;
   int* R = sh.s_cr + 1;
@@ -928,7 +1048,8 @@ struct CompRec {
 // in the same order, so the record equals what the refill would compute),
 // then the record.
 template <typename T>
-__global__ void __launch_bounds__(32) comp_setup_kernel(const DevPlan P, const SweepArgs a, CompRec* rec) {
+__global__ void __launch_bounds__(32) comp_setup_kernel(const __grid_constant__ DevPlan P,
+                                                         const __grid_constant__ SweepArgs a, CompRec* rec) {
   __shared__ int s_ek[MAX_EDITS];
   __shared__ double2 s_ev[MAX_EDITS];
   __shared__ int s_cr[1 + MAX_COMP];
@@ -1044,7 +1165,7 @@ __device__ __noinline__ void apply_compensation(int dim, T* y, const T* Minv, co
 // check_limit_violations passes): per branch loading = max(|S_from|, |S_to|)
 // / rate (0 for tripped or unlimited branches, NaN when not converged), the
 // number of branches above 1 and the largest loading.
-__device__ __noinline__ void row_flows(const SweepArgs a, const int row, const double2* V, const bool ok,
+__device__ __noinline__ void row_flows(const SweepArgs& a, const int row, const double2* V, const bool ok,
                                        double* s_red) {
   const int tid = threadIdx.x;
   const int q0 = a.trip_ptr != nullptr ? a.trip_ptr[row] : 0;
@@ -1086,7 +1207,7 @@ __device__ __noinline__ void row_flows(const SweepArgs a, const int row, const d
 }
 
 // Outputs of a row that is not simulated (its outage islands the grid).
-__device__ __noinline__ void skip_row_outputs(const SweepArgs a, const int row, const int n) {
+__device__ __noinline__ void skip_row_outputs(const SweepArgs& a, const int row, const int n) {
   const int tid = threadIdx.x;
   double2* vout = reinterpret_cast<double2*>(a.v_out) + (int64_t)row * n;
   for (int i = tid; i < n; i += BS) vout[i] = make_double2(NAN, NAN);
@@ -1447,7 +1568,8 @@ template <typename T>
 #ifndef GS2G_MIN_CTAS_PER_SM
 #define GS2G_MIN_CTAS_PER_SM 2
 #endif
-__global__ void __launch_bounds__(BS, GS2G_MIN_CTAS_PER_SM) sweep_kernel(const DevPlan P, const SweepArgs a) {
+__global__ void __launch_bounds__(BS, GS2G_MIN_CTAS_PER_SM) sweep_kernel(const __grid_constant__ DevPlan P,
+                                                                         const __grid_constant__ SweepArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_row;
   __shared__ int s_ne;
@@ -1521,9 +1643,33 @@ __device__ __forceinline__ unsigned cluster_nctarank() {
   return r;
 }
 
+// The other CTAs of a cluster while its leader runs a row: each command's
+// share of the factorization in the row's workspace, until the row is done.
+template <typename T>
+__device__ __forceinline__ void cluster_help(const DevPlan& P, double pivot_floor, char* ws, T* smem, const int* cmd,
+                                             int rank, int parts) {
+  const WsLayout L = ws_layout<T>(P);
+  T* S = reinterpret_cast<T*>(ws + L.S);
+  T* HV = reinterpret_cast<T*>(ws + L.HV);
+  for (;;) {
+    cluster_barrier();
+    const int c = ld_shared_rank0(cmd);
+    cluster_barrier();
+    if (c != CLUSTER_CMD_LU) break;
+    // the leader's Jacobian values are in place (posted after them): the
+    // head LU's share of each level, the Schur rows, two barriers (rows
+    // complete, J's tail coefficients added), then the shared dense LU
+    head_lu<T>(P, HV, pivot_floor, rank, parts);
+    schur_update<T>(P, HV, S, smem, rank, parts);
+    cluster_barrier();
+    cluster_barrier();  // the leader has added J's tail coefficients
+    dense_lu_cluster<T>(S, P.nt, P.ld, smem, pivot_floor, rank, parts);
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(BS, GS2G_MIN_CTAS_PER_SM)
-    sweep_kernel_cluster(const DevPlan P, const SweepArgs a) {
+    sweep_kernel_cluster(const __grid_constant__ DevPlan P, const __grid_constant__ SweepArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_row;
   __shared__ int s_cmd;
@@ -1562,8 +1708,6 @@ __global__ void __launch_bounds__(BS, GS2G_MIN_CTAS_PER_SM)
   }
   // one workspace per cluster
   char* ws = a.workspace + (int64_t)(blockIdx.x / parts) * a.ws_stride;
-  T* S = reinterpret_cast<T*>(ws + ws_layout<T>(P).S);
-  T* HV = reinterpret_cast<T*>(ws + ws_layout<T>(P).HV);
   prof.init(a.phase_cycles != nullptr && threadIdx.x == 0 && rank == 0);
   const ClusterLu cl{&s_cmd, parts};
   for (;;) {
@@ -1578,20 +1722,7 @@ __global__ void __launch_bounds__(BS, GS2G_MIN_CTAS_PER_SM)
       cluster_barrier();
       cluster_barrier();
     } else {
-      for (;;) {
-        cluster_barrier();
-        const int cmd = ld_shared_rank0(&s_cmd);
-        cluster_barrier();
-        if (cmd != CLUSTER_CMD_LU) break;
-        // the leader's Jacobian values are in place (posted after them): the
-        // head LU's share of each level, the Schur rows, two barriers (rows
-        // complete, J's tail coefficients added), then the shared dense LU
-        head_lu<T>(P, HV, a.pivot_floor, rank, parts);
-        schur_update<T>(P, HV, S, reinterpret_cast<T*>(smem_raw), rank, parts);
-        cluster_barrier();
-        cluster_barrier();  // the leader has added J's tail coefficients
-        dense_lu_cluster<T>(S, P.nt, P.ld, reinterpret_cast<T*>(smem_raw), a.pivot_floor, rank, parts);
-      }
+      cluster_help<T>(P, a.pivot_floor, ws, reinterpret_cast<T*>(smem_raw), &s_cmd, rank, parts);
     }
   }
   prof.flush(a.phase_cycles);
@@ -1657,6 +1788,70 @@ __global__ void __launch_bounds__(BS, GS2G_MIN_CTAS_PER_SM)
   }
 }
 
+// The hand-offs of a multi-grid chord sweep with a cluster of CTAs per row:
+// the queue of sweep_kernel_multi (row_list), the protocol of
+// sweep_kernel_cluster.  Every CTA of a cluster holds the row's grid; rows
+// whose dense tail is too small to share (below min_tail) are run by their
+// leader alone.
+template <typename T>
+__global__ void __launch_bounds__(BS, GS2G_MIN_CTAS_PER_SM)
+    sweep_kernel_multi_cluster(const GridEntry* __restrict__ grids, int n_grids, const int* __restrict__ row_begin,
+                               int n_entries, int* queue, char* workspace, int64_t ws_stride,
+                               unsigned long long* phase_cycles, const int* __restrict__ row_list, int min_tail) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int s_row;
+  __shared__ int s_cmd;
+  __shared__ int s_ne;
+  __shared__ int s_ek[MAX_EDITS];
+  __shared__ double2 s_ev[MAX_EDITS];
+  __shared__ double s_red[NWARP];
+  __shared__ T s_blk[64];
+  __shared__ __align__(16) GridEntry s_grid;
+  __shared__ int s_cr[1 + MAX_COMP];
+  __shared__ double s_cB[MAX_COMP * MAX_COMP];
+  __shared__ double s_cLU[MAX_COMP * MAX_COMP];
+  __shared__ int s_cpiv[MAX_COMP];
+  __shared__ double s_cw[MAX_COMP];
+  const RowShared<T> sh{&s_ne, s_ek, s_ev, s_red, s_blk, reinterpret_cast<T*>(smem_raw), s_cr, s_cB, s_cLU, s_cpiv,
+                        s_cw};
+  const int rank = (int)cluster_ctarank();
+  const int parts = (int)cluster_nctarank();
+  char* ws = workspace + (int64_t)(blockIdx.x / parts) * ws_stride;
+  PhaseProf prof;
+  prof.init(phase_cycles != nullptr && threadIdx.x == 0 && rank == 0);
+  const ClusterLu cl{&s_cmd, parts};
+  int cur = -1;
+  for (;;) {
+    if (rank == 0 && threadIdx.x == 0) s_row = atomicAdd(queue, 1);
+    cluster_barrier();
+    const int q = ld_shared_rank0(&s_row);
+    cluster_barrier();
+    if (q >= n_entries) break;
+    const int entry = row_list[q];
+    const int flag = entry & NO_RESCUE_BIT;
+    const int row = entry & ~NO_RESCUE_BIT;
+    int g = 0;
+    while (g + 1 < n_grids && row >= row_begin[g + 1]) ++g;
+    if (g != cur) {
+      const int* src = reinterpret_cast<const int*>(grids + g);
+      int* dst = reinterpret_cast<int*>(&s_grid);
+      for (int i = threadIdx.x; i < (int)(sizeof(GridEntry) / sizeof(int)); i += BS) dst[i] = src[i];
+      __syncthreads();
+      cur = g;
+    }
+    if (rank == 0) {
+      solve_row<T>(s_grid.P, s_grid.a, (row - row_begin[g]) | flag, ws, sh, prof,
+                   s_grid.P.nt >= min_tail ? &cl : nullptr);
+      if (threadIdx.x == 0) s_cmd = CLUSTER_CMD_DONE;
+      cluster_barrier();
+      cluster_barrier();
+    } else {
+      cluster_help<T>(s_grid.P, s_grid.a.pivot_floor, ws, reinterpret_cast<T*>(smem_raw), &s_cmd, rank, parts);
+    }
+  }
+  prof.flush(phase_cycles);
+}
+
 #include "chord_sweep.cuh"
 #include "adjoint.cuh"
 
@@ -1692,6 +1887,16 @@ cudaError_t opt_in_smem() {
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(sweep_kernel_cluster<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            smem_bytes<double>());
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(sweep_kernel_multi_cluster<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           smem_bytes<float>());
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(sweep_kernel_multi_cluster<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           smem_bytes<double>());
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(sweep_kernel_multi_cluster<float>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(sweep_kernel_multi_cluster<double>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(sweep_kernel_cluster<float>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;
@@ -1779,8 +1984,8 @@ int launch_comp_setup(const DevPlan& P, const SweepArgs& a, int prec, int n_rows
 
 int launch_chord(const DevPlan& P, const SweepArgs& a, int prec, int n_ctas, void* stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (n_ctas <= 0 || a.base_ws == nullptr || a.base_inv == nullptr || a.base_fwv == nullptr ||
-      a.base_bwv == nullptr || a.handoff == nullptr || a.n_handoff == nullptr || a.fixed_iters)
+  if (n_ctas <= 0 || a.base_ws == nullptr || a.base_inv == nullptr || a.base_slv == nullptr ||
+      a.handoff == nullptr || a.n_handoff == nullptr || a.fixed_iters || a.chord_slots < 1 || a.chord_slots > CK)
     return (int)cudaErrorInvalidValue;
   if (prec == 1 && chord_use_ysmem<float>(P)) {
     const int sm = chord_smem_bytes_ysmem<float>(P);
@@ -1828,29 +2033,65 @@ int launch_adjoint(const DevPlan& P, const SweepArgs& a, const double* rhs, doub
 
 int handoff_cluster_size() { return HANDOFF_CLUSTER; }
 
+namespace {
+// Clusters of 2, 4, 8 or 16 CTAs over n_ctas.
+struct ClusterLaunch {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[1];
+  ClusterLaunch(int prec, int cluster, int n_ctas, cudaStream_t st) {
+    cfg.gridDim = dim3((unsigned)n_ctas, 1, 1);
+    cfg.blockDim = dim3(BS, 1, 1);
+    cfg.dynamicSmemBytes = prec == 1 ? smem_bytes<float>() : smem_bytes<double>();
+    cfg.stream = st;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)cluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+  }
+};
+bool cluster_ok(int cluster, int n_ctas) {
+  return (cluster == 2 || cluster == 4 || cluster == 8 || cluster == 16) && n_ctas > 0 && n_ctas % cluster == 0;
+}
+}  // namespace
+
+int max_clusters(int prec, int cluster) {
+  if (!cluster_ok(cluster, cluster) || opt_in_smem() != cudaSuccess) return 0;
+  ClusterLaunch l(prec, cluster, cluster, nullptr);
+  int n = 0;
+  const cudaError_t e = prec == 1 ? cudaOccupancyMaxActiveClusters(&n, sweep_kernel_cluster<float>, &l.cfg)
+                                  : cudaOccupancyMaxActiveClusters(&n, sweep_kernel_cluster<double>, &l.cfg);
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // the size is not available here: not an error of the caller's
+    return 0;
+  }
+  return n;
+}
+
 int launch_sweep_cluster(const DevPlan& P, const SweepArgs& a, int prec, int cluster, int n_ctas, void* stream) {
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if ((cluster != 8 && cluster != 16) || n_ctas <= 0 || n_ctas % cluster != 0 || a.inverse_out != nullptr ||
-      a.factor_only)
+  if (!cluster_ok(cluster, n_ctas) || a.inverse_out != nullptr || a.factor_only) return (int)cudaErrorInvalidValue;
+  cudaError_t e = opt_in_smem();
+  if (e != cudaSuccess) return (int)e;
+  ClusterLaunch l(prec, cluster, n_ctas, static_cast<cudaStream_t>(stream));
+  e = prec == 1 ? cudaLaunchKernelEx(&l.cfg, sweep_kernel_cluster<float>, P, a)
+                : cudaLaunchKernelEx(&l.cfg, sweep_kernel_cluster<double>, P, a);
+  if (e != cudaSuccess) return (int)e;
+  return (int)cudaGetLastError();
+}
+
+int launch_sweep_multi_cluster(const GridEntry* d_grids, int n_grids, const int* d_row_begin, int n_entries, int* queue,
+                               char* workspace, int64_t ws_stride, unsigned long long* phase_cycles, int prec,
+                               int cluster, int n_ctas, void* stream, const int* row_list, int min_tail) {
+  if (!cluster_ok(cluster, n_ctas) || n_grids <= 0 || n_grids > MAX_GRIDS || row_list == nullptr)
     return (int)cudaErrorInvalidValue;
   cudaError_t e = opt_in_smem();
   if (e != cudaSuccess) return (int)e;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)n_ctas, 1, 1);
-  cfg.blockDim = dim3(BS, 1, 1);
-  cfg.dynamicSmemBytes = prec == 1 ? smem_bytes<float>() : smem_bytes<double>();
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)cluster;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (prec == 1)
-    e = cudaLaunchKernelEx(&cfg, sweep_kernel_cluster<float>, P, a);
-  else
-    e = cudaLaunchKernelEx(&cfg, sweep_kernel_cluster<double>, P, a);
+  ClusterLaunch l(prec, cluster, n_ctas, static_cast<cudaStream_t>(stream));
+  e = prec == 1 ? cudaLaunchKernelEx(&l.cfg, sweep_kernel_multi_cluster<float>, d_grids, n_grids, d_row_begin,
+                                     n_entries, queue, workspace, ws_stride, phase_cycles, row_list, min_tail)
+                : cudaLaunchKernelEx(&l.cfg, sweep_kernel_multi_cluster<double>, d_grids, n_grids, d_row_begin,
+                                     n_entries, queue, workspace, ws_stride, phase_cycles, row_list, min_tail);
   if (e != cudaSuccess) return (int)e;
   return (int)cudaGetLastError();
 }

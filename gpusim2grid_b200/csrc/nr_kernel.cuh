@@ -29,15 +29,9 @@ struct DevPlan {
   const int2* div_rec;   // L entries by level: HV position, HV position of its pivot
   const int* lev_piv_ptr;  // [n_levels + 1] into lev_piv
   const int* lev_piv;      // head pivots by level
-  const int* tidx;     // tail columns of the Schur chunks
   const int* sc_ptr;   // [nt + 1] Schur chunks per tail row
-  const int4* sc_rec;  // per chunk: L position, U position, offset into tidx, h | n << 1 | t << 7
-  const int* fw_ptr;  // [dim + 1]
-  const int* fw_col;
-  const int* fw_pos;
-  const int* bw_ptr;  // [p + 1]
-  const int* bw_row;
-  const int* bw_pos;
+  const int2* sc_rec;   // per chunk: L position, U stride or 0 (see plan.hpp)
+  const int2* sc_lane;  // [32 per chunk]: tail column or -1, U position
   // transposed solves (see plan.hpp) and the J-index -> factor position map
   const int* ut_ptr;
   const int* ut_row;
@@ -46,6 +40,15 @@ struct DevPlan {
   const int* lt_row;
   const int* lt_pos;
   const int* iperm;
+  // slices of the solves and of Ybus (see plan.hpp)
+  const int* sl_lev;
+  const int4* sl_rec;
+  const int* sl_col;
+  const int* sl_pos;
+  int n_ysl;          // Ybus slices
+  const int4* yl_rec;
+  const int* yl_col;
+  const double2* yl_val;  // base Ybus values in slice order
 };
 
 // One launch = one sweep over a list of rows.
@@ -122,9 +125,9 @@ struct SweepArgs {
   const double* base_v;  // complex [n_bus]: the voltage the base factor was taken at
   const char* base_inv;  // [dim x dim] of the sweep's type: column c = M0^-1 e_c (outage compensation)
   // the base factor's head values in solve order (of the sweep's type):
-  // base_fwv[q] = HV[fw_pos[q]], base_bwv[q] = HV[bw_pos[q]] (nullptr: gather)
-  const char* base_fwv;
-  const char* base_bwv;
+  // base_slv[e] = HV[sl_pos[e]] (the slices' order)
+  const char* base_slv;
+  int chord_slots;  // rows a chord CTA holds at a time, 1 .. chord_rows_per_cta()
   char* inverse_out;     // inverse mode: row r of the launch writes column r of M0^-1 here
   int factor_only;
   // branch flows and limit check when the row leaves (loading_out nullptr: off)
@@ -200,11 +203,14 @@ int launch_comp_setup(const DevPlan& P, const SweepArgs& a, int prec, int n_rows
 int sweep_ctas(int prec, int device);
 
 // The single-row sweep (prec 1: FP32 factors, 0: FP64) with a cluster of
-// `cluster` CTAs per row (8, or 16 up to handoff_cluster_size()): the
-// cluster's leading CTA runs the row (its workspace: the leader's block
-// index times ws_stride), and all of them share each of its head LUs, Schur
+// `cluster` CTAs per row (2, 4, 8, or 16 up to handoff_cluster_size()): the
+// cluster's leading CTA runs the row (its workspace: the cluster's index
+// times ws_stride), and all of them share each of its head LUs, Schur
 // updates and dense tail LUs.  n_ctas a multiple of the cluster size.
 int handoff_cluster_size();
+// Clusters of `cluster` CTAs of that sweep that the device holds at once (0: the
+// size is not available).
+int max_clusters(int prec, int cluster);
 
 // Batched adjoint (FP64): lam[r] = J_r^-T rhs[r] for the a.n_rows rows of a
 // sweep (a.v_out the converged voltages, a.status_out their statuses, the
@@ -232,6 +238,15 @@ struct GridEntry {
 int launch_sweep_multi(const GridEntry* d_grids, int n_grids, const int* d_row_begin, int n_rows, int* queue,
                        char* workspace, int64_t ws_stride, unsigned long long* phase_cycles, int prec, int n_ctas,
                        void* stream, const int* row_list = nullptr, const int* n_rows_dev = nullptr);
+
+// The hand-offs (row_list: global row ids, n_entries of them) of a multi-grid
+// chord sweep with `cluster` CTAs per row over n_ctas CTAs (a workspace per
+// cluster); rows whose dense tail is below min_tail are run by one CTA of
+// their cluster.
+int launch_sweep_multi_cluster(const GridEntry* d_grids, int n_grids, const int* d_row_begin, int n_entries, int* queue,
+                               char* workspace, int64_t ws_stride, unsigned long long* phase_cycles, int prec,
+                               int cluster, int n_ctas, void* stream, const int* row_list, int min_tail);
+
 // Multi-grid chord sweep over d_grids (policy 2, every grid with its base
 // factor and inverse; each grid's a.queue its own zeroed counter; a.handoff
 // one list for all grids, a.handoff_base the grid's first global row).

@@ -532,13 +532,15 @@ Plan build_plan(int n_bus, const int* ybus_indptr, const int* ybus_indices,
   for (int ti = 0; ti < P.nt; ++ti) {
     for (int q = P.schur_ptr[ti]; q < P.schur_ptr[ti + 1]; ++q) {
       const int s = P.schur_sn[q], a = P.schur_a[q], w = P.sn_w[s], t = P.sn_t[s];
-      if (t >= (1 << 22)) throw std::logic_error("build_plan: supernode too large for the Schur map");
       for (int k = 0; k < w; k += 2)
-        for (int b = 0; b < t; b += 32)
-          P.sc_rec.insert(P.sc_rec.end(), {P.sn_L[s] + a * w + k, P.sn_U[s] + k * t + b, P.sn_tidx[s] + b,
-                                           (k + 1 < w ? 1 : 0) | (std::min(32, t - b) << 1) | (t << 7)});
+        for (int b = 0; b < t; b += 32) {
+          P.sc_rec.insert(P.sc_rec.end(), {P.sn_L[s] + a * w + k, k + 1 < w ? t : 0});
+          for (int l = b; l < b + 32; ++l)
+            P.sc_lane.insert(P.sc_lane.end(),
+                             {l < t ? P.tidx[P.sn_tidx[s] + l] : -1, l < t ? P.sn_U[s] + k * t + l : 0});
+        }
     }
-    P.sc_ptr[ti + 1] = (int)P.sc_rec.size() / 4;
+    P.sc_ptr[ti + 1] = (int)P.sc_rec.size() / 2;
   }
   for (int64_t k = 0; k < P.nt; ++k) P.dense_madds += (P.nt - 1 - k) * (P.nt - 1 - k);
 
@@ -585,6 +587,74 @@ Plan build_plan(int n_bus, const int* ybus_indptr, const int* ybus_indices,
         P.lt_row[fl[i]] = r;
         P.lt_pos[fl[i]++] = P.fw_pos[q];
       }
+  }
+
+  // ---- slices ---------------------------------------------------------------
+  {
+    struct Row {
+      int row, ptr, len;
+    };
+    std::vector<Row> rows;
+    // rows -> slices appended to rec / col / pos (entry e of a row: e_col, e_pos),
+    // a row over as many lanes (up to `most`) as give each at most four entries
+    auto lanes_of = [](int len, int most) {
+      int g = 1;
+      while (g < most && 4 * g < len) g *= 2;
+      return g;
+    };
+    auto slices = [&](std::vector<int>& rec, std::vector<int>& col, std::vector<int>& pos, int most, auto e_col,
+                      auto e_pos) {
+      std::stable_sort(rows.begin(), rows.end(), [](const Row& a, const Row& b) { return a.len > b.len; });
+      for (size_t s0 = 0; s0 < rows.size();) {
+        const int g = lanes_of(rows[s0].len, most);
+        size_t s1 = s0;
+        while (s1 < rows.size() && s1 < s0 + 32 / g && lanes_of(rows[s1].len, most) == g) ++s1;
+        const int off = (int)col.size(), per = (rows[s0].len + g - 1) / g;
+        col.resize(col.size() + size_t(32) * per, 0);
+        pos.resize(pos.size() + size_t(32) * per, -1);
+        for (int l = 0; l < 32; ++l) {
+          const bool in = s0 + l / g < s1;
+          const Row r = in ? rows[s0 + l / g] : Row{-1, 0, 0};
+          const int sub = l % g, cnt = r.len > sub ? (r.len - sub + g - 1) / g : 0;
+          rec.insert(rec.end(), {r.row, cnt, off + l, g});
+          for (int k = 0; k < cnt; ++k) {
+            col[off + l + 32 * k] = e_col(r.ptr + sub + g * k);
+            pos[off + l + 32 * k] = e_pos(r.ptr + sub + g * k);
+          }
+        }
+        s0 = s1;
+      }
+      rows.clear();
+    };
+    P.sl_lev.assign(1, 0);
+    // the two lists that need no level order have rows enough for every warp: up
+    // to four lanes a row (32 took 1.5 times as long on the tail rows)
+    auto list = [&](auto e_col, auto e_pos, int most = 32) {
+      slices(P.sl_rec, P.sl_col, P.sl_pos, most, e_col, e_pos);
+      P.sl_lev.push_back((int)P.sl_rec.size() / 128);
+    };
+    auto fw_col = [&](int e) { return P.fw_col[e]; };
+    auto fw_pos = [&](int e) { return P.fw_pos[e]; };
+    auto bw_col = [&](int e) { return P.bw_row[e]; };
+    auto bw_pos = [&](int e) { return P.bw_pos[e]; };
+    for (int lv = 0; lv < P.n_levels; ++lv) {
+      for (int k : by_level[lv])
+        if (P.fw_ptr[k + 1] > P.fw_ptr[k]) rows.push_back({k, P.fw_ptr[k], P.fw_ptr[k + 1] - P.fw_ptr[k]});
+      list(fw_col, fw_pos);
+    }
+    for (int i = p; i < d; ++i)
+      if (P.fw_ptr[i + 1] > P.fw_ptr[i]) rows.push_back({i, P.fw_ptr[i], P.fw_ptr[i + 1] - P.fw_ptr[i]});
+    list(fw_col, fw_pos, 4);
+    // a row's head columns come before its tail columns
+    for (int k = 0; k < p; ++k)
+      if ((int)vst[k].size() > nh[k]) rows.push_back({k, P.bw_ptr[k] + nh[k], (int)vst[k].size() - nh[k]});
+    list(bw_col, bw_pos, 4);
+    for (int lv = P.n_levels - 1; lv >= 0; --lv) {
+      for (int k : by_level[lv]) rows.push_back({k, P.bw_ptr[k], nh[k]});
+      list(bw_col, bw_pos);
+    }
+    for (int i = 0; i < n_bus; ++i) rows.push_back({i, P.y_indptr[i], P.y_indptr[i + 1] - P.y_indptr[i]});
+    slices(P.yl_rec, P.yl_col, P.yl_k, 1, [&](int e) { return P.y_indices[e]; }, [](int e) { return e; });
   }
 
   // ---- Jacobian fill map -------------------------------------------------

@@ -90,11 +90,12 @@ struct Plan {
   std::vector<int> schur_ptr, schur_sn, schur_a;
   // The same update as chunks of up to 32 columns of one or two columns of a
   // supernode, the form the device runs: row ti owns chunks [sc_ptr[ti],
-  // sc_ptr[ti+1]), in supernode order; chunk c (four ints at sc_rec[4 c]: L
-  // position x, U position y, offset z into tidx, h | n << 1 | t << 7)
-  // subtracts from S[ti][tidx[z + b]], b < n,
-  //   HV[x] * HV[y + b] + (h ? HV[x + 1] * HV[y + t + b] : 0).
-  std::vector<int> sc_ptr, sc_rec;
+  // sc_ptr[ti+1]), in supernode order; chunk c has an L position x and a stride t
+  // (two ints at sc_rec[2 c], t = 0: one column), its lane l a tail column (-1:
+  // none) and a U position y (two ints at sc_lane[2 (32 c + l)]), and the lane
+  // subtracts from S[ti][column]
+  //   HV[x] * HV[y] + (t ? HV[x + 1] * HV[y + t] : 0).
+  std::vector<int> sc_ptr, sc_rec, sc_lane;
   int64_t schur_madds = 0, schur_volume = 0;
   int64_t dense_madds = 0;
 
@@ -110,6 +111,24 @@ struct Plan {
   std::vector<int> ut_ptr, ut_row, ut_pos;  // [dim + 1]
   // per head column i, (r, HV pos of l_ri) over rows r > i (head or tail)
   std::vector<int> lt_ptr, lt_row, lt_pos;  // [p + 1]
+
+  // ---- slices ---------------------------------------------------------------
+  // The same solves as lists of rows, a list cut into slices of 32 lanes, one
+  // warp's work: longest rows first, each row over g = 1, 2, .. 32 adjacent lanes
+  // (the fewest that leave a lane at most four entries, in lists L and L + 1 at most
+  // 4 lanes; one g per slice).  Lane
+  // sub of a row takes its entries sub, sub + g, ...; a slice's entries are
+  // transposed (entry k of lane l at off + 32 k, off the lane's first), so that
+  // the lanes of a warp read consecutive columns and values.  sl_rec: four ints
+  // per lane (row or -1, the lane's entries, off, g); list q is slices
+  // [sl_lev[q], sl_lev[q+1]).  With L = n_levels: list q < L holds the forward
+  // rows of level q; L the tail rows against the head; L + 1 the head rows' tail
+  // columns of the backward pass (all rows at once: they depend on the tail
+  // only); L + 2 + q the backward rows of level L - 1 - q against the head
+  // columns.  sl_pos: HV position of every entry's value (-1: padding).
+  std::vector<int> sl_lev, sl_rec, sl_col, sl_pos;
+  // Ybus rows the same way (one list, a row per lane): column and Ybus entry of every entry
+  std::vector<int> yl_rec, yl_col, yl_k;
 
   // ---- Jacobian fill map --------------------------------------------------
   // per Ybus entry k: destinations of its J11 (P-θ), J12 (P-Vm), J21 (Q-θ),

@@ -138,7 +138,7 @@ struct gs2g_session {
   DevBuf d_row_map;  // rows of gs2g_run_subset
   DevBuf d_base_ws;        // base case's factor for GS2G_REFACTOR_BASE_CHORD
   DevBuf d_base_inv;       // its inverse, column c = M0^-1 e_c (outage compensation)
-  DevBuf d_base_fwv, d_base_bwv;  // its head values in forward / backward solve order
+  DevBuf d_base_slv;  // its head values in the order of the solves' slices
   DevBuf d_handoff;        // rows the chord sweep hands to the single-row sweep
   DevBuf d_chord_steps;    // Newton steps the last chord sweep took on the base factor
   int chord = 2;           // policy 2: 0 single-row sweep, 1 chord sweep, 2 chord sweep with Broyden steps
@@ -200,15 +200,9 @@ void upload_plan(gs2g_session* s) {
   D.div_rec = reinterpret_cast<const int2*>(upload_vec(s, P.div_rec));
   D.lev_piv_ptr = upload_vec(s, P.lev_piv_ptr);
   D.lev_piv = upload_vec(s, P.lev_piv);
-  D.tidx = upload_vec(s, P.tidx);
   D.sc_ptr = upload_vec(s, P.sc_ptr);
-  D.sc_rec = reinterpret_cast<const int4*>(upload_vec(s, P.sc_rec));
-  D.fw_ptr = upload_vec(s, P.fw_ptr);
-  D.fw_col = upload_vec(s, P.fw_col);
-  D.fw_pos = upload_vec(s, P.fw_pos);
-  D.bw_ptr = upload_vec(s, P.bw_ptr);
-  D.bw_row = upload_vec(s, P.bw_row);
-  D.bw_pos = upload_vec(s, P.bw_pos);
+  D.sc_rec = reinterpret_cast<const int2*>(upload_vec(s, P.sc_rec));
+  D.sc_lane = reinterpret_cast<const int2*>(upload_vec(s, P.sc_lane));
   D.ut_ptr = upload_vec(s, P.ut_ptr);
   D.ut_row = upload_vec(s, P.ut_row);
   D.ut_pos = upload_vec(s, P.ut_pos);
@@ -216,6 +210,20 @@ void upload_plan(gs2g_session* s) {
   D.lt_row = upload_vec(s, P.lt_row);
   D.lt_pos = upload_vec(s, P.lt_pos);
   D.iperm = upload_vec(s, P.iperm);
+  D.sl_lev = upload_vec(s, P.sl_lev);
+  D.sl_rec = reinterpret_cast<const int4*>(upload_vec(s, P.sl_rec));
+  D.sl_col = upload_vec(s, P.sl_col);
+  D.sl_pos = upload_vec(s, P.sl_pos);
+  D.n_ysl = (int)P.yl_rec.size() / 128;
+  D.yl_rec = reinterpret_cast<const int4*>(upload_vec(s, P.yl_rec));
+  D.yl_col = upload_vec(s, P.yl_col);
+  std::vector<double> yv(2 * P.yl_k.size(), 0.0);
+  for (size_t e = 0; e < P.yl_k.size(); ++e)
+    if (P.yl_k[e] >= 0) {
+      yv[2 * e] = s->ybus[2 * (size_t)P.yl_k[e]];
+      yv[2 * e + 1] = s->ybus[2 * (size_t)P.yl_k[e] + 1];
+    }
+  D.yl_val = reinterpret_cast<const double2*>(upload_vec(s, yv));
 }
 
 // Ybus entry index of (i, j), -1 if not in the pattern.
@@ -620,8 +628,7 @@ gs2g::SweepArgs make_args(gs2g_session* s, const gs2g_run_opts& o, int n_rows, c
     a.base_ws = s->d_base_ws.as<char>();
     a.base_v = s->d_basev.as<double>();
     a.base_inv = s->d_base_inv.as<char>();
-    a.base_fwv = s->d_base_fwv.as<char>();
-    a.base_bwv = s->d_base_bwv.as<char>();
+    a.base_slv = s->d_base_slv.as<char>();
   }
   // defaults: a step on the shared base factor is cheap (several rows share
   // each factor read), so base_chord keeps it longer than adaptive keeps a
@@ -716,6 +723,7 @@ float launch(gs2g_session* s, const gs2g_run_opts& o, int n_rows, const double* 
     c.n_handoff = s->d_queue.as<int>() + 3;
     c.n_chord_steps = s->d_chord_steps.as<unsigned long long>();
     c.broyden = s->chord == 2;
+    c.chord_slots = gs2g::chord_rows_per_cta();
     // every row's outage compensation, set up in parallel ahead of the sweep
     if (a.edit_ptr != nullptr && a.base_v != nullptr) {
       ck((cudaError_t)gs2g::launch_comp_setup(s->dplan, c, o.precision, n_rows, s->d_comp.p, s->stream),
@@ -739,8 +747,7 @@ float launch(gs2g_session* s, const gs2g_run_opts& o, int n_rows, const double* 
     a.base_ws = nullptr;
     a.base_v = nullptr;
     a.base_inv = nullptr;
-    a.base_fwv = nullptr;
-    a.base_bwv = nullptr;
+    a.base_slv = nullptr;
     a.alt_v0 = nullptr;
     a.alt_s = nullptr;
     a.alt_i = nullptr;
@@ -1508,16 +1515,16 @@ void ensure_base_factor(gs2g_session* s, int prec) {
          "read base factor");
     auto packed = [&](const std::vector<int>& pos, DevBuf& dst) {
       std::vector<char> v(std::max<size_t>(pos.size(), 1) * elem);
-      for (size_t q = 0; q < pos.size(); ++q) std::memcpy(v.data() + q * elem, hv.data() + (size_t)pos[q] * elem, elem);
+      for (size_t q = 0; q < pos.size(); ++q)
+        if (pos[q] >= 0) std::memcpy(v.data() + q * elem, hv.data() + (size_t)pos[q] * elem, elem);
       dst.ensure(v.size());
       ck(cudaMemcpy(dst.p, v.data(), v.size(), cudaMemcpyHostToDevice), "upload base factor values");
     };
-    packed(s->plan.fw_pos, s->d_base_fwv);
-    packed(s->plan.bw_pos, s->d_base_bwv);
+    packed(s->plan.sl_pos, s->d_base_slv);
   }
   s->base_factor_prec = prec;
   s->tm.base_setup_ms = ms_since(t_setup);
-  s->tm.base_setup_bytes = (int64_t)(s->d_base_ws.n + s->d_base_inv.n + s->d_base_fwv.n + s->d_base_bwv.n);
+  s->tm.base_setup_bytes = (int64_t)(s->d_base_ws.n + s->d_base_inv.n + s->d_base_slv.n);
 }
 
 // The pinned result buffer for `nr` rows: V [nr x n] complex, then the
@@ -1727,6 +1734,7 @@ int gs2g_run_multi(gs2g_session* const* sessions, int n_sessions, const gs2g_run
       a.handoff_base = begin[i];
       a.n_chord_steps = s0->d_chord_steps.as<unsigned long long>();
       a.broyden = s0->chord == 2;
+      a.chord_slots = gs2g::chord_rows_per_cta();
       // the hand-offs continue from where the chord sweep left them
       gs2g::SweepArgs& b = ge[i].a;
       b.v0 = b.v_out;
