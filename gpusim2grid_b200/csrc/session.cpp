@@ -24,6 +24,7 @@
 #include <stdexcept>
 #include <string>
 #include <thread>
+#include <tuple>
 #include <vector>
 
 #include <pthread.h>
@@ -666,16 +667,35 @@ gs2g::SweepArgs make_args(gs2g_session* s, const gs2g_run_opts& o, int n_rows, c
   return a;
 }
 
-// Dense tail from which a row's factorizations are shared by a cluster.
-constexpr int kClusterTail = 64;
+// Dense tail from which a row's factorizations are shared by a cluster.  Four
+// FP64 steps of one row on one CTA / on clusters of 16, 8 and 4: tail 95 0.75 /
+// 0.76, 0.81, 0.84 ms; 133 1.07 / 0.96, 1.06, 1.13; 204 1.78 / 1.35, 1.53, 1.65;
+// 518 7.9 / 3.4, 4.1, 6.0.
+constexpr int kClusterTail = 160;
 
-// Cluster size for `rows` rows that each get a cluster within `n_ctas`
-// CTAs: 16, else 8, else 0 (one CTA per row).
-int cluster_for(int rows, int n_ctas) {
+// Cluster size for `rows` rows that each get a cluster: the largest of 16, 8, 4
+// and 2 whose clusters the device holds `rows` of at once and that stays
+// within `n_ctas` CTAs, else 0 (one CTA per row).  (A second round of clusters
+// costs more than smaller ones: 16 rows of the 2000-bus grid take 8.0 ms on
+// clusters of 16, which run in two rounds, and 4.4 ms on clusters of 8.)
+int cluster_for(int rows, int n_ctas, int prec) {
   if (rows <= 0) return 0;
-  for (int c = gs2g::handoff_cluster_size(); c >= 8; c /= 2)
-    if ((int64_t)rows * c <= n_ctas) return c;
+  for (int c = gs2g::handoff_cluster_size(); c >= 2; c /= 2)
+    if ((int64_t)rows * c <= n_ctas && rows <= gs2g::max_clusters(prec, c)) return c;
   return 0;
+}
+
+// CTAs of a chord sweep over `rows` rows and the rows each holds at a time:
+// `fit` CTAs are resident at once, `asked` (> 0) bounds the launch.  Rows that
+// would not fill every CTA are spread over more CTAs with fewer rows each: a
+// step of a CTA with one row is shorter than with four, and CTAs without rows
+// are SMs without work.
+std::pair<int, int> chord_shape(int rows, int fit, int asked) {
+  const int per = gs2g::chord_rows_per_cta();
+  const int most = asked > 0 ? std::min(asked, fit) : fit;
+  const int slots = std::max(1, std::min(per, (rows + most - 1) / std::max(most, 1)));
+  const int ctas = asked > 0 ? asked : fit;
+  return {std::max(1, std::min(ctas, (rows + slots - 1) / slots)), slots};
 }
 
 float launch(gs2g_session* s, const gs2g_run_opts& o, int n_rows, const double* v0, int64_t v0_stride,
@@ -690,12 +710,11 @@ float launch(gs2g_session* s, const gs2g_run_opts& o, int n_rows, const double* 
   // (or the rescue) to the single-row sweep that follows on the stream
   const bool chord = s->chord > 0 && use_rows && n_rows > 0 && o.refactor_policy == GS2G_REFACTOR_BASE_CHORD &&
                      a.base_ws != nullptr && a.base_inv != nullptr && !o.fixed_iters;
-  int n_chord = 0;
+  int n_chord = 0, slots = 1;
   int64_t cwsb = 0;
   if (chord) {
-    n_chord = n_ctas_req > 0 ? n_ctas_req : gs2g::chord_ctas(s->dplan, o.precision, s->device);
-    const int per = gs2g::chord_rows_per_cta();
-    n_chord = std::max(1, std::min(n_chord, (n_rows + per - 1) / per));
+    const int fit = gs2g::chord_ctas(s->dplan, o.precision, s->device);
+    std::tie(n_chord, slots) = chord_shape(n_rows, fit, n_ctas_req);
     cwsb = gs2g::chord_workspace_bytes(s->dplan, o.precision);
     s->d_handoff.ensure((size_t)n_rows * sizeof(int));
     if (a.edit_ptr != nullptr && a.base_v != nullptr) s->d_comp.ensure((size_t)n_rows * gs2g::comp_rec_bytes());
@@ -723,7 +742,7 @@ float launch(gs2g_session* s, const gs2g_run_opts& o, int n_rows, const double* 
     c.n_handoff = s->d_queue.as<int>() + 3;
     c.n_chord_steps = s->d_chord_steps.as<unsigned long long>();
     c.broyden = s->chord == 2;
-    c.chord_slots = gs2g::chord_rows_per_cta();
+    c.chord_slots = slots;
     // every row's outage compensation, set up in parallel ahead of the sweep
     if (a.edit_ptr != nullptr && a.base_v != nullptr) {
       ck((cudaError_t)gs2g::launch_comp_setup(s->dplan, c, o.precision, n_rows, s->d_comp.p, s->stream),
@@ -757,7 +776,7 @@ float launch(gs2g_session* s, const gs2g_run_opts& o, int n_rows, const double* 
   // on one SM each after every other row has finished, and small batches
   // (a single solve among them), which would leave the other SMs idle
   const bool few = s->handoff_cluster && s->dplan.nt >= kClusterTail && (chord || n_rows <= n_ctas);
-  const int csize = few ? cluster_for(n_next, chord ? n_ctas : gs2g::sweep_ctas(o.precision, s->device)) : 0;
+  const int csize = few ? cluster_for(n_next, chord ? n_ctas : gs2g::sweep_ctas(o.precision, s->device), o.precision) : 0;
   if (n_next > 0 && csize > 0) {
     ck((cudaError_t)gs2g::launch_sweep_cluster(s->dplan, a, o.precision, csize, n_next * csize, s->stream),
        "hand-off cluster launch");
@@ -1622,7 +1641,7 @@ int gs2g_run_subset(gs2g_session* s, const gs2g_run_opts* o_, int n_sub, const i
   int n_ctas = o.n_ctas > 0 ? o.n_ctas : gs2g::sweep_ctas(o.precision, s->device);
   // few rows with a dense tail worth sharing (an FP64 re-solve of the rows
   // a mixed sweep did not converge): a cluster of CTAs per row
-  const int csize = s->handoff_cluster && s->dplan.nt >= kClusterTail ? cluster_for(n_sub, n_ctas) : 0;
+  const int csize = s->handoff_cluster && s->dplan.nt >= kClusterTail ? cluster_for(n_sub, n_ctas, o.precision) : 0;
   const bool cluster = n_sub > 0 && csize > 0;
   n_ctas = cluster ? n_sub * csize : std::max(1, std::min(n_ctas, std::max(n_sub, 1)));
   const int64_t wsb = gs2g::workspace_bytes(s->dplan, o.precision);
@@ -1710,7 +1729,6 @@ int gs2g_run_multi(gs2g_session* const* sessions, int n_sessions, const gs2g_run
   int64_t cwsb = 0;
   int csmem = 0, n_chord = 0;
   if (chord) {
-    const int per = gs2g::chord_rows_per_cta();
     int big = 0;
     for (int i = 0; i < n_sessions; ++i) {
       cwsb = std::max(cwsb, gs2g::chord_workspace_bytes(sessions[i]->dplan, o.precision));
@@ -1720,8 +1738,9 @@ int gs2g_run_multi(gs2g_session* const* sessions, int n_sessions, const gs2g_run
         big = i;
       }
     }
-    n_chord = o.n_ctas > 0 ? o.n_ctas : gs2g::chord_ctas(sessions[big]->dplan, o.precision, s0->device);
-    n_chord = std::max(1, std::min(n_chord, (total + per - 1) / per));
+    int slots;
+    std::tie(n_chord, slots) =
+        chord_shape(total, gs2g::chord_ctas(sessions[big]->dplan, o.precision, s0->device), o.n_ctas);
     s0->d_handoff.ensure((size_t)total * sizeof(int));
     s0->d_chord_steps.ensure(sizeof(unsigned long long));
     gc = ge;
@@ -1734,7 +1753,7 @@ int gs2g_run_multi(gs2g_session* const* sessions, int n_sessions, const gs2g_run
       a.handoff_base = begin[i];
       a.n_chord_steps = s0->d_chord_steps.as<unsigned long long>();
       a.broyden = s0->chord == 2;
-      a.chord_slots = gs2g::chord_rows_per_cta();
+      a.chord_slots = slots;
       // the hand-offs continue from where the chord sweep left them
       gs2g::SweepArgs& b = ge[i].a;
       b.v0 = b.v_out;
@@ -1771,10 +1790,27 @@ int gs2g_run_multi(gs2g_session* const* sessions, int n_sessions, const gs2g_run
            reinterpret_cast<const gs2g::GridEntry*>(s0->d_multi.as<char>() + ge_bytes), n_sessions, csmem, phase,
            o.precision, n_chord, s0->stream),
        "multi-grid chord sweep launch");
-  if (total > 0)
-    ck((cudaError_t)gs2g::launch_sweep_multi(reinterpret_cast<const gs2g::GridEntry*>(s0->d_multi.p), n_sessions,
-                                             d_begin, total, s0->d_queue.as<int>(), s0->d_ws.as<char>(), wsb, phase,
-                                             o.precision, n_ctas, s0->stream,
+  // the hand-offs get clusters of CTAs as in launch(): how many there are
+  // decides the launch's shape
+  int n_next = total, csize = 0;
+  if (chord) {
+    ck(cudaMemcpyAsync(&n_next, s0->d_queue.as<int>() + 3, sizeof(int), cudaMemcpyDeviceToHost, s0->stream),
+       "hand-off count");
+    ck(cudaStreamSynchronize(s0->stream), "multi-grid chord sweep");
+    bool worth = false;
+    for (int i = 0; i < n_sessions; ++i) worth = worth || sessions[i]->dplan.nt >= kClusterTail;
+    csize = s0->handoff_cluster && worth ? cluster_for(n_next, n_ctas, o.precision) : 0;
+  }
+  const gs2g::GridEntry* d_ge = reinterpret_cast<const gs2g::GridEntry*>(s0->d_multi.p);
+  if (n_next > 0 && csize > 0)
+    ck((cudaError_t)gs2g::launch_sweep_multi_cluster(d_ge, n_sessions, d_begin, n_next, s0->d_queue.as<int>(),
+                                                     s0->d_ws.as<char>(), wsb, phase, o.precision, csize,
+                                                     n_next * csize, s0->stream, s0->d_handoff.as<int>(),
+                                                     kClusterTail),
+       "multi-grid hand-off cluster launch");
+  else if (n_next > 0)
+    ck((cudaError_t)gs2g::launch_sweep_multi(d_ge, n_sessions, d_begin, total, s0->d_queue.as<int>(),
+                                             s0->d_ws.as<char>(), wsb, phase, o.precision, n_ctas, s0->stream,
                                              chord ? s0->d_handoff.as<int>() : nullptr,
                                              chord ? s0->d_queue.as<int>() + 3 : nullptr),
        "multi-grid sweep launch");

@@ -1,0 +1,115 @@
+"""The factorization and the solves at the sizes where their tiles, slices and
+cluster splits change: dense tails around one and several 32- and 64-wide
+panels, remainders, grids without a head, and every cluster size."""
+
+import numpy as np
+import pytest
+
+from conftest import TOL_V_FP64, TOL_V_MIXED
+from gpusim2grid_b200 import AcPfGPU, ContingencyAnalysisGPU, InjectionSweepGPU, ScenarioSweepGPU, compute_many
+from gpusim2grid_b200.synthetic import grid_by_name, injection_scenarios, make_grid, n1_branches, scenario_outages
+from oracle.nr_oracle import nr_solve
+
+pytestmark = pytest.mark.gpu
+
+
+def _grid(n):
+    branches = min(n * (n - 1) // 2, max(n - 1, int(1.58 * n)))
+    return make_grid(n, branches, n // 5, max(1, int(0.75 * n)), seed=n, load_scale=0.1)
+
+
+# tails (default plan): from a handful of unknowns to several panels, whole and ragged
+SIZES = [2, 3, 9, 40, 83, 84, 95, 118, 150, 231, 402, 700]
+
+
+@pytest.mark.parametrize("n", SIZES)
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_solves_match_the_oracle(n, precision):
+    g = _grid(n)
+    p, q = injection_scenarios(g, 5, seed=3)
+    Y, V0, _, _, _, pv, pq = g.as_tuple()
+    sw = InjectionSweepGPU(g.as_tuple(), init_from_n_powerflow=False, precision=precision, nb_iter=10,
+                           scheduling="continuous", start="flat")
+    sw.set_injections(p, q, g.sn_mva)
+    for policy in (0, 1):  # the exact trailing clique, and the cost model's tail
+        sw.session.replan(policy, 40.0, -1)
+        sw.compute()
+        V, _, st, it = sw.results_view()
+        for r in range(5):
+            Vo, so, io, _ = nr_solve(Y, V0, (p[r] + 1j * q[r]) / g.sn_mva, pv, pq, max_iter=10, tol=1e-8)
+            assert st[r] == so == 0
+            if precision == "fp64":
+                assert it[r] == io
+            assert np.abs(V[r] - Vo).max() <= (TOL_V_FP64 if precision == "fp64" else TOL_V_MIXED)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("rows", [1, 18, 19, 37, 38, 74, 75, 148, 149])
+def test_small_batches_on_clusters_equal_one_cta_per_row(rows, precision):
+    """Clusters of 16, 8, 4 and 2 CTAs and none, by the number of rows."""
+    g = _grid(402)
+    p, q = injection_scenarios(g, rows, seed=5)
+    out = []
+    for cluster in (1, 0):
+        sw = InjectionSweepGPU(g.as_tuple(), init_from_n_powerflow=False, precision=precision, nb_iter=10,
+                               scheduling="continuous", start="flat")
+        sw.session.set_handoff(cluster)
+        sw.set_injections(p, q, g.sn_mva)
+        sw.compute()
+        out.append([a.copy() for a in sw.results_view()])
+        assert np.all(out[-1][2] == 0)
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+
+
+def test_single_solve_on_a_cluster_equals_one_cta():
+    g = grid_by_name("case2000_synth", 0)
+    got = []
+    for cluster in (1, 0):
+        ac = AcPfGPU(g.as_tuple(), init_from_n_powerflow=False)
+        ac.session.set_handoff(cluster)
+        t = ac.resolve(g.vinit(), 1.05 * g.sbus())
+        got.append((ac.solve(), t.nb_iter, t.residual))
+    np.testing.assert_array_equal(got[0][0], got[1][0])
+    assert got[0][1:] == got[1][1:]
+
+
+def test_multi_grid_handoffs_on_clusters_equal_one_cta_per_row():
+    grids = [grid_by_name("case118_synth", 0), grid_by_name("case2000_synth", 0)]
+    out = []
+    for cluster in (1, 0):
+        sweeps = []
+        for i, g in enumerate(grids):
+            p, q = injection_scenarios(g, 64, seed=20 + i)
+            f = ScenarioSweepGPU(g.as_tuple(), init_from_n_powerflow=False, precision="mixed", nb_iter=10,
+                                 scheduling="continuous", strategy="base_chord")
+            f.refactor_ratio = 0.05  # nearly every row leaves the chord for its own factor
+            f.set_branch_data(*g.branch_data())
+            f.set_injections(p, q, g.sn_mva)
+            f.set_topology(scenario_outages(g, 64, seed=40 + i))
+            f.session.set_handoff(cluster)
+            sweeps.append(f)
+        compute_many(sweeps)
+        assert sum(int(f.get_row_factorizations().sum()) for f in sweeps) > 0
+        out.append([a.copy() for f in sweeps for a in f.results_view()])
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("n", [84, 402])
+def test_base_chord_rows_match_the_oracle(n):
+    g = _grid(n)
+    rows = [[int(b)] for b in n1_branches(g)[:60]]
+    Y, V0, S, _, _, pv, pq = g.as_tuple()
+    from oracle.nr_oracle import trip_branches
+    ca = ContingencyAnalysisGPU(g.as_tuple(), init_from_n_powerflow=False, precision="mixed", nb_iter=10,
+                                scheduling="continuous", strategy="base_chord")
+    ca.set_branch_data(*g.branch_data())
+    ca.add_contingencies_by_branch_id(rows)
+    ca.compute()
+    V, _, st, _ = ca.results_view()
+    for r, ids in enumerate(rows):
+        Yr = trip_branches(Y, ids, g.branch_from, g.branch_to, g.yff, g.yft, g.ytf, g.ytt)
+        Vo, so, _, _ = nr_solve(Yr, V0, S, pv, pq, max_iter=10, tol=1e-8)
+        assert st[r] == so == 0
+        assert np.abs(V[r] - Vo).max() <= TOL_V_MIXED
