@@ -685,8 +685,10 @@ __host__ __device__ __forceinline__ int64_t align256(int64_t x) { return (x + 25
 
 constexpr int MAX_COMP = 16;  // compensated Jacobian positions per row (base_chord)
 
+// A row's workspace: everything but the dense tail first (up to S), so that a
+// small grid's can be held in shared memory (kSmallWs), then the tail.
 struct WsLayout {
-  int64_t V, I, F, HV, S, y, M, total;
+  int64_t V, I, F, HV, y, M, S, total;
 };
 
 template <typename T>
@@ -697,11 +699,22 @@ __host__ __device__ WsLayout ws_layout(const DevPlan& P) {
   w.I = o; o = align256(o + (int64_t)P.n_bus * 16);
   w.F = o; o = align256(o + (int64_t)P.dim * 8);
   w.HV = o; o = align256(o + (int64_t)P.n_hv * sizeof(T));
-  w.S = o; o = align256(o + (int64_t)P.nt * P.ld * sizeof(T));
   w.y = o; o = align256(o + (int64_t)P.dim * sizeof(T));
   w.M = o; o = align256(o + (int64_t)((P.n_bus + 31) / 32) * 4);  // masked-bus bitmap
+  w.S = o; o = align256(o + (int64_t)P.nt * P.ld * sizeof(T));
   w.total = o;
   return w;
+}
+
+// Grids whose workspace without the dense tail fits in this (up to about 140
+// buses in FP64, 200 in FP32) keep it in shared memory beside the dense LU's
+// scratch, still at 2 CTAs per SM: on a 118-bus grid every phase but the dense
+// LU is a chain of loads, 30 cycles from there instead of a few hundred
+// (one 118-bus solve 0.384 -> 0.352 ms, 186 N-1 rows 0.412 -> 0.382 ms).
+constexpr int kSmallWs = 20 * 1024;
+template <typename T>
+bool small_ws(const DevPlan& P) {
+  return ws_layout<T>(P).S <= kSmallWs;
 }
 
 // y_t <- Sinv y_t with an explicit inverse of the dense tail, column j at
@@ -1248,8 +1261,9 @@ struct ClusterLu {
   int parts;
 };
 
+// wss: the same workspace up to its dense tail, in ws or in shared memory.
 template <typename T>
-__device__ __forceinline__ void solve_row(const DevPlan& P, const SweepArgs& a, const int row_arg, char* ws,
+__device__ __forceinline__ void solve_row(const DevPlan& P, const SweepArgs& a, const int row_arg, char* ws, char* wss,
                                           const RowShared<T>& sh, PhaseProf& prof, const ClusterLu* cl = nullptr) {
   const int tid = threadIdx.x;
   const int row = row_arg & ~NO_RESCUE_BIT;
@@ -1257,12 +1271,12 @@ __device__ __forceinline__ void solve_row(const DevPlan& P, const SweepArgs& a, 
   // selection) is not restarted from it
   bool from_rescue_v = (row_arg & NO_RESCUE_BIT) != 0;
   const WsLayout L = ws_layout<T>(P);
-  double2* V = reinterpret_cast<double2*>(ws + L.V);
-  double2* I = reinterpret_cast<double2*>(ws + L.I);
-  double* F = reinterpret_cast<double*>(ws + L.F);
-  T* HV = reinterpret_cast<T*>(ws + L.HV);
+  double2* V = reinterpret_cast<double2*>(wss + L.V);
+  double2* I = reinterpret_cast<double2*>(wss + L.I);
+  double* F = reinterpret_cast<double*>(wss + L.F);
+  T* HV = reinterpret_cast<T*>(wss + L.HV);
   T* S = reinterpret_cast<T*>(ws + L.S);
-  T* y = reinterpret_cast<T*>(ws + L.y);
+  T* y = reinterpret_cast<T*>(wss + L.y);
   const double2* Y = reinterpret_cast<const double2*>(a.ybus);
   const int n = P.n_bus;
   int& s_ne = *sh.s_ne;
@@ -1304,7 +1318,7 @@ __device__ __forceinline__ void solve_row(const DevPlan& P, const SweepArgs& a, 
     const double2* sb = reinterpret_cast<const double2*>(a.sbus) + (int64_t)row * a.sbus_stride;
     for (int i = tid; i < n; i += BS) V[i] = v0[i];
     // buses outside the row's largest component (handle_disconnected_grid)
-    unsigned* mbits = reinterpret_cast<unsigned*>(ws + L.M);
+    unsigned* mbits = reinterpret_cast<unsigned*>(wss + L.M);
     const bool has_mask = a.mask_ptr != nullptr && a.mask_ptr[row + 1] > a.mask_ptr[row];
     if (has_mask) {
       for (int w = tid; w < (n + 31) / 32; w += BS) mbits[w] = 0u;
@@ -1564,12 +1578,13 @@ __device__ __forceinline__ void solve_row(const DevPlan& P, const SweepArgs& a, 
     __syncthreads();
 }
 
-template <typename T>
 #ifndef GS2G_MIN_CTAS_PER_SM
 #define GS2G_MIN_CTAS_PER_SM 2
 #endif
-__global__ void __launch_bounds__(BS, GS2G_MIN_CTAS_PER_SM) sweep_kernel(const __grid_constant__ DevPlan P,
-                                                                         const __grid_constant__ SweepArgs a) {
+// SMALL: the workspace up to the dense tail in shared memory (small_ws).
+template <typename T, bool SMALL>
+__global__ void __launch_bounds__(BS, GS2G_MIN_CTAS_PER_SM)
+    sweep_kernel(const __grid_constant__ DevPlan P, const __grid_constant__ SweepArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_row;
   __shared__ int s_ne;
@@ -1585,6 +1600,7 @@ __global__ void __launch_bounds__(BS, GS2G_MIN_CTAS_PER_SM) sweep_kernel(const _
   const RowShared<T> sh{&s_ne, s_ek, s_ev, s_red, s_blk, reinterpret_cast<T*>(smem_raw), s_cr, s_cB, s_cLU, s_cpiv,
                         s_cw};
   char* ws = a.workspace + (int64_t)blockIdx.x * a.ws_stride;
+  char* wss = SMALL ? reinterpret_cast<char*>(smem_raw) + dense_smem_elems<T>() * sizeof(T) : ws;
   PhaseProf prof;
   prof.init(a.phase_cycles != nullptr && threadIdx.x == 0);
   const int n_rows = a.n_rows_dev != nullptr ? *a.n_rows_dev : a.n_rows;
@@ -1596,7 +1612,7 @@ __global__ void __launch_bounds__(BS, GS2G_MIN_CTAS_PER_SM) sweep_kernel(const _
       prof.flush(a.phase_cycles);
       return;
     }
-    solve_row<T>(P, a, a.row_map != nullptr ? a.row_map[q] : q, ws, sh, prof);
+    solve_row<T>(P, a, a.row_map != nullptr ? a.row_map[q] : q, ws, wss, sh, prof);
   }
 }
 
@@ -1701,7 +1717,7 @@ __global__ void __launch_bounds__(BS, GS2G_MIN_CTAS_PER_SM)
       const int q = s_row;
       __syncthreads();  // every thread has read s_row before it is overwritten
       if (q >= n_rows) break;
-      solve_row<T>(P, a, a.row_map != nullptr ? a.row_map[q] : q, own, sh, prof);
+      solve_row<T>(P, a, a.row_map != nullptr ? a.row_map[q] : q, own, own, sh, prof);
     }
     prof.flush(a.phase_cycles);
     return;
@@ -1717,7 +1733,7 @@ __global__ void __launch_bounds__(BS, GS2G_MIN_CTAS_PER_SM)
     cluster_barrier();
     if (q >= n_rows) break;
     if (rank == 0) {
-      solve_row<T>(P, a, a.row_map != nullptr ? a.row_map[q] : q, ws, sh, prof, &cl);
+      solve_row<T>(P, a, a.row_map != nullptr ? a.row_map[q] : q, ws, ws, sh, prof, &cl);
       if (threadIdx.x == 0) s_cmd = CLUSTER_CMD_DONE;
       cluster_barrier();
       cluster_barrier();
@@ -1784,7 +1800,7 @@ __global__ void __launch_bounds__(BS, GS2G_MIN_CTAS_PER_SM)
     // a queue position goes through the grid's row order; a hand-off entry
     // is already the grid's row
     const int srow = row_list == nullptr && s_grid.a.row_map != nullptr ? s_grid.a.row_map[lr] : lr;
-    solve_row<T>(s_grid.P, s_grid.a, srow | flag, ws, sh, prof);
+    solve_row<T>(s_grid.P, s_grid.a, srow | flag, ws, ws, sh, prof);
   }
 }
 
@@ -1840,7 +1856,7 @@ __global__ void __launch_bounds__(BS, GS2G_MIN_CTAS_PER_SM)
       cur = g;
     }
     if (rank == 0) {
-      solve_row<T>(s_grid.P, s_grid.a, (row - row_begin[g]) | flag, ws, sh, prof,
+      solve_row<T>(s_grid.P, s_grid.a, (row - row_begin[g]) | flag, ws, ws, sh, prof,
                    s_grid.P.nt >= min_tail ? &cl : nullptr);
       if (threadIdx.x == 0) s_cmd = CLUSTER_CMD_DONE;
       cluster_barrier();
@@ -1874,10 +1890,17 @@ namespace {
 // Dynamic shared memory above 48 KB needs an opt-in per kernel (per device
 // context); cheap and idempotent, so it is set before every query / launch.
 cudaError_t opt_in_smem() {
-  cudaError_t e = cudaFuncSetAttribute(sweep_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaError_t e = cudaFuncSetAttribute(sweep_kernel<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        smem_bytes<float>());
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(sweep_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<double>());
+  e = cudaFuncSetAttribute(sweep_kernel<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           smem_bytes<double>());
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(sweep_kernel<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           smem_bytes<float>() + kSmallWs);
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(sweep_kernel<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           smem_bytes<double>() + kSmallWs);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(sweep_kernel_multi<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            smem_bytes<float>());
@@ -1913,9 +1936,9 @@ int sweep_ctas(int prec, int device) {
   opt_in_smem();
   int per_sm = 0;
   if (prec == 1)
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sweep_kernel<float>, BS, smem_bytes<float>());
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sweep_kernel<float, false>, BS, smem_bytes<float>());
   else
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sweep_kernel<double>, BS, smem_bytes<double>());
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sweep_kernel<double, false>, BS, smem_bytes<double>());
   if (per_sm < 1) per_sm = 1;
   return n_sm * per_sm;
 }
@@ -2101,10 +2124,16 @@ int launch_sweep(const DevPlan& P, const SweepArgs& a, int prec, int n_ctas, voi
   if (n_ctas <= 0) return (int)cudaErrorInvalidValue;
   const cudaError_t e = opt_in_smem();
   if (e != cudaSuccess) return (int)e;
-  if (prec == 1)
-    sweep_kernel<float><<<n_ctas, BS, smem_bytes<float>(), st>>>(P, a);
+  // (a factor that outlives the launch stays in the workspace)
+  const bool small = !a.factor_only && (prec == 1 ? small_ws<float>(P) : small_ws<double>(P));
+  if (prec == 1 && small)
+    sweep_kernel<float, true><<<n_ctas, BS, smem_bytes<float>() + kSmallWs, st>>>(P, a);
+  else if (prec == 1)
+    sweep_kernel<float, false><<<n_ctas, BS, smem_bytes<float>(), st>>>(P, a);
+  else if (small)
+    sweep_kernel<double, true><<<n_ctas, BS, smem_bytes<double>() + kSmallWs, st>>>(P, a);
   else
-    sweep_kernel<double><<<n_ctas, BS, smem_bytes<double>(), st>>>(P, a);
+    sweep_kernel<double, false><<<n_ctas, BS, smem_bytes<double>(), st>>>(P, a);
   return (int)cudaGetLastError();
 }
 

@@ -18,8 +18,9 @@ def _grid(n):
     return make_grid(n, branches, n // 5, max(1, int(0.75 * n)), seed=n, load_scale=0.1)
 
 
-# tails (default plan): from a handful of unknowns to several panels, whole and ragged
-SIZES = [2, 3, 9, 40, 83, 84, 95, 118, 150, 231, 402, 700]
+# tails (default plan): from a handful of unknowns to several panels, whole and ragged;
+# 130 to 210: where a row's workspace stops fitting in shared memory (FP64, then FP32)
+SIZES = [2, 3, 9, 40, 83, 84, 95, 118, 130, 140, 150, 190, 210, 231, 402, 700]
 
 
 @pytest.mark.parametrize("n", SIZES)
