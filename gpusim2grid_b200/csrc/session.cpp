@@ -152,6 +152,12 @@ struct gs2g_session {
   int last_rows_run = 0;
   // pinned double buffer for large result copies (see d2h_staged)
   mutable void* h_stage = nullptr;
+  // pinned buffer for small ones: a run's counters in the first kSmallHost
+  // bytes, results that fit in the second (one reader at a time), each set
+  // copied ahead of one synchronisation
+  char* h_small = nullptr;
+  mutable std::mutex small_mutex;
+  bool counts_valid = false;  // tm.total_iters / n_failed are the last run's
   // pinned host copy of the last run's results (gs2g_get_results_host)
   void* h_res = nullptr;
   size_t h_res_bytes = 0;
@@ -667,6 +673,12 @@ gs2g::SweepArgs make_args(gs2g_session* s, const gs2g_run_opts& o, int n_rows, c
   return a;
 }
 
+// Half of a session's small pinned buffer.  A run's half: its counters in 64
+// bytes, then the statuses and step counts of up to kSmallRows rows.  Seven
+// blocking copies of a few bytes took 60-80 us of a 118-bus solve's call.
+constexpr size_t kSmallHost = 64 * 1024;
+constexpr int kSmallRows = 4096;
+
 // Dense tail from which a row's factorizations are shared by a cluster.  Four
 // FP64 steps of one row on one CTA / on clusters of 16, 8 and 4: tail 95 0.75 /
 // 0.76, 0.81, 0.84 ms; 133 1.07 / 0.96, 1.06, 1.13; 204 1.78 / 1.35, 1.53, 1.65;
@@ -785,15 +797,34 @@ float launch(gs2g_session* s, const gs2g_run_opts& o, int n_rows, const double* 
        "sweep launch");
   }
   ck(cudaEventRecord(s->ev1, s->stream), "event");
+  // the counters (and a small batch's statuses and steps) travel behind the
+  // sweep and are there when it has been waited for
+  int* h_queue = reinterpret_cast<int*>(s->h_small);
+  auto* h_steps = reinterpret_cast<unsigned long long*>(s->h_small + 16);
+  ck(cudaMemcpyAsync(h_queue, s->d_queue.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, s->stream), "counters");
+  ck(cudaMemcpyAsync(h_steps, s->d_chord_steps.p, sizeof(*h_steps), cudaMemcpyDeviceToHost, s->stream), "step count");
+  const bool count = use_rows && n_rows > 0 && n_rows <= kSmallRows;
+  int* h_status = reinterpret_cast<int*>(s->h_small + 64);
+  int* h_iters = h_status + kSmallRows;
+  if (count) {
+    ck(cudaMemcpyAsync(h_status, out.status, n_rows * sizeof(int), cudaMemcpyDeviceToHost, s->stream), "statuses");
+    ck(cudaMemcpyAsync(h_iters, out.iters, n_rows * sizeof(int), cudaMemcpyDeviceToHost, s->stream), "steps");
+  }
   ck(cudaStreamSynchronize(s->stream), "sweep");
   float ms = 0;
   ck(cudaEventElapsedTime(&ms, s->ev0, s->ev1), "event time");
   for (int q = 0; q < GS2G_N_PHASES; ++q) s->tm.phase_cycles[q] = s->tm.phase_share[q] = 0;
-  ck(cudaMemcpy(&s->tm.n_rescued, s->d_queue.as<int>() + 1, sizeof(int), cudaMemcpyDeviceToHost), "rescue count");
-  ck(cudaMemcpy(&s->tm.n_base_start, s->d_queue.as<int>() + 2, sizeof(int), cudaMemcpyDeviceToHost), "start count");
-  unsigned long long cs = 0;
-  ck(cudaMemcpy(&cs, s->d_chord_steps.p, sizeof(cs), cudaMemcpyDeviceToHost), "step count");
-  s->tm.chord_steps = (int64_t)cs;
+  s->tm.n_rescued = h_queue[1];
+  s->tm.n_base_start = h_queue[2];
+  s->tm.chord_steps = (int64_t)*h_steps;
+  if (count) {
+    s->tm.total_iters = s->tm.n_failed = 0;
+    for (int r = 0; r < n_rows; ++r) {
+      s->tm.total_iters += h_iters[r];
+      s->tm.n_failed += h_status[r] == GS2G_ROW_MAX_ITER || h_status[r] == GS2G_ROW_DIVERGED;
+    }
+    s->counts_valid = true;
+  }
   if (o.profile_phases) {
     unsigned long long c[gs2g::N_PHASES];
     ck(cudaMemcpy(c, s->d_phase.p, sizeof(c), cudaMemcpyDeviceToHost), "read phases");
@@ -919,6 +950,7 @@ int gs2g_session_create(int device, int n_bus, const int* ybus_indptr, const int
   ck(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking), "stream");
   ck(cudaEventCreate(&s->ev0), "event");
   ck(cudaEventCreate(&s->ev1), "event");
+  ck(cudaMallocHost(reinterpret_cast<void**>(&s->h_small), 2 * kSmallHost), "pinned buffer");
   upload_plan(s.get());
   s->d_ybus.ensure(s->ybus.size() * sizeof(double));
   ck(cudaMemcpy(s->d_ybus.p, s->ybus.data(), s->ybus.size() * sizeof(double), cudaMemcpyHostToDevice), "upload Ybus");
@@ -1006,6 +1038,7 @@ int gs2g_session_destroy(gs2g_session* s) {
     for (cudaEvent_t e : s->ev_stage)
       if (e) cudaEventDestroy(e);
     if (s->h_stage) cudaFreeHost(s->h_stage);
+    if (s->h_small) cudaFreeHost(s->h_small);
     if (s->h_res) cudaFreeHost(s->h_res);
     if (s->stream) cudaStreamDestroy(s->stream);
     delete s;
@@ -1562,6 +1595,7 @@ void ensure_host_results(gs2g_session* s, size_t nr) {
 }
 
 RunPrep prepare_rows(gs2g_session* s, const gs2g_run_opts& o) {
+  s->counts_valid = false;
   if (o.refactor_policy == GS2G_REFACTOR_BASE_CHORD) ensure_base_factor(s, o.precision);
   const int nr = s->n_rows;
   const int n = s->n_bus;
@@ -1613,7 +1647,7 @@ int gs2g_run(gs2g_session* s, const gs2g_run_opts* o_) {
   s->last_rows_run = nr;
   s->mirror_valid = rp.ob.v_mirror != nullptr;
   s->tm.total_ms = ms_since(t0);
-  s->tm.total_iters = -1;
+  if (!s->counts_valid) s->tm.total_iters = -1;
   GS2G_CATCH
 }
 
@@ -1937,6 +1971,31 @@ int gs2g_get_results(const gs2g_session* s, double* v_out, double* residuals, in
   if (!s) throw std::invalid_argument("NULL session");
   DeviceGuard g(s->device);
   const size_t nr = s->last_rows_run, n = s->n_bus;
+  if (nr * (n * 2 * sizeof(double) + sizeof(double) + 2 * sizeof(int)) <= kSmallHost && nr) {
+    // small: all copies (on the default stream, behind whatever it holds), one wait
+    struct Part {
+      void* dst;
+      const void* src;
+      size_t bytes;
+    } parts[] = {{v_out, s->d_v_out.p, nr * n * 2 * sizeof(double)},
+                 {residuals, s->d_res.p, nr * sizeof(double)},
+                 {status, s->d_status.p, nr * sizeof(int)},
+                 {iters, s->d_iters.p, nr * sizeof(int)}};
+    const std::lock_guard<std::mutex> lock(s->small_mutex);
+    char* const h = s->h_small + kSmallHost;
+    size_t off = 0;
+    for (const Part& q : parts) {
+      if (q.dst) ck(cudaMemcpyAsync(h + off, q.src, q.bytes, cudaMemcpyDeviceToHost, nullptr), "read results");
+      off += q.bytes;
+    }
+    ck(cudaStreamSynchronize(nullptr), "read results");
+    off = 0;
+    for (const Part& q : parts) {
+      if (q.dst) std::memcpy(q.dst, h + off, q.bytes);
+      off += q.bytes;
+    }
+    return GS2G_OK;
+  }
   if (v_out && nr) d2h_staged(s, v_out, s->d_v_out.p, nr * n * 2 * sizeof(double));
   if (residuals && nr) ck(cudaMemcpy(residuals, s->d_res.p, nr * sizeof(double), cudaMemcpyDeviceToHost), "read res");
   if (status && nr) ck(cudaMemcpy(status, s->d_status.p, nr * sizeof(int), cudaMemcpyDeviceToHost), "read status");
@@ -2014,6 +2073,7 @@ int gs2g_get_timings(const gs2g_session* s, gs2g_timings* out) {
   GS2G_TRY
   if (!s || !out) throw std::invalid_argument("NULL argument");
   *out = s->tm;
+  if (s->counts_valid) return GS2G_OK;
   out->n_failed = 0;
   if (s->last_rows_run > 0) {
     DeviceGuard g(s->device);
