@@ -1,26 +1,29 @@
-// Dense FP32 LU (no pivoting) of one matrix by one CTA of 256 threads, for
-// the tail of the mixed-precision batched Newton–Raphson factorization.
-// Device code only.
+// Dense FP32 LU (no pivoting) of one matrix by one CTA of 256 threads (or by
+// the CTAs of a cluster), for the tail of the mixed-precision batched
+// Newton–Raphson factorization.  Device code only.
 //
-// Right-looking, 64-wide panels.  Per panel k0 (width kb; kb < 64 only for
-// the last panel, which has nothing below or to the right of it):
-//   1. the kb x kb diagonal block is copied to shared memory (identity
-//      padded to 64 x 64), factored by two warps holding one row per
-//      thread in registers, and written back;
-//   2. L21 = A21 U11^-1: one thread per row of A21, the row in registers,
-//      forward substitution against U11 rows read as broadcast float4;
-//   3. U12 = L11^-1 A12: one thread per column of A12, the column in
-//      registers, substitution against the rows of L11^T (unit diagonal),
-//      which is transposed into the idle tile staging area first;
-//   4. A22 -= L21 U12 on 128 x 128 output tiles: the tile's A (128 x 64) and
-//      B (64 x 128) operands are staged by cp.async in one piece, each
-//      thread accumulates an 8 x 8 block (rows tr + 16 i, columns
-//      4 tc + 64 h + e: within a warp 4 consecutive rows and 8 consecutive
-//      float4 columns, so shared-memory reads are conflict-free), and the
-//      next tile's operands are in flight while a tile's results are
-//      written back.
+// The Crout order and stages of dense_lu_f64.cuh on 32-wide panels, with the
+// update's products as FP32 FMAs (tcgen05 and mma.sync take FP32 operands only
+// as TF32, below the FP32 held here): per panel the column block and the row
+// block take all earlier panels' products at once, on tiles up to 256 high
+// (column block) or wide (row block), fed by a cp.async ring of 32-deep slabs;
+// then the diagonal block is factored by the whole CTA and the rows and columns
+// are solved against it, a row or column per lane.
+// What bounds it: few matrices, the chain of panels (about 14 us each beside
+// the update); one matrix per CTA on every SM, the update.  Against a
+// right-looking form with 64-wide panels, whose trailing update writes and
+// reads the whole matrix once per panel (us per factorization):
+//   n     one CTA       296 CTAs        cluster of 8   cluster of 16
+//   42      27 -> 20        28 -> 24        27 -> 23        29 -> 23
+//   133    130 -> 71       149 -> 91       142 -> 67       142 -> 75
+//   518   1042 -> 839     1811 -> 1338     513 -> 348      475 -> 328
+//   1148  6229 -> 5497   10638 -> 9205    1511 -> 1401    1225 -> 1065
+// (296 CTAs: 32 TFLOP/s at n = 1148.)  The same order with the products on the
+// FP64 tensor pipe (operands widened) took 1668 and 11559 us for 296 CTAs at
+// n = 518 and 1148, 308 and 1080 us on clusters of 16.  Largest error against
+// an FP64 factorization at n = 518: 3.7e-4 -> 2.8e-4.
 // A is row-major in global memory with leading dimension ld, a multiple of
-// 8 (rows 16-byte aligned); panels start at multiples of 64.
+// 4 (rows 16-byte aligned); panels start at multiples of 32.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -31,33 +34,51 @@ namespace gs2g {
 namespace dense32 {
 
 constexpr int BS = 256;
-constexpr int KP = 64;          // panel width
+constexpr int KP = 32;          // panel width
 constexpr int SD = KP + 4;      // diagonal block stride (16-byte rows)
-constexpr int TM = 128, TN = 128;
-constexpr int SA = KP + 4;      // A tile [TM][SA]
-constexpr int SB = TN + 4;      // B tile [KP][SB]
-#ifndef GS2G_DENSE32_EPI_ROWS
-#define GS2G_DENSE32_EPI_ROWS 2  // rows per epilogue batch (1, 2, 4 or 8)
-#endif
+constexpr int KS = 32;          // slab depth of the update's operand ring
+// operand strides: A's 4 mod 32 words, so that the 4 rows a warp reads at once
+// lie in different banks (its 8 column groups of B are consecutive)
+constexpr int SAK = KS + 4;
+template <int TN>
+__host__ __device__ constexpr int sbn() {
+  return TN + 8;
+}
+template <int TM, int TN>
+__host__ __device__ constexpr int stage_elems() {
+  return TM * SAK + KS * sbn<TN>();
+}
+
+// ring depth: three slabs of the 128-wide and smaller tiles, two of the 256-wide
+template <int TM, int TN>
+__host__ __device__ constexpr int n_stage() {
+  return TM * TN > 128 * 32 ? 2 : 3;
+}
+template <int TM, int TN>
+__host__ __device__ constexpr int ring_elems() {
+  return n_stage<TM, TN>() * stage_elems<TM, TN>();
+}
+constexpr int max_of(int a, int b) { return a > b ? a : b; }
 
 struct Smem {
   static constexpr int d_elems = KP * SD;
   static constexpr int r_elems = KP;  // reciprocal pivots
-  static constexpr int a_elems = TM * SA;
-  static constexpr int b_elems = KP * SB;
-  static constexpr int elems = d_elems + r_elems + a_elems + b_elems;
+  // outside the update the ring holds L11^T and a 32-row block per warp
+  static constexpr int ring = max_of(max_of(max_of(ring_elems<128, 32>(), ring_elems<32, 128>()),
+                                            max_of(ring_elems<256, 32>(), ring_elems<32, 256>())),
+                                     9 * d_elems);
+  static constexpr int elems = d_elems + r_elems + ring;
   static constexpr int bytes = elems * 4;
 };
-
 __device__ __forceinline__ float clamp_piv(float piv, double floor_) {
   const float f = (float)floor_;
   if (fabsf(piv) < f) return piv < 0.f ? -f : f;
   return piv;
 }
 
-// Shared-memory loads issued in program order (asm volatile): the TRSM
-// loops below hold 64 values per thread in registers, and letting the
-// compiler hoist their ~500 broadcast loads ahead of the arithmetic would
+// Shared-memory loads issued in program order (asm volatile): the
+// substitutions below hold 32 values per thread in registers, and letting
+// the compiler hoist their broadcast loads ahead of the arithmetic would
 // spill them.
 __device__ __forceinline__ float4 lds4(const float* p) {
   float4 v;
@@ -72,237 +93,291 @@ __device__ __forceinline__ float lds1(const float* p) {
   return v;
 }
 
-__device__ __forceinline__ void cp_async16(float* smem, const float* gmem, int src_bytes) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(src_bytes));
-}
+// This thread's share of a tile's operand slabs: PA 16-byte chunks of A (rows
+// i0 + ra + i * RA) and PB of B (k rows kb + i * RB, columns j0 + n..), the
+// same places in every slab, so the addresses only advance.  Rows past M and
+// columns past N are zero-filled.
+template <int TM, int TN>
+struct Stager {
+  static constexpr int PA = TM * KS / 4 / BS, RA = TM / PA, PB = TN * KS / 4 / BS, RB = KS / PB;
+  static_assert(PA * RA == TM && PB * RB == KS && RA * (KS / 4) == BS && RB * (TN / 4) == BS, "whole chunks");
+  const float* a;
+  const float* b;
+  int64_t lda, ldb, step_b;
+  unsigned sa, sb;  // shared-memory byte offsets within a stage
+  int arows, bbytes;
+  __device__ __forceinline__ Stager(const float* A, const float* B, int ld, int M, int N, int i0, int j0) {
+    const int tid = threadIdx.x;
+    const int ra = tid / (KS / 4), ka = (tid % (KS / 4)) * 4;
+    const int kb = tid / (TN / 4), n = (tid % (TN / 4)) * 4;
+    arows = M - i0 - ra;  // chunk i is in range for i * RA < arows
+    bbytes = (N - j0 - n) * 4;
+    bbytes = bbytes < 0 ? 0 : (bbytes > 16 ? 16 : bbytes);
+    a = A + (int64_t)(i0 + ra) * ld + ka;
+    b = B + (int64_t)kb * ld + j0 + n;
+    lda = (int64_t)RA * ld;
+    ldb = (int64_t)RB * ld;
+    step_b = (int64_t)KS * ld;
+    sa = (unsigned)(ra * SAK + ka) * 4;
+    sb = (unsigned)(TM * SAK + kb * sbn<TN>() + n) * 4;
+  }
+  // the next slab into the stage at shared-memory byte address st
+  __device__ __forceinline__ void next(unsigned st) {
+#pragma unroll
+    for (int i = 0; i < PA; ++i) {
+      const int bytes = i * RA < arows ? 16 : 0;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(st + sa + i * RA * SAK * 4),
+                   "l"(bytes ? a + i * lda : a), "r"(bytes));
+    }
+#pragma unroll
+    for (int i = 0; i < PB; ++i)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(st + sb + i * RB * sbn<TN>() * 4),
+                   "l"(b + i * ldb), "r"(bbytes));
+    a += KS;
+    b += step_b;
+  }
+};
 
-// Stage the A (rows i0.., 64 columns) and B (64 rows, columns j0..) tiles of
-// the trailing update, zero-filled outside [M) rows / [N) columns.
-__device__ __forceinline__ void stage_tile(float* sA, float* sB, const float* A21, const float* A12, int ld, int M,
-                                           int N, int i0, int j0) {
-  const int tid = threadIdx.x;
+// C[i0.., j0..] -= A[i0.., 0..K) B[0..K, j0..) for one TM x TN tile of an
+// M x N block (A, B, C parts of one matrix, leading dimension ld; K a
+// positive multiple of KS).  8 warps as WM x WN; a lane has R rows (4 apart)
+// of 4 columns, so that a k step of 4 takes R + 4 16-byte loads, each of few
+// distinct addresses, for 16 R products.  An element's products are summed
+// slab by slab, each slab from zero (as many roundings at the size of the
+// result as K has slabs, not as many as K), in the same order whatever the
+// tile shape, so every tiling gives the same bits.  Ends without a barrier;
+// the ring may be refilled only after one.
+template <int TM, int TN, int WM, int WN>
+__device__ __noinline__ void update_tile(float* C, const float* A, const float* B, int ld, int M, int N, int K,
+                                         int i0, int j0, float* ring) {
+  constexpr int R = TM / (4 * WM);
+  constexpr int SE = stage_elems<TM, TN>(), NSTAGE = n_stage<TM, TN>();
+  static_assert(WM * WN * 32 == BS && R > 0 && TN == 32 * WN, "8 warps tile TM x TN");
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int wr = (warp / WN) * 4 * R + (lane >> 3), wc = (warp % WN) * 32 + (lane & 7) * 4;
+  const int nslab = K / KS;
+  const unsigned sring = (unsigned)__cvta_generic_to_shared(ring);
+  Stager<TM, TN> stager(A, B, ld, M, N, i0, j0);
 #pragma unroll
-  for (int q = 0; q < (TM * KP / 4) / BS; ++q) {  // 8 chunks per thread
-    const int c = tid + q * BS;
-    const int r = c >> 4, k = (c & 15) * 4;
-    const bool in = i0 + r < M;
-    cp_async16(sA + r * SA + k, in ? A21 + (int64_t)(i0 + r) * ld + k : A21, in ? 16 : 0);
+  for (int s = 0; s < NSTAGE - 1; ++s) {
+    if (s < nslab) stager.next(sring + s * SE * 4);
+    asm volatile("cp.async.commit_group;\n" ::);
   }
+  int cur = 0, fill = NSTAGE - 1;  // ring positions of slab t and of slab t + NSTAGE - 1
+  float acc[R][4];
+  const int c = j0 + wc;
 #pragma unroll
-  for (int q = 0; q < (KP * TN / 4) / BS; ++q) {  // 8 chunks per thread
-    const int c = tid + q * BS;
-    const int k = c >> 5, n = (c & 31) * 4;
-    int bytes = (N - j0 - n) * 4;
-    bytes = bytes < 0 ? 0 : (bytes > 16 ? 16 : bytes);
-    cp_async16(sB + k * SB + n, bytes ? A12 + (int64_t)k * ld + j0 + n : A12, bytes);
+  for (int i = 0; i < R; ++i) {
+    const int r = i0 + wr + 4 * i;
+    const float* src = C + (int64_t)r * ld + c;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (r < M && c + 3 < N) {
+      v = *reinterpret_cast<const float4*>(src);
+    } else if (r < M) {
+      if (c < N) v.x = src[0];
+      if (c + 1 < N) v.y = src[1];
+      if (c + 2 < N) v.z = src[2];
+    }
+    acc[i][0] = v.x;
+    acc[i][1] = v.y;
+    acc[i][2] = v.z;
+    acc[i][3] = v.w;
   }
-  asm volatile("cp.async.commit_group;\n" ::);
-}
-
-// A22[M x N] -= A21[M x 64] A12[64 x N].  With parts > 1 the CTA takes the
-// output tiles part, part + parts, ... (the CTAs of a cluster split them).
-__device__ __noinline__ void trailing_update(float* A22, const float* A21, const float* A12, int ld, int M, int N, float* sA,
-                                float* sB, int part = 0, int parts = 1) {
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int tr = (warp >> 1) * 4 + (lane >> 3);  // 0..15
-  const int tc = (warp & 1) * 8 + (lane & 7);    // 0..15
-  const int n_ti = (M + TM - 1) / TM, n_tj = (N + TN - 1) / TN;
-  const int n_tiles = n_ti * n_tj;
-  if (part >= n_tiles) {
-    __syncthreads();
-    return;
-  }
-  stage_tile(sA, sB, A21, A12, ld, M, N, (part / n_tj) * TM, (part % n_tj) * TN);
-  for (int t = part; t < n_tiles; t += parts) {
-    const int i0 = (t / n_tj) * TM, j0 = (t % n_tj) * TN;
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    __syncthreads();
-    // bring this tile's output rows toward L2 while the tile computes
+  for (int t = 0; t < nslab; ++t) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(NSTAGE - 2) : "memory");
+    __syncthreads();  // slab t has landed; every warp is done with slab t - 1
+    if (t + NSTAGE - 1 < nslab) stager.next(sring + fill * SE * 4);
+    asm volatile("cp.async.commit_group;\n" ::);
+    const float* sA = ring + cur * SE + wr * SAK;
+    const float* sB = ring + cur * SE + TM * SAK + wc;
+    cur = cur + 1 < NSTAGE ? cur + 1 : 0;
+    fill = fill + 1 < NSTAGE ? fill + 1 : 0;
+    float p[R][4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int r = i0 + tr + 16 * i;
-      if (r < M && j0 + 4 * tc < N)
-        asm volatile("prefetch.global.L2 [%0];\n" ::"l"(A22 + (int64_t)r * ld + j0 + 4 * tc));
-      if (r < M && j0 + 64 + 4 * tc < N)
-        asm volatile("prefetch.global.L2 [%0];\n" ::"l"(A22 + (int64_t)r * ld + j0 + 64 + 4 * tc));
-    }
-    float acc[8][8];
+    for (int i = 0; i < R; ++i) p[i][0] = p[i][1] = p[i][2] = p[i][3] = 0.f;
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int k = 0; k < KS; k += 4) {
+      float4 b[4];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-#pragma unroll 4
-    for (int k = 0; k < KP; ++k) {
-      float a[8];
+      for (int h = 0; h < 4; ++h) b[h] = *reinterpret_cast<const float4*>(sB + (k + h) * sbn<TN>());
 #pragma unroll
-      for (int i = 0; i < 8; ++i) a[i] = sA[(tr + 16 * i) * SA + k];
-      const float4 b0 = *reinterpret_cast<const float4*>(sB + k * SB + 4 * tc);
-      const float4 b1 = *reinterpret_cast<const float4*>(sB + k * SB + 64 + 4 * tc);
-      const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+      for (int i = 0; i < R; ++i) {
+        const float4 av = *reinterpret_cast<const float4*>(sA + 4 * i * SAK + k);
+        const float a[4] = {av.x, av.y, av.z, av.w};
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();  // every thread is done reading this tile's operands
-    if (t + parts < n_tiles) {
-      const int t1 = t + parts;
-      stage_tile(sA, sB, A21, A12, ld, M, N, (t1 / n_tj) * TM, (t1 % n_tj) * TN);
-    }
-    // epilogue in batches of EB rows: all loads of a batch are issued before
-    // its stores (the compiler cannot reorder them across the stores)
-    constexpr int EB = GS2G_DENSE32_EPI_ROWS;
-#pragma unroll
-    for (int ib = 0; ib < 8; ib += EB) {
-      float4 cv[EB][2];
-#pragma unroll
-      for (int i = 0; i < EB; ++i) {
-        const int r = i0 + tr + 16 * (ib + i);
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int c = j0 + 64 * h + 4 * tc;
-          cv[i][h] = (r < M && c + 3 < N) ? *reinterpret_cast<const float4*>(A22 + (int64_t)r * ld + c)
-                                          : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int h = 0; h < 4; ++h) {
+          p[i][0] = fmaf(a[h], b[h].x, p[i][0]);
+          p[i][1] = fmaf(a[h], b[h].y, p[i][1]);
+          p[i][2] = fmaf(a[h], b[h].z, p[i][2]);
+          p[i][3] = fmaf(a[h], b[h].w, p[i][3]);
         }
       }
+    }
 #pragma unroll
-      for (int i = 0; i < EB; ++i) {
-        const int r = i0 + tr + 16 * (ib + i);
-        if (r >= M) continue;
-        float* crow = A22 + (int64_t)r * ld;
+    for (int i = 0; i < R; ++i)
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int c = j0 + 64 * h + 4 * tc;
-          const float* a = acc[ib + i] + 4 * h;
-          if (c + 3 < N) {
-            *reinterpret_cast<float4*>(crow + c) =
-                make_float4(cv[i][h].x - a[0], cv[i][h].y - a[1], cv[i][h].z - a[2], cv[i][h].w - a[3]);
-          } else {
+      for (int e = 0; e < 4; ++e) acc[i][e] -= p[i][e];
+  }
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-              if (c + e < N) crow[c + e] -= a[e];
-          }
-        }
+  for (int i = 0; i < R; ++i) {
+    const int r = i0 + wr + 4 * i;
+    if (r >= M) continue;
+    float* dst = C + (int64_t)r * ld + c;
+    if (c + 3 < N) {
+      *reinterpret_cast<float4*>(dst) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    } else {
+      if (c < N) dst[0] = acc[i][0];
+      if (c + 1 < N) dst[1] = acc[i][1];
+      if (c + 2 < N) dst[2] = acc[i][2];
+    }
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+}
+
+// Factor the identity-padded 32 x 32 block D (stride SD) in place, its first kb
+// steps; rp gets the reciprocal pivots (see dense_lu_f64.cuh).
+__device__ __noinline__ void factor_diag(float* D, float* rp, double pfloor, int kb) {
+  __shared__ __align__(16) float prow[2][KP];
+  const int r = threadIdx.x >> 3, q = threadIdx.x & 7, lane = threadIdx.x & 31;
+  float x[4];
+  {
+    const float4 v = *reinterpret_cast<const float4*>(D + r * SD + 4 * q);
+    x[0] = v.x;
+    x[1] = v.y;
+    x[2] = v.z;
+    x[3] = v.w;
+  }
+#pragma unroll
+  for (int j = 0; j < KP; ++j) {
+    if (j >= kb) break;  // the padding needs no step
+    if (r == j) {
+      if (q == j >> 2) {
+        x[j & 3] = clamp_piv(x[j & 3], pfloor);
+        rp[j] = 1.f / x[j & 3];
+      }
+      *reinterpret_cast<float4*>(&prow[j & 1][4 * q]) = make_float4(x[0], x[1], x[2], x[3]);
+    }
+    __syncthreads();
+    const float xj = __shfl_sync(0xffffffffu, x[j & 3], (lane & 24) | (j >> 2));
+    if (r > j && q >= j >> 2) {
+      const float l = xj * rp[j];
+      const float4 uv = *reinterpret_cast<const float4*>(&prow[j & 1][4 * q]);
+      const float u[4] = {uv.x, uv.y, uv.z, uv.w};
+      if (q > j >> 2) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) x[c] = fmaf(-l, u[c], x[c]);
+      } else {
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if (c > (j & 3)) x[c] = fmaf(-l, u[c], x[c]);
+        x[j & 3] = l;
       }
     }
   }
+  *reinterpret_cast<float4*>(D + r * SD + 4 * q) = make_float4(x[0], x[1], x[2], x[3]);
   __syncthreads();
 }
 
-// Factor the identity-padded 64 x 64 block D (stride SD) in place; rp gets
-// the reciprocal pivots.  Warps 0 and 1 hold one row each in registers
-// (thread r: row r).  Step j: thread j clamps its pivot and publishes its
-// row (final: L part, pivot, U part) to D; a 64-thread named barrier; rows
-// below j take l = x_j / u_jj and x_c -= l u_jc (c > j), reading row j as
-// broadcast float4.  One lightweight barrier per step; warps 2..7 skip.
-__device__ __noinline__ void factor_diag(float* D, float* rp, double pfloor) {
-  const int r = threadIdx.x;
-  if (r < KP) {
-    float x[KP];
-#pragma unroll
-    for (int q = 0; q < KP / 4; ++q) {
-      const float4 v = lds4(D + r * SD + 4 * q);
-      x[4 * q] = v.x;
-      x[4 * q + 1] = v.y;
-      x[4 * q + 2] = v.z;
-      x[4 * q + 3] = v.w;
-    }
-    asm volatile("bar.sync 1, 64;\n" ::: "memory");  // all rows read before any is rewritten
-#pragma unroll
-    for (int j = 0; j < KP; ++j) {
-      if (r == j) {
-        x[j] = clamp_piv(x[j], pfloor);
-        rp[j] = 1.f / x[j];
-#pragma unroll
-        for (int q = 0; q < KP / 4; ++q)
-          *reinterpret_cast<float4*>(D + j * SD + 4 * q) = make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
-      }
-      asm volatile("bar.sync 1, 64;\n" ::: "memory");
-      if (r > j) {
-        const float* uj = D + j * SD;
-        const float l = x[j] * (1.f / lds1(uj + j));
-        x[j] = l;
-#pragma unroll
-        for (int c = j + 1; c < KP && (c & 3); ++c) x[c] = fmaf(-l, lds1(uj + c), x[c]);
-#pragma unroll
-        for (int c4 = ((j + 1) + 3) & ~3; c4 < KP; c4 += 4) {
-          const float4 u = lds4(uj + c4);
-          x[c4] = fmaf(-l, u.x, x[c4]);
-          x[c4 + 1] = fmaf(-l, u.y, x[c4 + 1]);
-          x[c4 + 2] = fmaf(-l, u.z, x[c4 + 2]);
-          x[c4 + 3] = fmaf(-l, u.w, x[c4 + 3]);
-        }
-      }
-    }
-  }
-  __syncthreads();
-}
-
-// x <- x M^-1 for the 64 values x of one thread, M upper triangular given by
+// x <- x M^-1 for the 32 values x of one thread, M upper triangular given by
 // its rows (stride SD) in shared memory: after x_p is final, x_q -= x_p M_pq
 // for q > p.  SCALE: x_p is multiplied by rp[p] (1 / M_pp) first; else M has
 // a unit diagonal.
 template <bool SCALE>
-__device__ __forceinline__ void subst64(float (&x)[KP], const float* M, const float* rp) {
+__device__ __forceinline__ void subst32(float (&x)[KP], const float* M, const float* rp) {
 #pragma unroll
   for (int p = 0; p < KP; ++p) {
     if (SCALE) x[p] *= lds1(rp + p);
     const float xp = x[p];
     const float* mp = M + p * SD;
 #pragma unroll
-    for (int q = p + 1; q < KP && (q & 3); ++q) x[q] = fmaf(-xp, lds1(mp + q), x[q]);
-#pragma unroll
-    for (int q4 = ((p + 1) + 3) & ~3; q4 < KP; q4 += 4) {
+    for (int q4 = (p + 1) & ~3; q4 < KP; q4 += 4) {
       const float4 u = lds4(mp + q4);
-      x[q4] = fmaf(-xp, u.x, x[q4]);
-      x[q4 + 1] = fmaf(-xp, u.y, x[q4 + 1]);
-      x[q4 + 2] = fmaf(-xp, u.z, x[q4 + 2]);
-      x[q4 + 3] = fmaf(-xp, u.w, x[q4 + 3]);
+      if (q4 > p) x[q4] = fmaf(-xp, u.x, x[q4]);
+      if (q4 + 1 > p) x[q4 + 1] = fmaf(-xp, u.y, x[q4 + 1]);
+      if (q4 + 2 > p) x[q4 + 2] = fmaf(-xp, u.z, x[q4 + 2]);
+      if (q4 + 3 > p) x[q4 + 3] = fmaf(-xp, u.w, x[q4 + 3]);
     }
   }
 }
 
-// L21 = A21 U11^-1 (x U11 = a per row), one thread per row (with parts > 1:
-// rows part * BS + tid, then every parts * BS).
-__device__ __noinline__ void trsm_rows(float* A21, int ld, int M, const float* D, const float* rp, int part = 0,
-                                       int parts = 1) {
-  for (int r = part * BS + threadIdx.x; r < M; r += BS * parts) {
-    float4* row = reinterpret_cast<float4*>(A21 + (int64_t)r * ld);
+// L21 = A21 U11^-1 (x U11 = a per row) for 32 rows (n of them valid) by one
+// warp, a row per lane in registers.  The rows pass through the warp's block
+// of shared memory (stride SD: conflict-free) so that global memory is read
+// and written four whole rows at a time.
+__device__ __forceinline__ void trsm_rows32(float* A21, int ld, int n, const float* D, const float* rp, float* buf) {
+  const int lane = threadIdx.x & 31, r4 = lane >> 3, c4 = (lane & 7) * 4;
+#pragma unroll
+  for (int h = 0; h < KP; h += 4)
+    if (h + r4 < n)
+      *reinterpret_cast<float4*>(buf + (h + r4) * SD + c4) =
+          *reinterpret_cast<const float4*>(A21 + (int64_t)(h + r4) * ld + c4);
+  __syncwarp();
+  if (lane < n) {
     float x[KP];
 #pragma unroll
-    for (int q = 0; q < KP / 4; ++q) {
-      const float4 v = row[q];
-      x[4 * q] = v.x;
-      x[4 * q + 1] = v.y;
-      x[4 * q + 2] = v.z;
-      x[4 * q + 3] = v.w;
+    for (int q = 0; q < KP; q += 4) {
+      const float4 v = lds4(buf + lane * SD + q);
+      x[q] = v.x;
+      x[q + 1] = v.y;
+      x[q + 2] = v.z;
+      x[q + 3] = v.w;
     }
-    subst64<true>(x, D, rp);
+    subst32<true>(x, D, rp);
 #pragma unroll
-    for (int q = 0; q < KP / 4; ++q) row[q] = make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
+    for (int q = 0; q < KP; q += 4)
+      *reinterpret_cast<float4*>(buf + lane * SD + q) = make_float4(x[q], x[q + 1], x[q + 2], x[q + 3]);
   }
+  __syncwarp();
+#pragma unroll
+  for (int h = 0; h < KP; h += 4)
+    if (h + r4 < n)
+      *reinterpret_cast<float4*>(A21 + (int64_t)(h + r4) * ld + c4) =
+          *reinterpret_cast<const float4*>(buf + (h + r4) * SD + c4);
+  __syncwarp();
 }
 
 // U12 = L11^-1 A12 (per column: y^T L11^T = a^T, L11^T upper with unit
-// diagonal, given by its rows LT = rows of L11^T), one thread per column.
-__device__ __noinline__ void trsm_cols(float* A12, int ld, int N, const float* LT, int part = 0, int parts = 1) {
-  for (int c = part * BS + threadIdx.x; c < N; c += BS * parts) {
-    float y[KP];
-    const float* src = A12 + c;
+// diagonal, given by its rows LT), one column of A12 in registers.
+__device__ __forceinline__ void trsm_col(float* colp, int ld, const float* LT) {
+  float y[KP];
 #pragma unroll
-    for (int r = 0; r < KP; ++r, src += ld) {
-      y[r] = *src;
-      if ((r & 15) == 15) asm volatile("" ::: "memory");  // at most 16 loads in flight
+  for (int r = 0; r < KP; ++r) y[r] = colp[(int64_t)r * ld];
+  subst32<false>(y, LT, nullptr);
+#pragma unroll
+  for (int r = 0; r < KP; ++r) colp[(int64_t)r * ld] = y[r];
+}
+
+// Both substitutions of a panel with m rows below and m columns to the right
+// of its diagonal block, in groups of 32 rows or 32 columns taken by the
+// warps of the `parts` CTAs (this one: part).  LT: L11^T, followed by a block
+// per warp.
+__device__ __noinline__ void trsm_panel(float* A21, float* A12, int ld, int m, const float* D, const float* rp,
+                                        float* LT, int part, int parts) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int ng = (m + 31) / 32;
+  for (int t = part * (BS / 32) + warp; t < 2 * ng; t += parts * (BS / 32)) {
+    if (t < ng) {
+      trsm_rows32(A21 + (int64_t)t * 32 * ld, ld, min(32, m - 32 * t), D, rp, LT + Smem::d_elems * (1 + warp));
+    } else {
+      const int c = (t - ng) * 32 + lane;
+      if (c < m) trsm_col(A12 + c, ld, LT);
     }
-    subst64<false>(y, LT, nullptr);
-    // the stores walk the column again from an opaque copy of ld, so the 64
-    // load addresses are not kept alive across the substitution
-    int ld2;
-    asm volatile("mov.b32 %0, %1;\n" : "=r"(ld2) : "r"(ld));
-    float* dst = A12 + c;
-#pragma unroll
-    for (int r = 0; r < KP; ++r, dst += ld2) *dst = y[r];
+  }
+}
+
+// Load the kb x kb diagonal block at Akk into D (identity padded).
+__device__ __forceinline__ void load_diag(float* D, const float* Akk, int ld, int kb) {
+  for (int idx = threadIdx.x; idx < KP * KP; idx += BS) {
+    const int r = idx / KP, c = idx % KP;
+    D[r * SD + c] = (r < kb && c < kb) ? Akk[(int64_t)r * ld + c] : (r == c ? 1.f : 0.f);
+  }
+}
+
+// L11^T into LT (the idle tile staging area) for the column solves.
+__device__ __forceinline__ void transpose_l11(float* LT, const float* D) {
+  for (int idx = threadIdx.x; idx < KP * KP; idx += BS) {
+    const int r = idx / KP, c = idx % KP;
+    LT[c * SD + r] = r > c ? D[r * SD + c] : 0.f;
   }
 }
 
@@ -310,40 +385,46 @@ __device__ __noinline__ void trsm_cols(float* A12, int ld, int N, const float* L
 __device__ void lu(float* A, int n, int ld, float* smem, double pfloor) {
   float* D = smem;
   float* rp = D + Smem::d_elems;
-  float* sA = rp + Smem::r_elems;
-  float* sB = sA + Smem::a_elems;
+  float* ring = rp + Smem::r_elems;
   const int tid = threadIdx.x;
   for (int k0 = 0; k0 < n; k0 += KP) {
     const int kb = min(KP, n - k0);
+    const int m = n - k0 - kb;  // > 0 only with kb == 32
     float* Akk = A + (int64_t)k0 * ld + k0;
-    for (int idx = tid; idx < KP * KP; idx += BS) {
-      const int r = idx >> 6, c = idx & 63;
-      D[r * SD + c] = (r < kb && c < kb) ? Akk[(int64_t)r * ld + c] : (r == c ? 1.f : 0.f);
+    const float* Arow = A + (int64_t)k0 * ld;  // rows k0.. of the columns before the panel
+    if (k0 > 0) {
+      int i0 = 0, j0 = 0;
+      for (; n - k0 - i0 > 128; i0 += 256) {
+        update_tile<256, 32, 8, 1>(Akk, Arow, A + k0, ld, n - k0, kb, k0, i0, 0, ring);
+        __syncthreads();
+      }
+      if (i0 < n - k0) {
+        update_tile<128, 32, 8, 1>(Akk, Arow, A + k0, ld, n - k0, kb, k0, i0, 0, ring);
+        __syncthreads();
+      }
+      for (; m - j0 > 128; j0 += 256) {
+        update_tile<32, 256, 1, 8>(Akk + kb, Arow, A + k0 + kb, ld, kb, m, k0, 0, j0, ring);
+        __syncthreads();
+      }
+      if (j0 < m) {
+        update_tile<32, 128, 2, 4>(Akk + kb, Arow, A + k0 + kb, ld, kb, m, k0, 0, j0, ring);
+        __syncthreads();
+      }
     }
+    load_diag(D, Akk, ld, kb);
     __syncthreads();
-    factor_diag(D, rp, pfloor);
+    factor_diag(D, rp, pfloor, kb);
     for (int idx = tid; idx < kb * kb; idx += BS) {
       const int r = idx / kb, c = idx % kb;
       Akk[(int64_t)r * ld + c] = D[r * SD + c];
     }
-    const int m = n - k0 - kb;  // > 0 only with kb == 64
     if (m > 0) {
-      float* A21 = A + (int64_t)(k0 + kb) * ld + k0;
-      float* A12 = A + (int64_t)k0 * ld + k0 + kb;
-      float* A22 = A + (int64_t)(k0 + kb) * ld + k0 + kb;
-      // L11^T into the (idle) tile staging area for the column solves
-      float* LT = sA;
-      for (int idx = tid; idx < KP * KP; idx += BS) {
-        const int r = idx >> 6, c = idx & 63;
-        LT[c * SD + r] = r > c ? D[r * SD + c] : 0.f;
-      }
+      float* LT = ring;
+      transpose_l11(LT, D);
       __syncthreads();
-      trsm_rows(A21, ld, m, D, rp);
-      trsm_cols(A12, ld, m, LT);
-      __syncthreads();  // L21 and U12 complete (global writes of other threads)
-      trailing_update(A22, A21, A12, ld, m, m, sA, sB);
+      trsm_panel(A + (int64_t)(k0 + kb) * ld + k0, Akk + kb, ld, m, D, rp, LT, 0, 1);
     }
-    __syncthreads();
+    __syncthreads();  // L21, U12 and the diagonal block complete
   }
 }
 
@@ -356,43 +437,77 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
 
+// Height of the tiles a cluster splits a panel's update into: the column block
+// has mc rows, the row block mr columns, and a k step of a 32-, 64- or 128-high
+// tile takes about 5, 6 and 9 units (its loads from shared memory, then its
+// products, bound it), so the fewest units over the rounds.
+__device__ __forceinline__ int tile_height(int mc, int mr, int parts) {
+  int best = 32, cost = 1 << 30;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const int h = 32 << i, tiles = (mc + h - 1) / h + (mr + h - 1) / h;
+    const int c = (tiles + parts - 1) / parts * (i == 0 ? 5 : i == 1 ? 6 : 9);
+    if (c < cost) {
+      cost = c;
+      best = h;
+    }
+  }
+  return best;
+}
+
+// This CTA's tiles (H x 32 of the column block, 32 x H of the row block) of
+// panel k0's update.  WM x WN: the warps of a row-block tile.
+template <int H, int WM, int WN>
+__device__ __forceinline__ void cluster_update(float* A, int n, int ld, int k0, int kb, float* ring, int part,
+                                               int parts) {
+  const int m = n - k0 - kb;
+  float* Akk = A + (int64_t)k0 * ld + k0;
+  const float* Arow = A + (int64_t)k0 * ld;
+  const int nc = (n - k0 + H - 1) / H, nr = (m + H - 1) / H;
+  for (int t = part; t < nc + nr; t += parts) {
+    if (t < nc)
+      update_tile<H, 32, 8, 1>(Akk, Arow, A + k0, ld, n - k0, kb, k0, H * t, 0, ring);
+    else
+      update_tile<32, H, WM, WN>(Akk + kb, Arow, A + k0 + kb, ld, kb, m, k0, 0, H * (t - nc), ring);
+    __syncthreads();
+  }
+}
+
 // The same LU as lu(), by the `parts` CTAs of a cluster together (this CTA
-// has rank `part`); A in global memory, every CTA with its own scratch.
-// Each CTA factors the diagonal block itself (the 64 x 64 block is cheap and
-// every CTA needs it in its own shared memory), the row and column
-// substitutions and the trailing-update tiles are split by rank, and three
-// cluster barriers per panel order the stages.  Every element goes through
-// the same operations in the same order as in lu(), so the factor is
+// has rank `part`); A in global memory, every CTA with its own scratch.  The
+// update's blocks are split into tiles by rank, each CTA factors the diagonal block itself (every
+// CTA needs it in its own shared memory), the substitutions are split by rank,
+// and three cluster barriers per panel order the stages.  Every element goes
+// through the same operations in the same order as in lu(), so the factor is
 // bit-identical.  Every CTA of the cluster must call it with the same n.
 __device__ void lu_cluster(float* A, int n, int ld, float* smem, double pfloor, int part, int parts) {
   float* D = smem;
   float* rp = D + Smem::d_elems;
-  float* sA = rp + Smem::r_elems;
-  float* sB = sA + Smem::a_elems;
+  float* ring = rp + Smem::r_elems;
   const int tid = threadIdx.x;
   for (int k0 = 0; k0 < n; k0 += KP) {
     const int kb = min(KP, n - k0);
+    const int m = n - k0 - kb;
     float* Akk = A + (int64_t)k0 * ld + k0;
-    for (int idx = tid; idx < KP * KP; idx += BS) {
-      const int r = idx >> 6, c = idx & 63;
-      D[r * SD + c] = (r < kb && c < kb) ? Akk[(int64_t)r * ld + c] : (r == c ? 1.f : 0.f);
+    if (k0 > 0) {
+      const int h = tile_height(n - k0, m, parts);
+      if (h == 128)
+        cluster_update<128, 2, 4>(A, n, ld, k0, kb, ring, part, parts);
+      else if (h == 64)
+        cluster_update<64, 4, 2>(A, n, ld, k0, kb, ring, part, parts);
+      else
+        cluster_update<32, 8, 1>(A, n, ld, k0, kb, ring, part, parts);
+      cluster_sync_all();  // the panel's blocks complete
     }
+    load_diag(D, Akk, ld, kb);
     __syncthreads();
-    factor_diag(D, rp, pfloor);
+    factor_diag(D, rp, pfloor, kb);
     cluster_sync_all();  // every CTA holds the block: rank 0 may write it back below
-    const int m = n - k0 - kb;  // > 0 only with kb == 64
-    float* A21 = A + (int64_t)(k0 + kb) * ld + k0;
-    float* A12 = A + (int64_t)k0 * ld + k0 + kb;
-    float* A22 = A + (int64_t)(k0 + kb) * ld + k0 + kb;
     if (m > 0) {
-      float* LT = sA;
-      for (int idx = tid; idx < KP * KP; idx += BS) {
-        const int r = idx >> 6, c = idx & 63;
-        LT[c * SD + r] = r > c ? D[r * SD + c] : 0.f;
-      }
+      float* LT = ring;
+      transpose_l11(LT, D);
       __syncthreads();
-      trsm_rows(A21, ld, m, D, rp, part, parts);
-      trsm_cols(A12, ld, m, LT, part, parts);
+      trsm_panel(A + (int64_t)(k0 + kb) * ld + k0, Akk + kb, ld, m, D, rp, LT, part, parts);
     }
     if (part == 0)
       for (int idx = tid; idx < kb * kb; idx += BS) {
@@ -400,8 +515,6 @@ __device__ void lu_cluster(float* A, int n, int ld, float* smem, double pfloor, 
         Akk[(int64_t)r * ld + c] = D[r * SD + c];
       }
     cluster_sync_all();  // L21, U12 and the diagonal block complete
-    if (m > 0) trailing_update(A22, A21, A12, ld, m, m, sA, sB, part, parts);
-    cluster_sync_all();  // A22 complete
   }
 }
 
