@@ -14,11 +14,11 @@
 // right-looking form with 64-wide panels, whose trailing update writes and
 // reads the whole matrix once per panel (us per factorization):
 //   n     one CTA       296 CTAs        cluster of 8   cluster of 16
-//   42      27 -> 20        28 -> 24        27 -> 23        29 -> 23
-//   133    130 -> 71       149 -> 91       142 -> 67       142 -> 75
-//   518   1042 -> 839     1811 -> 1338     513 -> 348      475 -> 328
-//   1148  6229 -> 5497   10638 -> 9205    1511 -> 1401    1225 -> 1065
-// (296 CTAs: 32 TFLOP/s at n = 1148.)  The same order with the products on the
+//   42      27 -> 20        28 -> 23        27 -> 23        29 -> 23
+//   133    130 -> 75       149 -> 81       142 -> 67       142 -> 73
+//   518   1042 -> 815     1811 -> 1283     513 -> 350      475 -> 328
+//   1148  6229 -> 5413   10638 -> 9018    1511 -> 1424    1225 -> 1080
+// (296 CTAs: 33 TFLOP/s at n = 1148.)  The same order with the products on the
 // FP64 tensor pipe (operands widened) took 1668 and 11559 us for 296 CTAs at
 // n = 518 and 1148, 308 and 1080 us on clusters of 16.  Largest error against
 // an FP64 factorization at n = 518: 3.7e-4 -> 2.8e-4.
@@ -183,6 +183,9 @@ __device__ __noinline__ void update_tile(float* C, const float* A, const float* 
     acc[i][2] = v.z;
     acc[i][3] = v.w;
   }
+  // a warp of a last tile whose part lies past M or N only stages (296 CTAs at
+  // n = 200: 173 -> 159 us); in the 256 tiles the test cost 20 %
+  const bool idle = i0 + wr - (lane >> 3) >= M || j0 + (warp % WN) * 32 >= N;
   for (int t = 0; t < nslab; ++t) {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(NSTAGE - 2) : "memory");
     __syncthreads();  // slab t has landed; every warp is done with slab t - 1
@@ -192,6 +195,7 @@ __device__ __noinline__ void update_tile(float* C, const float* A, const float* 
     const float* sB = ring + cur * SE + TM * SAK + wc;
     cur = cur + 1 < NSTAGE ? cur + 1 : 0;
     fill = fill + 1 < NSTAGE ? fill + 1 : 0;
+    if (TM * TN == 128 * 32 && idle) continue;
     float p[R][4];
 #pragma unroll
     for (int i = 0; i < R; ++i) p[i][0] = p[i][1] = p[i][2] = p[i][3] = 0.f;

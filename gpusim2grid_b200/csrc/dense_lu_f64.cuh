@@ -171,6 +171,11 @@ __device__ __noinline__ void update_tile(double* C, const double* A, const doubl
       acc[i][j][1] = v.y;
     }
   }
+  // a warp whose part lies past M or N only stages: the pipe is the others'
+  // (296 CTAs with this and the 64 tiles of the remainders: n = 200 224 -> 190 us,
+  // 518 1806 -> 1643, 1148 12768 -> 12358); in a cluster's 32 x 32 tiles the test
+  // cost 5-15 %
+  const bool idle = i0 + wr >= M || j0 + wc >= N;
   for (int t = 0; t < nslab; ++t) {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(NSTAGE - 2) : "memory");
     __syncthreads();  // slab t has landed; every warp is done with slab t - 1
@@ -180,6 +185,7 @@ __device__ __noinline__ void update_tile(double* C, const double* A, const doubl
     const double* sB = ring + cur * SE + TM * SAK + q * sbn<TN>() + wc + g;
     cur = cur + 1 < NSTAGE ? cur + 1 : 0;
     fill = fill + 1 < NSTAGE ? fill + 1 : 0;
+    if (TM * TN > 32 * 32 && idle) continue;
 #pragma unroll
     for (int k = 0; k < KS; k += 4) {
       double a[MT], b[NT];
@@ -389,11 +395,17 @@ __device__ void lu(double* A, int n, int ld, double* smem, double pfloor) {
     const double* Arow = A + (int64_t)k0 * ld;  // rows k0.. of the columns before the panel
     if (k0 > 0) {
       for (int i0 = 0; i0 < n - k0; i0 += 128) {
-        update_tile<128, 32, 8, 1>(Akk, Arow, A + k0, ld, n - k0, kb, k0, i0, 0, ring);
+        if (n - k0 - i0 > 64)
+          update_tile<128, 32, 8, 1>(Akk, Arow, A + k0, ld, n - k0, kb, k0, i0, 0, ring);
+        else
+          update_tile<64, 32, 8, 1>(Akk, Arow, A + k0, ld, n - k0, kb, k0, i0, 0, ring);
         __syncthreads();
       }
       for (int j0 = 0; j0 < m; j0 += 128) {
-        update_tile<32, 128, 1, 8>(Akk + kb, Arow, A + k0 + kb, ld, kb, m, k0, 0, j0, ring);
+        if (m - j0 > 64)
+          update_tile<32, 128, 1, 8>(Akk + kb, Arow, A + k0 + kb, ld, kb, m, k0, 0, j0, ring);
+        else
+          update_tile<32, 64, 2, 4>(Akk + kb, Arow, A + k0 + kb, ld, kb, m, k0, 0, j0, ring);
         __syncthreads();
       }
     }
