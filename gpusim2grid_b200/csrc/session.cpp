@@ -77,6 +77,54 @@ double ms_since(std::chrono::steady_clock::time_point t0) {
 
 }  // namespace
 
+namespace {
+
+// Size of half of a session's small pinned block.  A run's half: its counters in
+// 64 bytes, then the statuses and step counts of up to kSmallRows rows.  Seven
+// blocking copies of a few bytes took 60-80 us of a 118-bus solve's call.
+constexpr size_t kSmallHost = 64 * 1024;
+constexpr int kSmallRows = 4096;
+
+// The blocks: one slab per process, pinned once (cudaHostAlloc takes 2.5 ms,
+// more than the rest of a small session's creation), a block per session from
+// its second run on until it is destroyed.  Sessions beyond kBlocks, or a slab
+// that cannot be had, do with blocking copies.  The slab lives as long as the
+// process: freeing it while the driver shuts down is not allowed.
+class SmallBlocks {
+ public:
+  static SmallBlocks& get() {
+    static SmallBlocks* b = new SmallBlocks;
+    return *b;
+  }
+  char* take() {
+    const std::lock_guard<std::mutex> lock(m_);
+    if (!tried_) {
+      tried_ = true;
+      void* p = nullptr;
+      if (cudaHostAlloc(&p, kBlocks * 2 * kSmallHost, cudaHostAllocPortable) == cudaSuccess)
+        for (int i = 0; i < kBlocks; ++i) free_.push_back(static_cast<char*>(p) + i * 2 * kSmallHost);
+      else
+        cudaGetLastError();  // not an error of the run
+    }
+    if (free_.empty()) return nullptr;
+    char* const b = free_.back();
+    free_.pop_back();
+    return b;
+  }
+  void put(char* b) {
+    const std::lock_guard<std::mutex> lock(m_);
+    free_.push_back(b);
+  }
+
+ private:
+  static constexpr int kBlocks = 32;
+  std::mutex m_;
+  std::vector<char*> free_;
+  bool tried_ = false;
+};
+
+}  // namespace
+
 struct gs2g_session {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -85,7 +133,7 @@ struct gs2g_session {
   gs2g::Plan plan;
   gs2g::DevPlan dplan{};
   std::vector<int> y_ip, y_ix, pv, pq;  // canonical pattern and bus sets, for re-planning
-  std::vector<std::unique_ptr<DevBuf>> plan_bufs;
+  DevBuf d_plan;  // the plan's arrays
   int n_bus = 0;
   std::vector<double> ybus;  // canonical values, interleaved complex
   std::vector<double> vinit, sbus, base_v;
@@ -152,11 +200,12 @@ struct gs2g_session {
   int last_rows_run = 0;
   // pinned double buffer for large result copies (see d2h_staged)
   mutable void* h_stage = nullptr;
-  // pinned buffer for small ones: a run's counters in the first kSmallHost
-  // bytes, results that fit in the second (one reader at a time), each set
-  // copied ahead of one synchronisation
+  // pinned block for small ones (SmallBlocks; NULL in a session's first run): a
+  // run's counters in the first half, results that fit in the second (one
+  // reader at a time), each set copied ahead of one synchronisation
   char* h_small = nullptr;
   mutable std::mutex small_mutex;
+  int n_launched = 0;
   bool counts_valid = false;  // tm.total_iters / n_failed are the last run's
   // pinned host copy of the last run's results (gs2g_get_results_host)
   void* h_res = nullptr;
@@ -170,19 +219,45 @@ struct gs2g_session {
 
 namespace {
 
-template <typename T>
-const T* upload_vec(gs2g_session* s, const std::vector<T>& v) {
-  auto b = std::make_unique<DevBuf>();
-  b->ensure(std::max<size_t>(v.size() * sizeof(T), 16));
-  if (!v.empty()) ck(cudaMemcpy(b->p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice), "upload plan");
-  const T* p = b->as<T>();
-  s->plan_bufs.push_back(std::move(b));
-  return p;
-}
+// The plan's arrays in one device block: a small plan is packed on the host and
+// copied at once (an allocation and a copy for each of its 35 arrays cost a
+// small grid's session 0.9 ms), a large one array by array.
+class PlanUpload {
+ public:
+  template <typename D, typename T>
+  void put(const D*& dst, const std::vector<T>& v) {
+    items_.push_back({&dst, v.data(), v.size() * sizeof(T), total_});
+    total_ += (std::max<size_t>(v.size() * sizeof(T), 16) + 255) / 256 * 256;
+  }
+  void run(DevBuf& block) {
+    constexpr size_t kPack = 4 << 20;
+    block.ensure(total_);
+    char* const base = block.as<char>();
+    std::vector<char> host(total_ <= kPack ? total_ : 0);
+    for (const Item& it : items_) {
+      const void* at = base + it.off;
+      std::memcpy(it.dst, &at, sizeof(at));
+      if (it.bytes == 0) continue;
+      if (!host.empty()) std::memcpy(host.data() + it.off, it.src, it.bytes);
+      else ck(cudaMemcpy(base + it.off, it.src, it.bytes, cudaMemcpyHostToDevice), "upload plan");
+    }
+    if (!host.empty()) ck(cudaMemcpy(base, host.data(), total_, cudaMemcpyHostToDevice), "upload plan");
+  }
+
+ private:
+  struct Item {
+    void* dst;  // where the array's device address goes
+    const void* src;
+    size_t bytes, off;
+  };
+  std::vector<Item> items_;
+  size_t total_ = 0;
+};
 
 void upload_plan(gs2g_session* s) {
   const gs2g::Plan& P = s->plan;
   gs2g::DevPlan& D = s->dplan;
+  PlanUpload up;
   D.n_bus = P.n_bus;
   D.nnz_y = P.nnz_y;
   D.dim = P.dim;
@@ -191,46 +266,47 @@ void upload_plan(gs2g_session* s) {
   D.ld = P.ld;
   D.n_hv = P.n_hv;
   D.n_levels = P.n_levels;
-  D.y_indptr = upload_vec(s, P.y_indptr);
-  D.y_indices = upload_vec(s, P.y_indices);
-  D.y_row = upload_vec(s, P.y_row);
-  D.jmap = upload_vec(s, P.jmap);
+  up.put(D.y_indptr, P.y_indptr);
+  up.put(D.y_indices, P.y_indices);
+  up.put(D.y_row, P.y_row);
+  up.put(D.jmap, P.jmap);
   D.n_y_tail = (int)P.y_tail.size();
-  D.y_tail = upload_vec(s, P.y_tail);
-  D.fP = upload_vec(s, P.fP);
-  D.fQ = upload_vec(s, P.fQ);
-  D.lev_ptr = upload_vec(s, P.lev_ptr);
-  D.lev_big = upload_vec(s, P.lev_big);
-  D.task_rec = reinterpret_cast<const int4*>(upload_vec(s, P.task_rec));
-  D.pairs = reinterpret_cast<const int2*>(upload_vec(s, P.pairs));
-  D.div_ptr = upload_vec(s, P.div_ptr);
-  D.div_rec = reinterpret_cast<const int2*>(upload_vec(s, P.div_rec));
-  D.lev_piv_ptr = upload_vec(s, P.lev_piv_ptr);
-  D.lev_piv = upload_vec(s, P.lev_piv);
-  D.sc_ptr = upload_vec(s, P.sc_ptr);
-  D.sc_rec = reinterpret_cast<const int2*>(upload_vec(s, P.sc_rec));
-  D.sc_lane = reinterpret_cast<const int2*>(upload_vec(s, P.sc_lane));
-  D.ut_ptr = upload_vec(s, P.ut_ptr);
-  D.ut_row = upload_vec(s, P.ut_row);
-  D.ut_pos = upload_vec(s, P.ut_pos);
-  D.lt_ptr = upload_vec(s, P.lt_ptr);
-  D.lt_row = upload_vec(s, P.lt_row);
-  D.lt_pos = upload_vec(s, P.lt_pos);
-  D.iperm = upload_vec(s, P.iperm);
-  D.sl_lev = upload_vec(s, P.sl_lev);
-  D.sl_rec = reinterpret_cast<const int4*>(upload_vec(s, P.sl_rec));
-  D.sl_col = upload_vec(s, P.sl_col);
-  D.sl_pos = upload_vec(s, P.sl_pos);
+  up.put(D.y_tail, P.y_tail);
+  up.put(D.fP, P.fP);
+  up.put(D.fQ, P.fQ);
+  up.put(D.lev_ptr, P.lev_ptr);
+  up.put(D.lev_big, P.lev_big);
+  up.put(D.task_rec, P.task_rec);
+  up.put(D.pairs, P.pairs);
+  up.put(D.div_ptr, P.div_ptr);
+  up.put(D.div_rec, P.div_rec);
+  up.put(D.lev_piv_ptr, P.lev_piv_ptr);
+  up.put(D.lev_piv, P.lev_piv);
+  up.put(D.sc_ptr, P.sc_ptr);
+  up.put(D.sc_rec, P.sc_rec);
+  up.put(D.sc_lane, P.sc_lane);
+  up.put(D.ut_ptr, P.ut_ptr);
+  up.put(D.ut_row, P.ut_row);
+  up.put(D.ut_pos, P.ut_pos);
+  up.put(D.lt_ptr, P.lt_ptr);
+  up.put(D.lt_row, P.lt_row);
+  up.put(D.lt_pos, P.lt_pos);
+  up.put(D.iperm, P.iperm);
+  up.put(D.sl_lev, P.sl_lev);
+  up.put(D.sl_rec, P.sl_rec);
+  up.put(D.sl_col, P.sl_col);
+  up.put(D.sl_pos, P.sl_pos);
   D.n_ysl = (int)P.yl_rec.size() / 128;
-  D.yl_rec = reinterpret_cast<const int4*>(upload_vec(s, P.yl_rec));
-  D.yl_col = upload_vec(s, P.yl_col);
+  up.put(D.yl_rec, P.yl_rec);
+  up.put(D.yl_col, P.yl_col);
   std::vector<double> yv(2 * P.yl_k.size(), 0.0);
   for (size_t e = 0; e < P.yl_k.size(); ++e)
     if (P.yl_k[e] >= 0) {
       yv[2 * e] = s->ybus[2 * (size_t)P.yl_k[e]];
       yv[2 * e + 1] = s->ybus[2 * (size_t)P.yl_k[e] + 1];
     }
-  D.yl_val = reinterpret_cast<const double2*>(upload_vec(s, yv));
+  up.put(D.yl_val, yv);
+  up.run(s->d_plan);
 }
 
 // Ybus entry index of (i, j), -1 if not in the pattern.
@@ -673,12 +749,6 @@ gs2g::SweepArgs make_args(gs2g_session* s, const gs2g_run_opts& o, int n_rows, c
   return a;
 }
 
-// Half of a session's small pinned buffer.  A run's half: its counters in 64
-// bytes, then the statuses and step counts of up to kSmallRows rows.  Seven
-// blocking copies of a few bytes took 60-80 us of a 118-bus solve's call.
-constexpr size_t kSmallHost = 64 * 1024;
-constexpr int kSmallRows = 4096;
-
 // Dense tail from which a row's factorizations are shared by a cluster.  Four
 // FP64 steps of one row on one CTA / on clusters of 16, 8 and 4: tail 95 0.75 /
 // 0.76, 0.81, 0.84 ms; 133 1.07 / 0.96, 1.06, 1.13; 204 1.78 / 1.35, 1.53, 1.65;
@@ -799,13 +869,19 @@ float launch(gs2g_session* s, const gs2g_run_opts& o, int n_rows, const double* 
   ck(cudaEventRecord(s->ev1, s->stream), "event");
   // the counters (and a small batch's statuses and steps) travel behind the
   // sweep and are there when it has been waited for
-  int* h_queue = reinterpret_cast<int*>(s->h_small);
-  auto* h_steps = reinterpret_cast<unsigned long long*>(s->h_small + 16);
-  ck(cudaMemcpyAsync(h_queue, s->d_queue.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, s->stream), "counters");
-  ck(cudaMemcpyAsync(h_steps, s->d_chord_steps.p, sizeof(*h_steps), cudaMemcpyDeviceToHost, s->stream), "step count");
-  const bool count = use_rows && n_rows > 0 && n_rows <= kSmallRows;
-  int* h_status = reinterpret_cast<int*>(s->h_small + 64);
-  int* h_iters = h_status + kSmallRows;
+  if (s->n_launched++ > 0 && !s->h_small) s->h_small = SmallBlocks::get().take();
+  int counters[4];
+  unsigned long long steps = 0;
+  const bool behind = s->h_small != nullptr;
+  const bool count = behind && use_rows && n_rows > 0 && n_rows <= kSmallRows;
+  int* const h_queue = reinterpret_cast<int*>(s->h_small);
+  char* const h_steps = s->h_small + 16;
+  int* const h_status = reinterpret_cast<int*>(s->h_small + 64);
+  int* const h_iters = h_status + kSmallRows;
+  if (behind) {
+    ck(cudaMemcpyAsync(h_queue, s->d_queue.p, sizeof(counters), cudaMemcpyDeviceToHost, s->stream), "counters");
+    ck(cudaMemcpyAsync(h_steps, s->d_chord_steps.p, sizeof(steps), cudaMemcpyDeviceToHost, s->stream), "step count");
+  }
   if (count) {
     ck(cudaMemcpyAsync(h_status, out.status, n_rows * sizeof(int), cudaMemcpyDeviceToHost, s->stream), "statuses");
     ck(cudaMemcpyAsync(h_iters, out.iters, n_rows * sizeof(int), cudaMemcpyDeviceToHost, s->stream), "steps");
@@ -814,9 +890,16 @@ float launch(gs2g_session* s, const gs2g_run_opts& o, int n_rows, const double* 
   float ms = 0;
   ck(cudaEventElapsedTime(&ms, s->ev0, s->ev1), "event time");
   for (int q = 0; q < GS2G_N_PHASES; ++q) s->tm.phase_cycles[q] = s->tm.phase_share[q] = 0;
-  s->tm.n_rescued = h_queue[1];
-  s->tm.n_base_start = h_queue[2];
-  s->tm.chord_steps = (int64_t)*h_steps;
+  if (behind) {
+    std::memcpy(counters, h_queue, sizeof(counters));
+    std::memcpy(&steps, h_steps, sizeof(steps));
+  } else {
+    ck(cudaMemcpy(counters, s->d_queue.p, sizeof(counters), cudaMemcpyDeviceToHost), "counters");
+    ck(cudaMemcpy(&steps, s->d_chord_steps.p, sizeof(steps), cudaMemcpyDeviceToHost), "step count");
+  }
+  s->tm.n_rescued = counters[1];
+  s->tm.n_base_start = counters[2];
+  s->tm.chord_steps = (int64_t)steps;
   if (count) {
     s->tm.total_iters = s->tm.n_failed = 0;
     for (int r = 0; r < n_rows; ++r) {
@@ -950,7 +1033,6 @@ int gs2g_session_create(int device, int n_bus, const int* ybus_indptr, const int
   ck(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking), "stream");
   ck(cudaEventCreate(&s->ev0), "event");
   ck(cudaEventCreate(&s->ev1), "event");
-  ck(cudaMallocHost(reinterpret_cast<void**>(&s->h_small), 2 * kSmallHost), "pinned buffer");
   upload_plan(s.get());
   s->d_ybus.ensure(s->ybus.size() * sizeof(double));
   ck(cudaMemcpy(s->d_ybus.p, s->ybus.data(), s->ybus.size() * sizeof(double), cudaMemcpyHostToDevice), "upload Ybus");
@@ -1019,7 +1101,6 @@ int gs2g_session_replan(gs2g_session* s, int tail_policy, double dense_rate, int
                                   s->pq.data(), (int)s->pq.size(), topt);
   ck(cudaStreamSynchronize(s->stream), "replan");
   s->plan = std::move(P);
-  s->plan_bufs.clear();
   upload_plan(s);
   s->base_factor_prec = -1;
   s->tm.plan_ms = s->plan.build_ms;
@@ -1038,7 +1119,7 @@ int gs2g_session_destroy(gs2g_session* s) {
     for (cudaEvent_t e : s->ev_stage)
       if (e) cudaEventDestroy(e);
     if (s->h_stage) cudaFreeHost(s->h_stage);
-    if (s->h_small) cudaFreeHost(s->h_small);
+    if (s->h_small) SmallBlocks::get().put(s->h_small);
     if (s->h_res) cudaFreeHost(s->h_res);
     if (s->stream) cudaStreamDestroy(s->stream);
     delete s;
@@ -1971,7 +2052,7 @@ int gs2g_get_results(const gs2g_session* s, double* v_out, double* residuals, in
   if (!s) throw std::invalid_argument("NULL session");
   DeviceGuard g(s->device);
   const size_t nr = s->last_rows_run, n = s->n_bus;
-  if (nr * (n * 2 * sizeof(double) + sizeof(double) + 2 * sizeof(int)) <= kSmallHost && nr) {
+  if (nr * (n * 2 * sizeof(double) + sizeof(double) + 2 * sizeof(int)) <= kSmallHost && nr && s->h_small) {
     // small: all copies (on the default stream, behind whatever it holds), one wait
     struct Part {
       void* dst;
