@@ -127,6 +127,7 @@ struct SweepArgs {
   // the base factor's head values in solve order (of the sweep's type):
   // base_slv[e] = HV[sl_pos[e]] (the slices' order)
   const char* base_slv;
+  int chord_first;  // mixed grids: the first chord CTA that starts on this grid
   int chord_slots;  // rows a chord CTA holds at a time, 1 .. chord_rows_per_cta()
   char* inverse_out;     // inverse mode: row r of the launch writes column r of M0^-1 here
   int factor_only;

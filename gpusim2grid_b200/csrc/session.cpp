@@ -1883,6 +1883,15 @@ int gs2g_run_multi(gs2g_session* const* sessions, int n_sessions, const gs2g_run
       b.alt_i = nullptr;
     }
   }
+  if (chord) {
+    std::stable_sort(gc.begin(), gc.end(),
+                     [](const gs2g::GridEntry& x, const gs2g::GridEntry& y) { return x.P.dim > y.P.dim; });
+    int64_t rows = 0;
+    for (auto& e : gc) {
+      e.a.chord_first = (int)(rows * n_chord / std::max(total, 1));
+      rows += e.a.n_rows;
+    }
+  }
   s0->d_ws.ensure(std::max((size_t)wsb * n_ctas, (size_t)cwsb * n_chord));
   for (auto& e : gc) e.a.workspace = s0->d_ws.as<char>();
   const size_t ge_bytes = sizeof(gs2g::GridEntry) * n_sessions;
