@@ -114,3 +114,24 @@ def test_base_chord_rows_match_the_oracle(n):
         Vo, so, _, _ = nr_solve(Yr, V0, S, pv, pq, max_iter=10, tol=1e-8)
         assert st[r] == so == 0
         assert np.abs(V[r] - Vo).max() <= TOL_V_MIXED
+
+
+def test_small_results_in_every_run_and_session():
+    """A session's first run and results are copied one by one, later ones
+    through a pinned block, of which there are 32: every copy is the same."""
+    g = _grid(40)
+    p, q = injection_scenarios(g, 3, seed=4)
+    sweeps = []
+    ref = None
+    for _ in range(34):
+        sw = InjectionSweepGPU(g.as_tuple(), init_from_n_powerflow=False, precision="fp64", nb_iter=10,
+                               scheduling="continuous", start="flat")
+        sw.set_injections(p, q, g.sn_mva)
+        for _ in range(3):
+            sw.compute()
+            got = [a.copy() for a in sw.session.results()] + [sw.session.timings()["total_iters"]]
+            ref = ref or got
+            for a, b in zip(got, ref):
+                np.testing.assert_array_equal(a, b)
+        sweeps.append(sw)
+    assert ref[-1] == ref[3].sum()
