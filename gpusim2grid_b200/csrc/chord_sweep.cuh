@@ -488,11 +488,59 @@ __device__ __noinline__ void chord_lists(const DevPlan& P, const T* __restrict__
   }
 }
 
+// U tail rows (tid + u * BS from r0) of the product below for every thread of
+// a warp; a row past the tail reads the last one and is not written.
+template <typename T, int U>
+__device__ __forceinline__ void chord_dense_rows(const T* __restrict__ Sinv, const int dim, const int nt, const int r0,
+                                                 const SlotVec<T>* ys, SlotVec<T>* yt) {
+  constexpr int N = U == 1 ? 16 : U == 2 ? 8 : 4;  // columns in flight
+  const T* at[U];
+  SlotVec<T> acc[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    at[u] = Sinv + min(r0 + (int)threadIdx.x + u * BS, nt - 1);
+#pragma unroll
+    for (int s = 0; s < CK; ++s) acc[u].v[s] = T(0);
+  }
+  int j = 0;
+  for (; j + N <= nt; j += N) {
+    T c[N][U];
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+      for (int u = 0; u < U; ++u) c[i][u] = at[u][(int64_t)i * dim];
+#pragma unroll
+    for (int u = 0; u < U; ++u) at[u] += (int64_t)N * dim;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const SlotVec<T> yj = ys[j + i];
+#pragma unroll
+      for (int u = 0; u < U; ++u) fms_slots(acc[u], -c[i][u], yj);
+    }
+  }
+  for (; j < nt; ++j) {
+    const SlotVec<T> yj = ys[j];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      fms_slots(acc[u], -*at[u], yj);
+      at[u] += dim;
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int r = r0 + (int)threadIdx.x + u * BS;
+    if (r < nt) yt[r] = acc[u];
+  }
+}
+
 // y_t <- Sinv y_t for all slots: the tail block of the base inverse (column j
 // at Minv + (p + j) * dim + p) times the CK columns held in shared memory.
 // Each thread owns up to four tail rows per pass; for each column a warp
-// reads 32 consecutive entries.  Eight columns in flight: 16 were no faster, and
-// loading the next 4 while 4 are multiplied was 1.8 times as slow.
+// reads 32 consecutive entries.  The chain of loads bounds it, so a warp takes
+// the row count its rows need as a constant and issues about 16 loads at a time
+// (with the row count tested at each load: 2000-bus N-1 sweep 5.53 -> 5.15 ms,
+// 6500-bus injections 15.6 -> 14.3); bit-identical.  Loading the next 4 columns
+// while 4 are multiplied was 1.8 times as slow.
 template <typename T>
 __device__ __noinline__ void chord_dense(const int p, const int nt, const int dim, const T* __restrict__ Minv,
                                           SlotVec<T>* y, SlotVec<T>* ys) {
@@ -501,24 +549,12 @@ __device__ __noinline__ void chord_dense(const int p, const int nt, const int di
   __syncthreads();
   const T* Sinv = Minv + (int64_t)p * dim + p;
   for (int r0 = 0; r0 < nt; r0 += 4 * BS) {
-    SlotVec<T> acc[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int s = 0; s < CK; ++s) acc[u].v[s] = T(0);
-    const int nr = min(4, (nt - r0 - tid + BS - 1) / BS);  // rows of this thread in the pass (may be <= 0)
-    const T* base = Sinv + r0 + tid;
-#pragma unroll 8
-    for (int j = 0; j < nt; ++j) {
-      const SlotVec<T> yj = ys[j];
-      const T* col = base + (int64_t)j * dim;
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (u < nr) fms_slots(acc[u], -col[u * BS], yj);
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (u < nr) y[p + r0 + tid + u * BS] = acc[u];
+    const int left = nt - r0 - (tid & ~31);  // rows from the warp's first on
+    if (left <= 0) continue;
+    if (left > 3 * BS) chord_dense_rows<T, 4>(Sinv, dim, nt, r0, ys, y + p);
+    else if (left > 2 * BS) chord_dense_rows<T, 3>(Sinv, dim, nt, r0, ys, y + p);
+    else if (left > BS) chord_dense_rows<T, 2>(Sinv, dim, nt, r0, ys, y + p);
+    else chord_dense_rows<T, 1>(Sinv, dim, nt, r0, ys, y + p);
   }
   __syncthreads();
 }
