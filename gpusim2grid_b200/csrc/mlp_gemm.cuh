@@ -299,11 +299,14 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     const int ew = warp - 2, quad = warp & 3, half = ew >> 2;
     float* buf = epi_smem + ew * 32 * EPI_LD;
     int n = 0;
-    for (int t = blockIdx.x; t < n_tiles && !*fail; t += gridDim.x, ++n) {
+    for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, ++n) {
       const int s = t / (g.tiles_m * g.tiles_n), mn = t % (g.tiles_m * g.tiles_n);
       const int m0 = (mn / g.tiles_n) * GT, n0 = (mn % g.tiles_n) * BN;
       const int acc = n & 1;
-      if (!mbar_wait(smem_u32(&tfull[acc]), (uint32_t)((n / 2) & 1), fail)) break;
+      // the whole warp goes on or gives up: lanes whose waits end differently
+      // (one sees the flag, another the barrier) must not part ahead of the
+      // .aligned loads; a tile that is full when the flag goes up is finished
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&tfull[acc]), (uint32_t)((n / 2) & 1), fail))) break;
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
 #pragma unroll 1
       for (int cc = 0; cc < BN / 2; cc += 32) {
