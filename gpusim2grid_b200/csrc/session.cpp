@@ -1099,7 +1099,10 @@ int gs2g_session_replan(gs2g_session* s, int tail_policy, double dense_rate, int
   topt.force_tau = force_tau;
   gs2g::Plan P = gs2g::build_plan(s->n_bus, s->y_ip.data(), s->y_ix.data(), s->pv.data(), (int)s->pv.size(),
                                   s->pq.data(), (int)s->pq.size(), topt);
-  ck(cudaStreamSynchronize(s->stream), "replan");
+  // the plan's device block may be written in place (PlanUpload): nothing may
+  // still read it, sweeps that gs2g_run_rows_noalloc left on a caller's stream
+  // included
+  ck(cudaDeviceSynchronize(), "replan");
   s->plan = std::move(P);
   upload_plan(s);
   s->base_factor_prec = -1;

@@ -114,3 +114,42 @@ def test_noalloc_rejects_base_chord_and_bad_rounds():
                                         out.data_ptr(), res.data_ptr(), st.data_ptr(), it.data_ptr(), None)
         assert rc == 1 and word in capi.gs2g_last_error()
     s.close()
+
+
+def test_replan_waits_for_sweeps_on_other_streams():
+    """The plan's device arrays are replaced only when no sweep of the session
+    reads them any more, on whichever stream it was enqueued."""
+    import torch
+    from gpusim2grid_b200._native import lib as G
+    from gpusim2grid_b200.synthetic import grid_by_name, injection_scenarios
+
+    g = grid_by_name("case2000_synth", 0)
+    Y, V0, S, _, _, pv, pq = g.as_tuple()
+    s = G.Session(0, g.n_bus, Y.indptr.astype(np.int32), Y.indices.astype(np.int32), Y.data, V0, S, pv, pq, 1)
+    n = 64
+    p, q = injection_scenarios(g, n, seed=9)
+    dev = torch.device("cuda", 0)
+    v0 = torch.from_numpy(V0.astype(np.complex128)).to(dev)
+    sbus = torch.from_numpy(((p + 1j * q) / g.sn_mva).astype(np.complex128)).to(dev)
+    capi = _capi()
+    opts = RunOpts(max_iter=10, tol=1e-8, precision=0, iters_per_round=1)
+    other = torch.cuda.Stream()
+    out = []
+    for replan in (False, True):
+        v_out = torch.full((n, g.n_bus), complex("nan+nanj"), dtype=torch.complex128, device=dev)
+        res = torch.full((n,), -1.0, dtype=torch.float64, device=dev)
+        st = torch.full((n,), -1, dtype=torch.int32, device=dev)
+        it = torch.full((n,), -1, dtype=torch.int32, device=dev)
+        torch.cuda.synchronize()
+        rc = capi.gs2g_run_rows_noalloc(s.handle(), n, v0.data_ptr(), 0, sbus.data_ptr(), g.n_bus,
+                                        ctypes.byref(opts), v_out.data_ptr(), res.data_ptr(), st.data_ptr(),
+                                        it.data_ptr(), other.cuda_stream)
+        assert rc == 0, capi.gs2g_last_error()
+        if replan:
+            s.replan(0, 40.0, -1)
+            assert other.query()
+        torch.cuda.synchronize()
+        out.append([t.cpu().numpy() for t in (v_out, res, st, it)])
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+    s.close()
