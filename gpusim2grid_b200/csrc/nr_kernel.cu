@@ -1637,10 +1637,10 @@ __device__ __forceinline__ int ld_shared_rank0(const int* p) {
 // loop in its workspace as sweep_kernel does, and the other CTAs join each
 // of its factorizations: the sparse head LU (each level's tasks split),
 // the Schur update of the dense tail (split by tail rows) and the dense tail
-// LU (dense_lu_cluster).  For the few rows the chord sweep
-// hands off and the few rows of an FP64 re-solve, whose factorizations
-// would otherwise each run on one SM after every other row has finished.
-// When the rows outnumber the clusters, every CTA takes rows of its own.
+// LU (dense_lu_cluster).  For small batches, the few rows the chord sweep
+// hands off and the few rows of an FP64 re-solve, whose factorizations would
+// otherwise each run on one SM while the others idle.  A cluster takes rows
+// from the queue until it is empty, all of them in the cluster's workspace.
 // Protocol, all through cluster barriers (every CTA passes the same number):
 // per row, the leader takes a queue entry and publishes it (barrier), every
 // CTA reads it (barrier); then for each factorization the leader posts
@@ -1650,7 +1650,7 @@ __device__ __forceinline__ int ld_shared_rank0(const int* p) {
 // together; after the row it posts
 // CLUSTER_CMD_DONE (barrier, read, barrier).
 // Largest cluster a row gets (16 needs the non-portable cluster-size opt-in;
-// the launch picks 16 or 8 by the number of rows, see launch_sweep_cluster).
+// the session picks 16, 8, 4 or 2 by the number of rows, see cluster_for).
 constexpr int HANDOFF_CLUSTER = 16;
 
 __device__ __forceinline__ unsigned cluster_nctarank() {
@@ -1661,8 +1661,11 @@ __device__ __forceinline__ unsigned cluster_nctarank() {
 
 // The other CTAs of a cluster while its leader runs a row: each command's
 // share of the factorization in the row's workspace, until the row is done.
+// A function of its own: inlined, it shares the row loop's registers (one
+// 2000-bus solve, four or five factorizations: FP64 4.08 -> 4.00 ms, FP32 3.70
+// -> 3.63).
 template <typename T>
-__device__ __forceinline__ void cluster_help(const DevPlan& P, double pivot_floor, char* ws, T* smem, const int* cmd,
+__device__ __noinline__ void cluster_help(const DevPlan& P, double pivot_floor, char* ws, T* smem, const int* cmd,
                                              int rank, int parts) {
   const WsLayout L = ws_layout<T>(P);
   T* S = reinterpret_cast<T*>(ws + L.S);
@@ -1705,23 +1708,6 @@ __global__ void __launch_bounds__(BS, GS2G_MIN_CTAS_PER_SM)
   const int parts = (int)cluster_nctarank();  // the launch's cluster size
   const int n_rows = a.n_rows_dev != nullptr ? *a.n_rows_dev : a.n_rows;
   PhaseProf prof;
-  if ((int64_t)n_rows * parts > gridDim.x) {
-    // more rows than clusters: sharing the LUs would leave rows waiting for a
-    // cluster, so every CTA runs rows of its own, as sweep_kernel does (the
-    // choice is the same for the whole grid: no cluster barrier is used)
-    prof.init(a.phase_cycles != nullptr && threadIdx.x == 0);
-    char* own = a.workspace + (int64_t)blockIdx.x * a.ws_stride;
-    for (;;) {
-      if (threadIdx.x == 0) s_row = atomicAdd(a.queue, 1);
-      __syncthreads();
-      const int q = s_row;
-      __syncthreads();  // every thread has read s_row before it is overwritten
-      if (q >= n_rows) break;
-      solve_row<T>(P, a, a.row_map != nullptr ? a.row_map[q] : q, own, own, sh, prof);
-    }
-    prof.flush(a.phase_cycles);
-    return;
-  }
   // one workspace per cluster
   char* ws = a.workspace + (int64_t)(blockIdx.x / parts) * a.ws_stride;
   prof.init(a.phase_cycles != nullptr && threadIdx.x == 0 && rank == 0);
