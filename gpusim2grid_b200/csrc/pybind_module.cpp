@@ -233,6 +233,7 @@ class Session {
 
   void set_chord(int mode) { check(gs2g_session_set_chord(h(), mode)); }
   void set_handoff(int cluster) { check(gs2g_session_set_handoff(h(), cluster)); }
+  int cluster_size() const { return gs2g_cluster_size(h()); }
   void set_results_mirror(bool on) { check(gs2g_session_set_results_mirror(h(), on ? 1 : 0)); }
   void set_row_order(bool on) { check(gs2g_session_set_row_order(h(), on ? 1 : 0)); }
   // adjoint: raw device pointers of rhs / lam [n_rows x dim_J] (caller-owned)
@@ -686,6 +687,7 @@ PYBIND11_MODULE(_gs2g, m) {
       .def("branch_loading", &Session::branch_loading)
       .def("set_chord", &Session::set_chord, py::arg("mode"))
       .def("set_handoff", &Session::set_handoff, py::arg("cluster"))
+      .def("cluster_size", &Session::cluster_size)
       .def("set_results_mirror", &Session::set_results_mirror, py::arg("on"))
       .def("set_row_order", &Session::set_row_order, py::arg("on"))
       .def("solve_jt", &Session::solve_jt, py::arg("n_rows"), py::arg("rhs"), py::arg("lam"))

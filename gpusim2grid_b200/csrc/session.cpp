@@ -207,6 +207,7 @@ struct gs2g_session {
   mutable std::mutex small_mutex;
   int n_launched = 0;
   bool counts_valid = false;  // tm.total_iters / n_failed are the last run's
+  int cluster = 0;            // CTAs per row of the last single-row launch (0: one)
   // pinned host copy of the last run's results (gs2g_get_results_host)
   void* h_res = nullptr;
   size_t h_res_bytes = 0;
@@ -783,8 +784,8 @@ std::pair<int, int> chord_shape(int rows, int fit, int asked) {
 float launch(gs2g_session* s, const gs2g_run_opts& o, int n_rows, const double* v0, int64_t v0_stride,
              const double* sbus, int64_t sbus_stride, bool use_rows, const OutBufs& out, int n_ctas_req) {
   gs2g::SweepArgs a = make_args(s, o, n_rows, v0, v0_stride, sbus, sbus_stride, use_rows, out);
-  int n_ctas = n_ctas_req > 0 ? n_ctas_req : gs2g::sweep_ctas(o.precision, s->device);
-  n_ctas = std::max(1, std::min(n_ctas, std::max(n_rows, 1)));
+  const int most = n_ctas_req > 0 ? n_ctas_req : gs2g::sweep_ctas(o.precision, s->device);
+  const int n_ctas = std::max(1, std::min(most, std::max(n_rows, 1)));
   const int64_t wsb = gs2g::workspace_bytes(s->dplan, o.precision);
   s->d_queue.ensure(4 * sizeof(int));  // [0] row queue, [1] rescue count, [2] alternative starts, [3] hand-offs
   // policy 2 (continuous): the chord sweep takes every row first, several
@@ -854,11 +855,12 @@ float launch(gs2g_session* s, const gs2g_run_opts& o, int n_rows, const double* 
     a.alt_i = nullptr;
   }
   // rows with a dense tail worth sharing, few enough that each gets a cluster
-  // of 16 (or 8) CTAs: the hand-offs, whose factorizations would otherwise run
-  // on one SM each after every other row has finished, and small batches
-  // (a single solve among them), which would leave the other SMs idle
-  const bool few = s->handoff_cluster && s->dplan.nt >= kClusterTail && (chord || n_rows <= n_ctas);
-  const int csize = few ? cluster_for(n_next, chord ? n_ctas : gs2g::sweep_ctas(o.precision, s->device), o.precision) : 0;
+  // of CTAs: the hand-offs, whose factorizations would otherwise run on one SM
+  // each after every other row has finished, and small batches (a single solve
+  // among them), which would leave the other SMs idle
+  const bool few = s->handoff_cluster && s->dplan.nt >= kClusterTail;
+  const int csize = few ? cluster_for(n_next, chord ? n_ctas : most, o.precision) : 0;
+  s->cluster = csize;
   if (n_next > 0 && csize > 0) {
     ck((cudaError_t)gs2g::launch_sweep_cluster(s->dplan, a, o.precision, csize, n_next * csize, s->stream),
        "hand-off cluster launch");
@@ -1762,6 +1764,7 @@ int gs2g_run_subset(gs2g_session* s, const gs2g_run_opts* o_, int n_sub, const i
   const int csize = s->handoff_cluster && s->dplan.nt >= kClusterTail ? cluster_for(n_sub, n_ctas, o.precision) : 0;
   const bool cluster = n_sub > 0 && csize > 0;
   n_ctas = cluster ? n_sub * csize : std::max(1, std::min(n_ctas, std::max(n_sub, 1)));
+  s->cluster = csize;
   const int64_t wsb = gs2g::workspace_bytes(s->dplan, o.precision);
   s->d_ws.ensure((size_t)wsb * n_ctas);
   s->d_queue.ensure(3 * sizeof(int));
@@ -1928,6 +1931,7 @@ int gs2g_run_multi(gs2g_session* const* sessions, int n_sessions, const gs2g_run
     for (int i = 0; i < n_sessions; ++i) worth = worth || sessions[i]->dplan.nt >= kClusterTail;
     csize = s0->handoff_cluster && worth ? cluster_for(n_next, n_ctas, o.precision) : 0;
   }
+  for (int i = 0; i < n_sessions; ++i) sessions[i]->cluster = csize;
   const gs2g::GridEntry* d_ge = reinterpret_cast<const gs2g::GridEntry*>(s0->d_multi.p);
   if (n_next > 0 && csize > 0)
     ck((cudaError_t)gs2g::launch_sweep_multi_cluster(d_ge, n_sessions, d_begin, n_next, s0->d_queue.as<int>(),
@@ -2181,6 +2185,8 @@ int gs2g_get_timings(const gs2g_session* s, gs2g_timings* out) {
   }
   GS2G_CATCH
 }
+
+int gs2g_cluster_size(const gs2g_session* s) { return s ? s->cluster : 0; }
 
 int gs2g_sync(gs2g_session* s) {
   GS2G_TRY

@@ -203,6 +203,9 @@ int gs2g_session_set_chord(gs2g_session* s, int mode);
  * 64 always use one CTA.  No counterpart in the reference (its batch LU has
  * no per-row kernel). */
 int gs2g_session_set_handoff(gs2g_session* s, int cluster);
+/* CTAs that shared each row's factorizations in the session's last run (of a
+ * base_chord run: those of its hand-offs); 0: one CTA per row. */
+int gs2g_cluster_size(const gs2g_session* s);
 /* Order in which the persistent sweeps take the rows: on = 1 (default) by a
  * difficulty estimate, largest first -- the row's distance from the base
  * injections (sum over buses of |dP| + |dQ|, from gs2g_set_injections) plus

@@ -63,6 +63,25 @@ def test_small_batches_on_clusters_equal_one_cta_per_row(rows, precision):
         np.testing.assert_array_equal(a, b)
 
 
+@pytest.mark.parametrize("n_ctas,sizes", [(0, {16}), (4, {0}), (8, {2}), (64, {16}), (63, {8})])
+def test_a_callers_cta_count_bounds_the_clusters(n_ctas, sizes):
+    """n_ctas is the number of CTAs a run may have, clusters included."""
+    from gpusim2grid_b200._native import lib
+    g = _grid(900)
+    p, q = injection_scenarios(g, 4, seed=5)
+    sw = InjectionSweepGPU(g.as_tuple(), init_from_n_powerflow=False, precision="fp64", nb_iter=10,
+                           scheduling="continuous", start="flat")
+    sw.set_injections(p, q, g.sn_mva)
+    s = sw.session
+    for rows in (None, np.arange(4, dtype=np.int32)):  # the whole batch, then a subset of it
+        if rows is None:
+            s.run(10, 1e-8, False, lib.PREC_FP64, lib.START_VINIT, n_ctas=n_ctas)
+        else:
+            s.run_subset(rows, 10, 1e-8, False, lib.PREC_FP64, lib.START_VINIT, n_ctas=n_ctas)
+        assert s.cluster_size() in sizes
+        assert np.all(s.results()[2] == 0)
+
+
 def test_single_solve_on_a_cluster_equals_one_cta():
     g = grid_by_name("case2000_synth", 0)
     got = []
