@@ -758,7 +758,8 @@ constexpr int kClusterTail = 160;
 
 // Cluster size for `rows` rows that each get a cluster: the largest of 16, 8, 4
 // and 2 whose clusters the device holds `rows` of at once and that stays
-// within `n_ctas` CTAs, else 0 (one CTA per row).  (A second round of clusters
+// within `n_ctas` CTAs (the caller's, else the device's: not the batch's rows, of
+// which hand-offs are a part), else 0 (one CTA per row).  (A second round of clusters
 // costs more than smaller ones: 16 rows of the 2000-bus grid take 8.0 ms on
 // clusters of 16, which run in two rounds, and 4.4 ms on clusters of 8.)
 int cluster_for(int rows, int n_ctas, int prec) {
@@ -859,7 +860,7 @@ float launch(gs2g_session* s, const gs2g_run_opts& o, int n_rows, const double* 
   // each after every other row has finished, and small batches (a single solve
   // among them), which would leave the other SMs idle
   const bool few = s->handoff_cluster && s->dplan.nt >= kClusterTail;
-  const int csize = few ? cluster_for(n_next, chord ? n_ctas : most, o.precision) : 0;
+  const int csize = few ? cluster_for(n_next, most, o.precision) : 0;
   s->cluster = csize;
   if (n_next > 0 && csize > 0) {
     ck((cudaError_t)gs2g::launch_sweep_cluster(s->dplan, a, o.precision, csize, n_next * csize, s->stream),
@@ -1839,8 +1840,8 @@ int gs2g_run_multi(gs2g_session* const* sessions, int n_sessions, const gs2g_run
   }
   const double upload_ms = ms_since(t0);
   const int total = begin[n_sessions];
-  int n_ctas = o.n_ctas > 0 ? o.n_ctas : gs2g::sweep_ctas(o.precision, s0->device);
-  n_ctas = std::max(1, std::min(n_ctas, std::max(total, 1)));
+  const int most = o.n_ctas > 0 ? o.n_ctas : gs2g::sweep_ctas(o.precision, s0->device);
+  const int n_ctas = std::max(1, std::min(most, std::max(total, 1)));
   // policy 2 (continuous): a multi-grid chord sweep first (several rows per
   // CTA on each grid's base factor), then the single-row sweep continues the
   // rows it hands off, from v_out / iters_out on their own factors
@@ -1929,7 +1930,7 @@ int gs2g_run_multi(gs2g_session* const* sessions, int n_sessions, const gs2g_run
     ck(cudaStreamSynchronize(s0->stream), "multi-grid chord sweep");
     bool worth = false;
     for (int i = 0; i < n_sessions; ++i) worth = worth || sessions[i]->dplan.nt >= kClusterTail;
-    csize = s0->handoff_cluster && worth ? cluster_for(n_next, n_ctas, o.precision) : 0;
+    csize = s0->handoff_cluster && worth ? cluster_for(n_next, most, o.precision) : 0;
   }
   for (int i = 0; i < n_sessions; ++i) sessions[i]->cluster = csize;
   const gs2g::GridEntry* d_ge = reinterpret_cast<const gs2g::GridEntry*>(s0->d_multi.p);

@@ -82,6 +82,27 @@ def test_a_callers_cta_count_bounds_the_clusters(n_ctas, sizes):
         assert np.all(s.results()[2] == 0)
 
 
+def _leaving(g, rows, seed):
+    """A mixed sweep whose rows all leave the chord for their own factor."""
+    p, q = injection_scenarios(g, rows, seed=seed)
+    sw = InjectionSweepGPU(g.as_tuple(), init_from_n_powerflow=False, precision="mixed", nb_iter=10,
+                           scheduling="continuous", strategy="base_chord")
+    sw.refactor_ratio = 1e-9
+    sw.set_injections(p, q, g.sn_mva)
+    return sw
+
+
+@pytest.mark.parametrize("multi", [False, True])
+def test_handoffs_get_clusters_by_the_chip(multi):
+    """The rows that a chord sweep hands off share the chip, however few rows
+    the batch had."""
+    sweeps = [_leaving(_grid(n), 3, n) for n in ((900, 700) if multi else (900,))]
+    compute_many(sweeps) if multi else sweeps[0].compute(batch_size=0)
+    for sw in sweeps:
+        assert np.all(sw.get_row_factorizations() > 0)
+        assert sw.session.cluster_size() in (8, 16)
+
+
 def test_single_solve_on_a_cluster_equals_one_cta():
     g = grid_by_name("case2000_synth", 0)
     got = []
