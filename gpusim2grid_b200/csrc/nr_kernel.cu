@@ -1873,6 +1873,8 @@ int64_t workspace_hv_offset(const DevPlan& P, int prec) {
 }
 
 namespace {
+// Shared memory of which an SM holds one CTA's (max_clusters' query alone).
+constexpr int kSmEach = 128 * 1024;
 // Dynamic shared memory above 48 KB needs an opt-in per kernel (per device
 // context); cheap and idempotent, so it is set before every query / launch.
 cudaError_t opt_in_smem() {
@@ -1891,11 +1893,9 @@ cudaError_t opt_in_smem() {
   e = cudaFuncSetAttribute(sweep_kernel_multi<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            smem_bytes<float>());
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(sweep_kernel_cluster<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           smem_bytes<float>());
+  e = cudaFuncSetAttribute(sweep_kernel_cluster<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmEach);
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(sweep_kernel_cluster<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           smem_bytes<double>());
+  e = cudaFuncSetAttribute(sweep_kernel_cluster<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmEach);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(sweep_kernel_multi_cluster<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            smem_bytes<float>());
@@ -2065,9 +2065,10 @@ bool cluster_ok(int cluster, int n_ctas) {
 }
 }  // namespace
 
-int max_clusters(int prec, int cluster) {
+int max_clusters(int prec, int cluster, bool sm_each) {
   if (!cluster_ok(cluster, cluster) || opt_in_smem() != cudaSuccess) return 0;
   ClusterLaunch l(prec, cluster, cluster, nullptr);
+  if (sm_each) l.cfg.dynamicSmemBytes = kSmEach;
   int n = 0;
   const cudaError_t e = prec == 1 ? cudaOccupancyMaxActiveClusters(&n, sweep_kernel_cluster<float>, &l.cfg)
                                   : cudaOccupancyMaxActiveClusters(&n, sweep_kernel_cluster<double>, &l.cfg);

@@ -209,9 +209,9 @@ int sweep_ctas(int prec, int device);
 // times ws_stride), and all of them share each of its head LUs, Schur
 // updates and dense tail LUs.  n_ctas a multiple of the cluster size.
 int handoff_cluster_size();
-// Clusters of `cluster` CTAs of that sweep that the device holds at once (0: the
-// size is not available).
-int max_clusters(int prec, int cluster);
+// Clusters of `cluster` CTAs of that sweep that the device holds at once, or holds
+// with an SM to each CTA (0: the size is not available).
+int max_clusters(int prec, int cluster, bool sm_each);
 
 // Batched adjoint (FP64): lam[r] = J_r^-T rhs[r] for the a.n_rows rows of a
 // sweep (a.v_out the converged voltages, a.status_out their statuses, the

@@ -750,22 +750,43 @@ gs2g::SweepArgs make_args(gs2g_session* s, const gs2g_run_opts& o, int n_rows, c
   return a;
 }
 
-// Dense tail from which a row's factorizations are shared by a cluster.  Four
-// FP64 steps of one row on one CTA / on clusters of 16, 8 and 4: tail 95 0.75 /
-// 0.76, 0.81, 0.84 ms; 133 1.07 / 0.96, 1.06, 1.13; 204 1.78 / 1.35, 1.53, 1.65;
-// 518 7.9 / 3.4, 4.1, 6.0.
-constexpr int kClusterTail = 160;
+// Dense tails from which a row's factorizations are shared by a cluster, of 16, 8
+// or 4 CTAs and of 2: with an SM to each CTA, and with the two on an SM that fit.
+// (The table is in cluster_for.)
+constexpr int kClusterTail = 140, kClusterTailTwo = 256;
+constexpr int kPairTail = 176, kPairTailTwo = 300;
 
-// Cluster size for `rows` rows that each get a cluster: the largest of 16, 8, 4
-// and 2 whose clusters the device holds `rows` of at once and that stays
-// within `n_ctas` CTAs (the caller's, else the device's: not the batch's rows, of
-// which hand-offs are a part), else 0 (one CTA per row).  (A second round of clusters
-// costs more than smaller ones: 16 rows of the 2000-bus grid take 8.0 ms on
-// clusters of 16, which run in two rounds, and 4.4 ms on clusters of 8.)
-int cluster_for(int rows, int n_ctas, int prec) {
+// Cluster size for `rows` rows with dense tails of `tail` (the largest) that each
+// get a cluster: the largest of 16, 8, 4 and 2 whose clusters the device holds
+// `rows` of at once and that stays within `n_ctas` CTAs (the caller's, else the
+// device's: not the batch's rows, of which hand-offs are a part), else 0 (one CTA
+// per row).  A second round of clusters costs more than smaller ones: 16 rows of
+// the 2000-bus grid took 8.0 ms on clusters of 16, which run in two rounds, and
+// 4.4 ms on clusters of 8.  Four steps with a factorization each, us on one CTA a
+// row / on the largest size that leaves an SM to each CTA / on the largest size
+// that fits (two to an SM):
+//   FP64  tail  133        150        179             204             262
+//   1 row       994  954   1100 1010  1357 1141       1668 1313       2303 1603
+//   14 rows    1022  972   1115 1017  1379 1170 1297  1665 1372 1526  2329 1674 1906
+//   33 rows    1025 1002   1117 1068  1379 1230 1324  1676 1471 1563  2335 1840 1985
+//   71 rows    1022 1092   1125 1161  1388 1366 1381  1704 1661 1685  2337 2149 2167
+//   148 rows   1025        1131       1397      1568  1941      2007  2852      2905
+//   FP32  tail  133        150        179             204             262
+//   1 row       883  883    994  901  1217 1028       1472 1205       2014 1478
+//   14 rows     891  884    986  933  1227 1067 1166  1473 1245 1375  2038 1498 1721
+//   33 rows     907  915   1002  967  1233 1105 1194  1501 1321 1421  2053 1638 1770
+//   71 rows     912  981   1000 1053  1237 1232 1258  1489 1467 1513  2070 1909 1930
+//   148 rows    923        1006       1249      1408  1517      1703  2129      2254
+// Below, clusters gain nothing (tail 119: 858 / 859, 793 / 783 for one row); above,
+// two CTAs to an SM pay (tail 341, 71 rows: 3783 3260 2981 and 2893 2526 2510; 148
+// rows: 4071 and 4027, 3524 and 3413; tail 541: 9035 and 8958, 7772 and 6910).
+int cluster_for(int tail, int rows, int n_ctas, int prec) {
   if (rows <= 0) return 0;
-  for (int c = gs2g::handoff_cluster_size(); c >= 2; c /= 2)
-    if ((int64_t)rows * c <= n_ctas && rows <= gs2g::max_clusters(prec, c)) return c;
+  for (int c = gs2g::handoff_cluster_size(); c >= 2; c /= 2) {
+    if ((int64_t)rows * c > n_ctas || tail < (c == 2 ? kPairTail : kClusterTail)) continue;
+    const bool two = tail >= (c == 2 ? kPairTailTwo : kClusterTailTwo);
+    if (rows <= gs2g::max_clusters(prec, c, !two)) return c;
+  }
   return 0;
 }
 
@@ -859,8 +880,7 @@ float launch(gs2g_session* s, const gs2g_run_opts& o, int n_rows, const double* 
   // of CTAs: the hand-offs, whose factorizations would otherwise run on one SM
   // each after every other row has finished, and small batches (a single solve
   // among them), which would leave the other SMs idle
-  const bool few = s->handoff_cluster && s->dplan.nt >= kClusterTail;
-  const int csize = few ? cluster_for(n_next, most, o.precision) : 0;
+  const int csize = s->handoff_cluster ? cluster_for(s->dplan.nt, n_next, most, o.precision) : 0;
   s->cluster = csize;
   if (n_next > 0 && csize > 0) {
     ck((cudaError_t)gs2g::launch_sweep_cluster(s->dplan, a, o.precision, csize, n_next * csize, s->stream),
@@ -1762,7 +1782,7 @@ int gs2g_run_subset(gs2g_session* s, const gs2g_run_opts* o_, int n_sub, const i
   int n_ctas = o.n_ctas > 0 ? o.n_ctas : gs2g::sweep_ctas(o.precision, s->device);
   // few rows with a dense tail worth sharing (an FP64 re-solve of the rows
   // a mixed sweep did not converge): a cluster of CTAs per row
-  const int csize = s->handoff_cluster && s->dplan.nt >= kClusterTail ? cluster_for(n_sub, n_ctas, o.precision) : 0;
+  const int csize = s->handoff_cluster ? cluster_for(s->dplan.nt, n_sub, n_ctas, o.precision) : 0;
   const bool cluster = n_sub > 0 && csize > 0;
   n_ctas = cluster ? n_sub * csize : std::max(1, std::min(n_ctas, std::max(n_sub, 1)));
   s->cluster = csize;
@@ -1928,9 +1948,9 @@ int gs2g_run_multi(gs2g_session* const* sessions, int n_sessions, const gs2g_run
     ck(cudaMemcpyAsync(&n_next, s0->d_queue.as<int>() + 3, sizeof(int), cudaMemcpyDeviceToHost, s0->stream),
        "hand-off count");
     ck(cudaStreamSynchronize(s0->stream), "multi-grid chord sweep");
-    bool worth = false;
-    for (int i = 0; i < n_sessions; ++i) worth = worth || sessions[i]->dplan.nt >= kClusterTail;
-    csize = s0->handoff_cluster && worth ? cluster_for(n_next, most, o.precision) : 0;
+    int tail = 0;
+    for (int i = 0; i < n_sessions; ++i) tail = std::max(tail, sessions[i]->dplan.nt);
+    csize = s0->handoff_cluster ? cluster_for(tail, n_next, most, o.precision) : 0;
   }
   for (int i = 0; i < n_sessions; ++i) sessions[i]->cluster = csize;
   const gs2g::GridEntry* d_ge = reinterpret_cast<const gs2g::GridEntry*>(s0->d_multi.p);

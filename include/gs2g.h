@@ -192,16 +192,16 @@ int gs2g_session_replan(gs2g_session* s, int tail_policy, double dense_rate, int
  * convergence); mode 1: plain chord steps, the same decisions as the
  * single-row sweep; mode 0: every row in the single-row sweep. */
 int gs2g_session_set_chord(gs2g_session* s, int mode);
-/* Rows that factor their own Jacobian after a chord sweep (its hand-offs),
- * and the rows of a gs2g_run_subset when there are few of them (at most one
- * per 8 CTAs of a full launch: the FP64 re-solve of the rows a mixed sweep
- * did not converge): cluster = 1 (default) runs each such row on a cluster
- * of 16 CTAs (8 when 16 per row do not fit in one launch), the leading CTA
- * running the row and all of them sharing each of its head LUs, Schur
- * updates and dense tail LUs (bit-identical to the one-CTA factorization,
- * FP32 and FP64); 0 runs each on one CTA.  Grids whose dense tail is under
- * 64 always use one CTA.  No counterpart in the reference (its batch LU has
- * no per-row kernel). */
+/* Rows that are few and factor their own Jacobian: the hand-offs of a chord
+ * sweep, small batches and single solves, the rows of a gs2g_run_subset (the
+ * FP64 re-solve of the rows a mixed sweep did not converge).  cluster = 1
+ * (default) runs each such row on a cluster of 16, 8, 4 or 2 CTAs, by the grid's
+ * dense tail and by how many rows there are; the leading CTA runs the row and
+ * all of them share each of its head LUs, Schur updates and dense tail LUs
+ * (bit-identical to the one-CTA factorization, FP32 and FP64).  The clusters
+ * stay within gs2g_run_opts.n_ctas where that is given.  0 runs each row on one
+ * CTA, as do grids whose dense tail is under 140.  No counterpart in the
+ * reference (its batch LU has no per-row kernel). */
 int gs2g_session_set_handoff(gs2g_session* s, int cluster);
 /* CTAs that shared each row's factorizations in the session's last run (of a
  * base_chord run: those of its hand-offs); 0: one CTA per row. */

@@ -44,11 +44,18 @@ def test_solves_match_the_oracle(n, precision):
             assert np.abs(V[r] - Vo).max() <= (TOL_V_FP64 if precision == "fp64" else TOL_V_MIXED)
 
 
+# (buses, rows, CTAs per row): dense tails of 133 (no clusters), 150 (none of 2), 204 (an SM
+# to each CTA) and 341 (two on an SM); rows well inside what any B200 holds of each size
+CLUSTERS = [(402, 1, 0), (402, 20, 0), (500, 1, 16), (500, 10, 8), (500, 25, 4), (500, 50, 0), (700, 1, 16),
+            (700, 12, 8), (700, 25, 4), (700, 60, 2), (700, 100, 0), (1200, 1, 16), (1200, 20, 8), (1200, 50, 4),
+            (1200, 100, 2), (1200, 149, 0)]
+
+
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
-@pytest.mark.parametrize("rows", [1, 18, 19, 37, 38, 74, 75, 148, 149])
-def test_small_batches_on_clusters_equal_one_cta_per_row(rows, precision):
-    """Clusters of 16, 8, 4 and 2 CTAs and none, by the number of rows."""
-    g = _grid(402)
+@pytest.mark.parametrize("n,rows,size", CLUSTERS)
+def test_small_batches_on_clusters_equal_one_cta_per_row(n, rows, size, precision):
+    """Clusters of 16, 8, 4 and 2 CTAs and none, by the dense tail and the number of rows."""
+    g = _grid(n)
     p, q = injection_scenarios(g, rows, seed=5)
     out = []
     for cluster in (1, 0):
@@ -57,6 +64,7 @@ def test_small_batches_on_clusters_equal_one_cta_per_row(rows, precision):
         sw.session.set_handoff(cluster)
         sw.set_injections(p, q, g.sn_mva)
         sw.compute()
+        assert sw.session.cluster_size() == (size if cluster else 0)
         out.append([a.copy() for a in sw.results_view()])
         assert np.all(out[-1][2] == 0)
     for a, b in zip(*out):
