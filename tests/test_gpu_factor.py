@@ -6,7 +6,8 @@ import numpy as np
 import pytest
 
 from conftest import TOL_V_FP64, TOL_V_MIXED
-from gpusim2grid_b200 import AcPfGPU, ContingencyAnalysisGPU, InjectionSweepGPU, ScenarioSweepGPU, compute_many
+from gpusim2grid_b200 import (AcPfGPU, ContingencyAnalysisGPU, InjectionSweepGPU, RowStatus, ScenarioSweepGPU,
+                              compute_many)
 from gpusim2grid_b200.synthetic import grid_by_name, injection_scenarios, make_grid, n1_branches, scenario_outages
 from oracle.nr_oracle import nr_solve
 
@@ -123,23 +124,30 @@ def test_single_solve_on_a_cluster_equals_one_cta():
     assert got[0][1:] == got[1][1:]
 
 
-def test_multi_grid_handoffs_on_clusters_equal_one_cta_per_row():
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("rows,size", [(1, 16), (10, 8), (25, 4), (50, 2), (90, 0)])
+def test_multi_grid_handoffs_on_clusters_equal_one_cta_per_row(rows, size, precision):
+    """Every row of a small and a large grid leaves the chord; the small grid's
+    (dense tail 42) are run by one CTA of their cluster."""
     grids = [grid_by_name("case118_synth", 0), grid_by_name("case2000_synth", 0)]
     out = []
     for cluster in (1, 0):
         sweeps = []
         for i, g in enumerate(grids):
-            p, q = injection_scenarios(g, 64, seed=20 + i)
-            f = ScenarioSweepGPU(g.as_tuple(), init_from_n_powerflow=False, precision="mixed", nb_iter=10,
+            p, q = injection_scenarios(g, rows, seed=20 + i)
+            f = ScenarioSweepGPU(g.as_tuple(), init_from_n_powerflow=False, precision=precision, nb_iter=10,
                                  scheduling="continuous", strategy="base_chord")
-            f.refactor_ratio = 0.05  # nearly every row leaves the chord for its own factor
+            f.refactor_ratio = 1e-9
             f.set_branch_data(*g.branch_data())
             f.set_injections(p, q, g.sn_mva)
-            f.set_topology(scenario_outages(g, 64, seed=40 + i))
+            f.set_topology(scenario_outages(g, rows, seed=40 + i))
             f.session.set_handoff(cluster)
             sweeps.append(f)
         compute_many(sweeps)
-        assert sum(int(f.get_row_factorizations().sum()) for f in sweeps) > 0
+        for f in sweeps:
+            ran = f.results_view()[2] != RowStatus.NOT_SIMULATED  # an outage that splits the grid is not simulated
+            assert np.any(ran) and np.all(f.get_row_factorizations()[ran] > 0)
+            assert f.session.cluster_size() == (size if cluster else 0)
         out.append([a.copy() for f in sweeps for a in f.results_view()])
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
