@@ -256,9 +256,11 @@ class WarmStartMLP:
         w["loss"].zero_()
         self._forward(X, w)
         self._backward(X, T, w, scale)
+        # each its own tensor (one that is kept must not keep all of them), copied
+        # behind the pass, ahead of the wait for its error flag
+        grads = [(self._view(self.grad, l, False).clone(), self._view(self.grad, l, True).clone())
+                 for l in range(self.layers + 1)]
         self.check()
-        flat = self.grad.clone()
-        grads = [(self._view(flat, l, False), self._view(flat, l, True)) for l in range(self.layers + 1)]
         return grads, float(w["loss"].item())
 
     def check(self):

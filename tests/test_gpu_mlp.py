@@ -198,3 +198,18 @@ def test_fused_inputs_equal_the_torch_path(g118):
         # equal up to the fp32 summation order of two trips at one bus (one bf16 step at most)
         assert torch.all((a - b).abs() <= 2 ** -7 * b.abs().clamp(min=1e-3))
         assert torch.all(X[37:] == 0) and torch.all(X[:, ls.n_in:] == 0)
+
+
+def test_gradients_are_tensors_of_their_own():
+    """Keeping (or saving) one layer's gradient keeps that layer's memory, and the next call leaves it alone."""
+    import torch
+    from gpusim2grid_b200.warmstart import WarmStartMLP
+    net = WarmStartMLP(100, 60, hidden=128, layers=2, seed=3)
+    X = net.device_inputs(torch.randn(128, 100, device="cuda"))
+    T = net.device_targets(torch.randn(128, 60, device="cuda"))
+    first, _ = net.gradients(X, T)
+    kept = [t.clone() for pair in first for t in pair]
+    net.gradients(X, 2 * T)
+    for got, want in zip((t for pair in first for t in pair), kept):
+        assert got.untyped_storage().nbytes() == got.numel() * got.element_size()
+        assert torch.equal(got, want)
