@@ -72,6 +72,47 @@ def test_small_batches_on_clusters_equal_one_cta_per_row(n, rows, size, precisio
         np.testing.assert_array_equal(a, b)
 
 
+FORMS = {
+    "chunked": dict(nb_iter=6),
+    "rounds": dict(scheduling="continuous", nb_iter=6, nb_iter_per_round=2),
+    "adaptive": dict(scheduling="continuous", nb_iter=10, strategy="adaptive"),
+    "scaled": dict(scheduling="continuous", nb_iter=10, scaling_max_voltage_change=True, max_dVa=0.05, max_dVm=0.01),
+    "masked": dict(scheduling="continuous", nb_iter=10, handle_disconnected_grid=True),
+    "base_chord": dict(scheduling="continuous", nb_iter=10, strategy="base_chord"),
+}
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("form", FORMS)
+def test_options_on_clusters_equal_one_cta_per_row(form, precision):
+    """Outage rows (some split the grid, one has a start that is not finite) in every
+    schedule and option, on clusters and on one CTA each: the same bits."""
+    g = _grid(700)
+    safe = set(int(b) for b in n1_branches(g))
+    splits = [b for b in range(g.n_branch) if b not in safe][:4]
+    rows = [[b] for b in splits] + [[b] for b in sorted(safe)[:6]] + [sorted(safe)[8:10]]
+    out = []
+    for cluster in (1, 0):
+        ca = ContingencyAnalysisGPU(g.as_tuple(), init_from_n_powerflow=False, precision=precision, **FORMS[form])
+        ca.set_branch_data(*g.branch_data())
+        ca.set_branch_limits(np.full(g.n_branch, 50.0))
+        ca.add_contingencies_by_branch_id(rows)
+        ca.session.set_handoff(cluster)
+        if form == "base_chord":
+            ca.session.set_chord(0)  # every row in the single-row sweep
+        start = np.tile(g.vinit(), (len(rows), 1))
+        start[5] = np.nan
+        ca.set_start_voltages(start)
+        ca.compute()
+        if form != "masked":  # (there the FP64 re-solve of a failed row may be the last run)
+            assert ca.session.cluster_size() == (8 if cluster else 0)
+        out.append([ca.V_results, ca.get_row_status(), ca.get_row_iterations(), ca.get_row_factorizations(),
+                    *ca.branch_loading()])
+    assert len(splits) == 4 and np.any(out[0][1] == RowStatus.CONVERGED)
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+
+
 @pytest.mark.parametrize("n_ctas,sizes", [(0, {16}), (4, {0}), (8, {2}), (64, {16}), (63, {8})])
 def test_a_callers_cta_count_bounds_the_clusters(n_ctas, sizes):
     """n_ctas is the number of CTAs a run may have, clusters included."""

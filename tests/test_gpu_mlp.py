@@ -213,3 +213,28 @@ def test_gradients_are_tensors_of_their_own():
     for got, want in zip((t for pair in first for t in pair), kept):
         assert got.untyped_storage().nbytes() == got.numel() * got.element_size()
         assert torch.equal(got, want)
+
+
+def test_network_from_another_thread():
+    """A thread that has made no CUDA call of its own runs the network: the
+    tensor maps are encoded before anything is launched."""
+    import threading
+    import torch
+    from gpusim2grid_b200.warmstart import WarmStartMLP
+    net = WarmStartMLP(100, 60, hidden=128, layers=2, seed=3)
+    X = net.device_inputs(torch.randn(128, 100, device="cuda"))
+    want = net.predict(X).clone()
+    got = []
+
+    def work():
+        try:
+            got.append(net.predict(X).clone())
+        except Exception as e:  # shown by the assertion below
+            got.append(e)
+
+    t = threading.Thread(target=work)
+    t.start()
+    t.join()
+    assert isinstance(got[0], torch.Tensor), got[0]
+    torch.cuda.synchronize()
+    assert torch.equal(got[0], want)
