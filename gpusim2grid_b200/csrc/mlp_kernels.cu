@@ -357,9 +357,19 @@ bool operand_map(CUtensorMap* map, const void* p, int ld, bool mn, int rows, int
   const cuuint64_t dims[2] = {(cuuint64_t)(mn ? rows : K), (cuuint64_t)(mn ? K : rows)};
   const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
   const cuuint32_t boxes[2] = {64u, (cuuint32_t)(mn ? 64 : box)}, ones[2] = {1u, 1u};
-  return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(p), dims, strides, boxes, ones,
-                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  const auto run = [&] {
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(p), dims, strides, boxes, ones,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = run();
+  if (r == CUDA_ERROR_INVALID_CONTEXT) {
+    // a thread's first CUDA call: the runtime binds its context with its first
+    // launch or here, the driver's encoder does not
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) r = run();
+  }
+  return r == CUDA_SUCCESS;
 }
 
 template <int BN, bool A_MN, bool B_MN, int OP>
