@@ -265,7 +265,7 @@ class Session {
 
   // the base case is a single solve: the reference's step-then-test order by default
   py::tuple solve_base(int max_iter, double tol, int precision, double pivot_floor, bool step_then_check) {
-    gs2g_run_opts o = make_opts(max_iter, tol, false, precision, GS2G_START_VINIT, pivot_floor, 1, false, 0, 0.0, 0,
+    gs2g_run_opts o = make_opts(max_iter, tol, false, precision, GS2G_START_VINIT, pivot_floor, 0, false, 0, 0.0, 0,
                                 false, 1, step_then_check);
     py::array_t<cplx> V(n_bus_);
     int st = 0, it = 0;

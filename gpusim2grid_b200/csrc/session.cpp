@@ -1560,7 +1560,7 @@ int gs2g_solve_base(gs2g_session* s, const gs2g_run_opts* o_, double* v_out, int
   s->b_status.ensure(sizeof(int));
   s->b_iters.ensure(sizeof(int));
   OutBufs ob{s->b_v.as<double>(), s->b_res.as<double>(), s->b_status.as<int>(), s->b_iters.as<int>()};
-  const float ms = launch(s, o, 1, s->d_vinit.as<double>(), 0, s->d_sbus.as<double>(), 0, false, ob, 1);
+  const float ms = launch(s, o, 1, s->d_vinit.as<double>(), 0, s->d_sbus.as<double>(), 0, false, ob, o.n_ctas);
   s->tm.kernel_ms = ms;
   int st = 0, it = 0;
   double res = 0;
@@ -1598,7 +1598,7 @@ int gs2g_set_base_v(gs2g_session* s, const double* v, double* residual) {
   o.fixed_iters = 1;
   o.precision = GS2G_PREC_FP64;
   OutBufs ob{s->b_v.as<double>(), s->b_res.as<double>(), s->b_status.as<int>(), s->b_iters.as<int>()};
-  launch(s, o, 1, s->d_basev.as<double>(), 0, s->d_sbus.as<double>(), 0, false, ob, 1);
+  launch(s, o, 1, s->d_basev.as<double>(), 0, s->d_sbus.as<double>(), 0, false, ob, o.n_ctas);
   double res = 0;
   ck(cudaMemcpy(&res, s->b_res.p, sizeof(double), cudaMemcpyDeviceToHost), "read residual");
   s->base_v.assign(v, v + 2 * n);

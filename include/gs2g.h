@@ -76,7 +76,7 @@ typedef struct gs2g_run_opts {
   int precision;      /* GS2G_PREC_* */
   int start;          /* GS2G_START_* */
   double pivot_floor; /* static-pivot floor, 0 disables */
-  int n_ctas;         /* persistent CTAs, <= 0 for one full wave */
+  int n_ctas;         /* CTAs the run may have (persistent, clusters included), <= 0: the device's */
   int profile_phases; /* 1: record per-phase SM cycles (gs2g_timings.phase_*) */
   /* GS2G_REFACTOR_EVERY: a new LU every Newton step (the reference's default
    * 'direct_refactor_every' strategy).  GS2G_REFACTOR_ADAPTIVE: keep the last

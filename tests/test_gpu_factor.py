@@ -130,6 +130,9 @@ def test_a_callers_cta_count_bounds_the_clusters(n_ctas, sizes):
             s.run_subset(rows, 10, 1e-8, False, lib.PREC_FP64, lib.START_VINIT, n_ctas=n_ctas)
         assert s.cluster_size() in sizes
         assert np.all(s.results()[2] == 0)
+    # a base solve, whose callers give no count, has the device
+    s.solve_base(10, 1e-8, lib.PREC_FP64)
+    assert s.cluster_size() == 16
 
 
 def _leaving(g, rows, seed):
