@@ -227,9 +227,9 @@ __device__ __noinline__ void head_lu(const DevPlan& P, T* HV, const double pfloo
 // chunk is up to 32 columns of one supernode: they differ, so the lanes add to
 // the row without conflicts, and its U values are consecutive.  The chunks of
 // a row are added in supernode order.  Bound by the chain and the instructions
-// of a chunk (17 columns on average): so a lane reads all it needs of a chunk
-// in one 16-byte record (column, U and L positions), loaded ahead, and the two
-// rows' additions overlap.  (Records shared by the warp and handed out by
+// of a chunk (17 columns on average): so what a lane needs of a chunk is two
+// 8-byte loads (the chunk's L position and U stride, the same for all lanes; its
+// own column and U position), made ahead, and the two rows' additions overlap.  (Records shared by the warp and handed out by
 // shuffles, one row at a time: 15.8e9 SM cycles of a 2000-bus FP64 sweep; one
 // lane per target column, summing its contributions one dependent load after
 // another: 37e9.)
