@@ -78,8 +78,8 @@ def test_cluster_handoffs_equal_one_cta_handoffs(name, kind, precision):
     on a cluster of CTAs per row when every such row can have a cluster (the
     N-1 sweep: about a dozen rows), all CTAs of the cluster sharing each
     Schur update and dense tail LU (FP32 or FP64); with more hand-offs than
-    clusters (heavily loaded scenarios) every CTA takes rows of its own.  The
-    shared factorization is bit-identical to the one-CTA one, so every output
+    clusters (heavily loaded scenarios) each row has one CTA.  The shared
+    factorization is bit-identical to the one-CTA one, so every output
     must be too."""
     from gpusim2grid_b200.synthetic import grid_by_name, scenario_outages
     g = grid_by_name(name, 0)
@@ -101,6 +101,8 @@ def test_cluster_handoffs_equal_one_cta_handoffs(name, kind, precision):
             sw.set_topology(scenario_outages(g, n, max_trips=2, seed=32))
         sw.session.set_handoff(cluster)
         sw.compute()
+        if kind == "n1":
+            assert (sw.session.cluster_size() > 0) == bool(cluster)
         out.append((sw.V_results, sw.get_row_status(), sw.get_row_iterations(), sw.get_row_factorizations()))
     (V0, s0, i0, f0), (V1, s1, i1, f1) = out
     assert f0.sum() > 0  # some rows were handed off and factored their own Jacobian
@@ -112,10 +114,10 @@ def test_cluster_handoffs_equal_one_cta_handoffs(name, kind, precision):
 
 @pytest.mark.parametrize("name", ["case2000_synth", "case6500_synth"])
 def test_fp64_subset_on_clusters_equals_one_cta(name):
-    """A small FP64 re-solve (gs2g_run_subset with at most one row per 8 CTAs:
-    the fallback of rows a mixed sweep did not converge) runs each row on a
-    cluster of 8 CTAs sharing its Schur updates and dense LUs; bit-identical
-    to the one-CTA rows and to the same rows of a full FP64 run."""
+    """A small FP64 re-solve (gs2g_run_subset: the fallback of rows a mixed
+    sweep did not converge) runs each row on a cluster of 16 CTAs sharing its
+    factorizations; bit-identical to the one-CTA rows and to the same rows of a
+    full FP64 run."""
     from gpusim2grid_b200._native import lib
     from gpusim2grid_b200.synthetic import grid_by_name
     g = grid_by_name(name, 0)
@@ -133,6 +135,7 @@ def test_fp64_subset_on_clusters_equals_one_cta(name):
         s.set_handoff(cluster)
         s.run(10, 1e-8, False, lib.PREC_FP64, lib.START_VINIT, refactor=lib.REFACTOR_EVERY)
         s.run_subset(sub, 10, 1e-8, False, lib.PREC_FP64, lib.START_VINIT, refactor=lib.REFACTOR_EVERY)
+        assert s.cluster_size() == (16 if cluster else 0)
         V, res, st, it = s.results()
         out.append((V[sub], st[sub], it[sub]))
     for k in range(3):
