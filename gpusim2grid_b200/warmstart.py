@@ -260,8 +260,9 @@ class WarmStartMLP:
         # behind the pass, ahead of the wait for its error flag
         grads = [(self._view(self.grad, l, False).clone(), self._view(self.grad, l, True).clone())
                  for l in range(self.layers + 1)]
+        loss = w["loss"].to("cpu", non_blocking=True)  # there when the flag is: one wait for both
         self.check()
-        return grads, float(w["loss"].item())
+        return grads, float(loss)
 
     def check(self):
         if int(self.err.item()) != 0:
